@@ -316,10 +316,11 @@ int yb_svd_init(const void* a, void* work32, const int64_t* blocks, int n_blocks
 int yb_svd_sweeps(void* work, const int64_t* blocks, int n_blocks, const int32_t* pair_items,
                   int n_pair_items, int max_rounds, int precision, int dtype, int max_sweeps,
                   double tol_stop, int64_t* state, void* stream);
-/* yb_svd_block_sweeps: the FP32 phase with rows grouped into super-vectors of
- * rows_per_super (16, 8 or 4) rows: one CTA per pair of super-vectors holds their rows in
- * shared memory (2 * rows_per_super * lmax FP32 elements, lmax >= every L), runs up to
- * inner_sweeps Jacobi sweeps among them and applies the accumulated rotation to the W rows.
+/* yb_svd_block_sweeps: a phase with rows grouped into super-vectors of rows_per_super (16, 8
+ * or 4) rows, one CTA per pair of super-vectors (lmax >= every L). Where a kernel holds rows of
+ * lmax elements in registers (yb_jacobi.cu) a sweep rotates every pair of rows once; longer rows
+ * lie in shared memory (2 * rows_per_super * lmax elements), where the CTA runs up to
+ * inner_sweeps Jacobi sweeps among its rows and applies the accumulated rotation to the W rows.
  * super_items: int32 pairs (block, super pair index 0..[15]/2-1); max_rounds = max([15]) - 1.
  * precision 32: the FP32 phase (rows_per_super 16, 8 or 4; super-vector count [15]);
  * precision 64: the FP64 phase on the FP64 workspace (rows_per_super 4 or 8; count [23]).
