@@ -1228,7 +1228,8 @@ class SvdSpy:
             e0.record()
             r = orig_call(name, *a, **k)
             e1.record()
-            fp64 = (name == 'yb_svd_sweeps' and a[6] == 64) or (name == 'yb_svd_block_sweeps' and a[7] == 64)
+            fp64 = (name == 'yb_svd_sweeps' and a[6] == 64) or (name == 'yb_svd_block_sweeps' and a[7] == 64) or \
+                (name == 'yb_svd_row_sweeps' and a[5] == 64)
             self.ev.setdefault('fp64_sweeps' if fp64 else name, []).append((e0, e1))
             return r
 
@@ -1259,7 +1260,7 @@ class SvdSpy:
         work = sum(self.work) / steps
         peak = fp64_peak_tflops(torch, dev)
         achieved = work / t64 / 1e12 if t64 > 0 else 0.0
-        return {"bound": "fp64", "kernel": "Jacobi FP64 phase (yb_svd_block_sweeps / yb_svd_sweeps)",
+        return {"bound": "fp64", "kernel": "Jacobi FP64 phase (yb_svd_row_sweeps / yb_svd_block_sweeps)",
                 "achieved": achieved, "peak": peak,
                 "unit": "TFLOP/s", "frac": achieved / peak, "peak_source": "measured live: cuBLAS DGEMM 4096^3",
                 "traffic": None, "launches": n64, "ms_per_launch": t64 / max(n64, 1) * 1e3,

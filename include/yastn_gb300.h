@@ -316,11 +316,10 @@ int yb_svd_init(const void* a, void* work32, const int64_t* blocks, int n_blocks
 int yb_svd_sweeps(void* work, const int64_t* blocks, int n_blocks, const int32_t* pair_items,
                   int n_pair_items, int max_rounds, int precision, int dtype, int max_sweeps,
                   double tol_stop, int64_t* state, void* stream);
-/* yb_svd_block_sweeps: a phase with rows grouped into super-vectors of rows_per_super (16, 8
- * or 4) rows, one CTA per pair of super-vectors (lmax >= every L). Where a kernel holds rows of
- * lmax elements in registers (yb_jacobi.cu) a sweep rotates every pair of rows once; longer rows
- * lie in shared memory (2 * rows_per_super * lmax elements), where the CTA runs up to
- * inner_sweeps Jacobi sweeps among its rows and applies the accumulated rotation to the W rows.
+/* yb_svd_block_sweeps: the FP32 phase with rows grouped into super-vectors of
+ * rows_per_super (16, 8 or 4) rows: one CTA per pair of super-vectors holds their rows in
+ * shared memory (2 * rows_per_super * lmax FP32 elements, lmax >= every L), runs up to
+ * inner_sweeps Jacobi sweeps among them and applies the accumulated rotation to the W rows.
  * super_items: int32 pairs (block, super pair index 0..[15]/2-1); max_rounds = max([15]) - 1.
  * precision 32: the FP32 phase (rows_per_super 16, 8 or 4; super-vector count [15]);
  * precision 64: the FP64 phase on the FP64 workspace (rows_per_super 4 or 8; count [23]).
@@ -328,6 +327,16 @@ int yb_svd_sweeps(void* work, const int64_t* blocks, int n_blocks, const int32_t
 int yb_svd_block_sweeps(void* work32, const int64_t* blocks, int n_blocks, const int32_t* super_items,
                         int n_items, int max_rounds, int rows_per_super, int precision, int dtype, int max_sweeps,
                         int inner_sweeps, double tol_stop, int lmax, int64_t* state, void* stream);
+/* yb_svd_row_sweeps: a phase (precision 32 or 64) with a row of X and W per warp, every pair of
+ * rows above the noise norm rotated once a sweep, for rows of lmax <= yb_svd_row_limit(precision,
+ * dtype) elements (0: no such kernel; YB_ERR_TOO_LARGE above it). n_pairs: number of pair_items.
+ * aux: scratch of yb_svd_row_aux(n_blocks, n_pairs) int64 words, 16-byte aligned (no initial
+ * values). One cooperative launch whose waits are bounded; state as for yb_svd_sweeps. */
+int64_t yb_svd_row_aux(int64_t n_blocks, int64_t n_pairs);
+int yb_svd_row_limit(int precision, int dtype);
+int yb_svd_row_sweeps(void* work, const int64_t* blocks, int n_blocks, const int32_t* pair_items,
+                      int n_pairs, int precision, int dtype, int max_sweeps, double tol_stop, int lmax,
+                      int64_t* state, int64_t* aux, int64_t aux_words, void* stream);
 int yb_svd_widen(const void* work32, void* work64, const int64_t* blocks, int n_blocks, int dtype,
                  int64_t* state, void* stream);
 int yb_svd_shift_prefill(void* work64, const int64_t* blocks, int n_blocks, int dtype,

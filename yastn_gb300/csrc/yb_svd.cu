@@ -999,11 +999,6 @@ int launch_sweeps(T* work, const int64_t* blocks, int n_blocks, const int32_t* p
 
 }  // namespace
 
-// yb_jacobi.cu: rows in registers; YB_ERR_TOO_LARGE where no kernel holds rows of lmax elements
-int jacobi_rows(void* work, const int64_t* blocks, int n_blocks, const int32_t* items, int n_items, int max_rounds,
-                int rows_per_super, int precision, bool cplx, int max_sweeps, int inner_sweeps, double tol_stop,
-                int lmax, int64_t* state, cudaStream_t s);
-
 template <typename T>
 int block_sweeps_t(T* w, const int64_t* blocks, int n_blocks, const int32_t* super_items, int n_items,
                           int max_rounds, int rows_per_super, int max_sweeps, int inner_sweeps, double tol_stop,
@@ -1161,11 +1156,7 @@ int yb_svd_block_sweeps(void* work32, const int64_t* blocks, int n_blocks, const
   if (n_blocks == 0 || n_items == 0 || max_sweeps <= 0) return YB_OK;
   if (!work32 || !blocks || !super_items || !state || lmax <= 0 || inner_sweeps <= 0) return YB_ERR_INVALID;
   if (precision != 32 && precision != 64) return YB_ERR_INVALID;
-  if (dtype != YB_F64 && dtype != YB_C128) return YB_ERR_INVALID;
   cudaStream_t s = (cudaStream_t)stream;
-  const int got = yb::jacobi_rows(work32, blocks, n_blocks, super_items, n_items, max_rounds, rows_per_super,
-                                  precision, dtype == YB_C128, max_sweeps, inner_sweeps, tol_stop, lmax, state, s);
-  if (got != YB_ERR_TOO_LARGE) return got;
   if (precision == 64) {
     if (rows_per_super != 4 && rows_per_super != 8) return YB_ERR_INVALID;
     if (dtype == YB_F64)

@@ -525,6 +525,21 @@ def _svd_state_check(state, nb, phase, require_converged):
     return st[2:R * nb:R]
 
 
+def _row_sweeps(plan, precision, code):
+    """True where the sweeps keep a row per warp (yb_svd_row_sweeps): rows of up to 2624 (FP32),
+    1312 (FP64; half of each for complex data) elements, unless a super-vector height is forced.
+    Longer rows do not fit a warp's registers: they take the shared-memory kernel."""
+    return ROWS_PER_SUPER[0] is None and plan.lmax <= N.lib().yb_svd_row_limit(precision, code)
+
+
+def _run_row_sweeps(plan, work, dblocks, dpairs, nb, precision, code, max_sweeps, tol, state):
+    n_pairs = len(plan.pair_items)
+    words = N.lib().yb_svd_row_aux(nb, n_pairs)
+    aux = torch.empty(words, dtype=torch.int64, device=work.device)
+    N.call('yb_svd_row_sweeps', _ptr(work), _ptr(dblocks), nb, _ptr(dpairs), n_pairs, precision, code, max_sweeps, tol,
+           plan.lmax, _ptr(state), _ptr(aux), words, _stream())
+
+
 def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
     """Mixed-precision batched Jacobi of ``plan`` on ``data``; writes U, S (and Vh for mode 0)."""
     nb = len(plan.blocks)
@@ -547,7 +562,9 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
     else:
         N.call('yb_svd_init', _ptr(data), _ptr(w32), _ptr(dblocks), nb, code, _ptr(state), sp, _ptr(aux[:nb]), st,
                launches=2)
-    if plan.rows_per_super and BLOCKED_FP32[0]:
+    if BLOCKED_FP32[0] and _row_sweeps(plan, 32, code):
+        _run_row_sweeps(plan, w32, dblocks, dpairs, nb, 32, code, MAX_SWEEPS32, TOL_STOP32, state)
+    elif plan.rows_per_super and BLOCKED_FP32[0]:
         (dsup,) = _dev(plan, 'svd_super', (plan.super_items,), dev)
         N.call('yb_svd_block_sweeps', _ptr(w32), _ptr(dblocks), nb, _ptr(dsup), len(plan.super_items),
                plan.super_rounds, plan.rows_per_super, 32, code, MAX_SWEEPS32, INNER_SWEEPS32, TOL_STOP32,
@@ -574,7 +591,9 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
     else:
         run_gemm(plan.xform, w64, data, w64)
     tol64 = TOL_STOP64_QR if plan.qr else (TOL_STOP64 if mode == 0 else TOL_STOP64_EIGH)
-    if plan.rows_per_super64 and BLOCKED_FP64[0]:
+    if BLOCKED_FP64[0] and _row_sweeps(plan, 64, code):
+        _run_row_sweeps(plan, w64, dblocks, dpairs, nb, 64, code, max_sweeps, tol64, state)
+    elif plan.rows_per_super64 and BLOCKED_FP64[0]:
         (dsup64,) = _dev(plan, 'svd_super64', (plan.super_items64,), dev)
         N.call('yb_svd_block_sweeps', _ptr(w64), _ptr(dblocks), nb, _ptr(dsup64), len(plan.super_items64),
                plan.super_rounds64, plan.rows_per_super64, 64, code, max_sweeps, 1, tol64, plan.lmax,
