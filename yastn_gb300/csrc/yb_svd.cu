@@ -512,165 +512,6 @@ __global__ void svd_qr_load_kernel(const T* __restrict__ A, T* __restrict__ work
   }
 }
 
-template <typename T>
-__device__ __forceinline__ T ldcg_t(const T* p) { return __ldcg(p); }
-
-// Householder reflector of row j of Z on its elements [j, L) (LAPACK larfg): beta real,
-// tau = (beta - alpha) / beta, v = x / (alpha - beta) with v_0 = 1 implicit; Z[j] = beta,
-// v stored in Z[j+1..L), tau in tau[j]. One warp.
-template <typename T>
-__device__ void qr_reflector(T* __restrict__ z, T* __restrict__ tau, int64_t j, int64_t L, int lane) {
-  __syncwarp();  // the row was just rewritten by other lanes of this warp
-  double xn = 0.0;
-  for (int64_t l = j + 1 + lane; l < L; l += 32) xn += cabs2(ldcg_t(z + l));
-  xn = warp_sum(xn);
-  const T alpha = ldcg_t(z + j);
-  double ar, ai;
-  if constexpr (Num<T>::cplx) { ar = alpha.x; ai = alpha.y; } else { ar = alpha; ai = 0.0; }
-  if (xn == 0.0 && ai == 0.0) {
-    if (lane == 0) tau[j] = Num<T>::zero();
-    return;
-  }
-  const double beta = -copysign(sqrt(ar * ar + ai * ai + xn), ar);
-  T tv, sc;
-  if constexpr (Num<T>::cplx) {
-    tv = make_double2((beta - ar) / beta, -ai / beta);
-    // 1 / (alpha - beta)
-    const double dr = ar - beta, di = ai, d2 = dr * dr + di * di;
-    sc = make_double2(dr / d2, -di / d2);
-  } else {
-    tv = (beta - ar) / beta;
-    sc = 1.0 / (ar - beta);
-  }
-  for (int64_t l = j + 1 + lane; l < L; l += 32) z[l] = Num<T>::mul(sc, ldcg_t(z + l));
-  if (lane == 0) {
-    if constexpr (Num<T>::cplx) z[j] = make_double2(beta, 0.0); else z[j] = beta;
-    tau[j] = tv;
-  }
-}
-
-// Applies I - t v v^H (v_0 = 1 at element j, v_l at elements l > j of vrow) to a row segment
-// x[j..L) of Z: w = x_j + sum_l conj(v_l) x_l; x_j -= t w; x_l -= t w v_l. One warp.
-template <typename T>
-__device__ __forceinline__ void qr_apply(T* __restrict__ x, const T* __restrict__ vrow, T t, int64_t j, int64_t L,
-                                         int lane) {
-  const T xj = ldcg_t(x + j);
-  T w = Num<T>::zero();
-  for (int64_t l = j + 1 + lane; l < L; l += 32) w = Num<T>::fmac(ldcg_t(x + l), ldcg_t(vrow + l), w);
-  warp_sum_t<T>(w);
-  w = Num<T>::add(w, xj);
-  const T tw = Num<T>::mul(t, w);
-  if (lane == 0) x[j] = Num<T>::sub(xj, tw);
-  for (int64_t l = j + 1 + lane; l < L; l += 32) x[l] = Num<T>::sub(ldcg_t(x + l), Num<T>::mul(tw, ldcg_t(vrow + l)));
-  __syncwarp();
-}
-
-// Waits (lane 0 polls, bounded) until *flag >= target; on timeout raises *err and returns
-// (the caller carries on with whatever it reads: the host sees the error word and fails).
-__device__ __forceinline__ void qr_wait(const unsigned long long* flag, unsigned long long target,
-                                        unsigned long long* err, int lane) {
-  if (lane == 0) {
-    long long spins = 0;
-    while (*(volatile const unsigned long long*)flag < target) {
-      __nanosleep(32);
-      if (++spins > kSpinLimit) {
-        atomicExch(err, 1ull);
-        break;
-      }
-    }
-    __threadfence();
-  }
-  __syncwarp();
-}
-
-__device__ __forceinline__ void qr_publish(unsigned long long* flag, unsigned long long value, int lane) {
-  __syncwarp();
-  if (lane == 0) {
-    __threadfence();
-    atomicMax(flag, value);
-  }
-}
-
-// One cooperative launch: groups of `group` CTAs factor one block at a time. Row c of Z is
-// handled by warp c mod (8 group) of the group throughout, so a row is only ever rewritten by
-// the warp that reads it, and the only exchange is each reflector: the warp owning row j+1
-// updates it first in step j, makes reflector j+1 and publishes it through the block's
-// ready counter (flags[b] = number of reflectors published); every warp waits for reflector j
-// before applying it, so warps run ahead of each other as far as the data allows. Then (one
-// group barrier) R's rows, the FP32 start X32 = scale R, W32 = I and the reflectors are
-// written; after a second barrier every warp forms its own columns of Q independently
-// (Q e_c = H_0 ... H_c e_c), in place of its rows of Z.
-template <typename T, typename T32>
-__global__ void __launch_bounds__(kThreads) svd_qr_kernel(T* __restrict__ work, T32* __restrict__ work32,
-                                                          const int64_t* __restrict__ blocks, int n_blocks,
-                                                          int group, unsigned long long* __restrict__ qctrl,
-                                                          const double* __restrict__ scale) {
-  const int g = blockIdx.x / group, rank = blockIdx.x % group;
-  const int n_groups = gridDim.x / group;
-  if (g >= n_groups) return;
-  unsigned long long* flags = qctrl;  // [n_blocks ready counters][C_REC words per group]
-  unsigned long long* ctrl = qctrl + n_blocks + (int64_t)g * C_REC;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t gw = (int64_t)rank * kWarps + warp, nwg = (int64_t)group * kWarps;
-  const int64_t gt = (int64_t)rank * kThreads + threadIdx.x, ngt = (int64_t)group * kThreads;
-  for (int b = g; b < n_blocks; b += n_groups) {
-    const int64_t* r = blocks + (int64_t)b * YB_SVD_REC;
-    if (!r[R_QR]) continue;
-    const int64_t k = r[R_K], L = r[R_LQ];
-    T* Z = work + r[R_Z];
-    T* V = work + r[R_VQ];
-    T* tau = work + r[R_TAU];
-    T* RR = work + r[R_RR];
-    T32* X32 = work32 + r[R_X32];
-    T32* W32 = work32 + r[R_W32];
-    unsigned long long* ready = flags + b;
-    const double sc = scale ? scale[b] : 0.0;  // no FP32 Jacobi start for yb_qr
-    // factorisation
-    if (gw == 0) {
-      qr_reflector<T>(Z, tau, 0, L, lane);
-      qr_publish(ready, 1ull, lane);
-    }
-    for (int64_t j = 0; j < k; ++j) {
-      const int64_t first = j + 1 + ((gw - (j + 1)) % nwg + nwg) % nwg;
-      if (first >= k) break;  // no rows of this warp below row j: none below any later row either
-      qr_wait(ready, (unsigned long long)(j + 1), ctrl + C_ERR, lane);
-      const T* vrow = Z + j * L;
-      const T t = Num<T>::conj(ldcg_t(tau + j));  // M <- H^H M
-      for (int64_t c = first; c < k; c += nwg) {
-        qr_apply<T>(Z + c * L, vrow, t, j, L, lane);
-        if (c == j + 1) {
-          qr_reflector<T>(Z + c * L, tau, j + 1, L, lane);
-          qr_publish(ready, (unsigned long long)(j + 2), lane);
-        }
-      }
-    }
-    if (!grid_barrier(ctrl, group)) return;
-    // R rows, the FP32 start, the reflectors
-    for (int64_t e = gt; e < k * k; e += ngt) {
-      const int64_t i = e / k, c = e - i * k;
-      const T v = (c >= i) ? ldcg_t(Z + c * L + i) : Num<T>::zero();
-      RR[e] = v;
-      if (scale) {
-        X32[e] = to32(rscale(v, sc));
-        W32[e] = (i == c) ? Num<T32>::one() : Num<T32>::zero();
-      }
-    }
-    for (int64_t e = gt; e < k * L; e += ngt) {
-      const int64_t j = e / L, l = e - j * L;
-      V[e] = (l > j) ? ldcg_t(Z + e) : Num<T>::zero();
-    }
-    if (!grid_barrier(ctrl, group)) return;
-    // Q's columns: row c of Z becomes (H_0 ... H_c e_c)^T
-    for (int64_t c = gw; c < k; c += nwg) {
-      T* x = Z + c * L;
-      for (int64_t l = lane; l < L; l += 32) x[l] = (l == c) ? Num<T>::one() : Num<T>::zero();
-      __syncwarp();
-      for (int64_t j = c; j >= 0; --j) qr_apply<T>(x, V + j * L, ldcg_t(tau + j), j, L, lane);
-    }
-    if (!grid_barrier(ctrl, group)) return;
-  }
-}
-
 // Candidate vectors of the blocked completion: G (L x nz, row-major per record) filled with
 // values uniform in [-1, 1) from a counter-based hash of (record, element) (deterministic;
 // any full-rank draw works: the candidates are projected and orthonormalised afterwards).
@@ -999,6 +840,12 @@ int launch_sweeps(T* work, const int64_t* blocks, int n_blocks, const int32_t* p
 
 }  // namespace
 
+// yb_qr_f64.cu, yb_qr_c128.cu: the factorisation of every block (yb_qr.cuh)
+int qr_factor_f64(void* work, void* work32, const int64_t* blocks, int n_blocks, double* scale, int64_t* qctrl,
+                  int qctrl_words, cudaStream_t s);
+int qr_factor_c128(void* work, void* work32, const int64_t* blocks, int n_blocks, double* scale, int64_t* qctrl,
+                   int qctrl_words, cudaStream_t s);
+
 template <typename T>
 int block_sweeps_t(T* w, const int64_t* blocks, int n_blocks, const int32_t* super_items, int n_items,
                           int max_rounds, int rows_per_super, int max_sweeps, int inner_sweeps, double tol_stop,
@@ -1017,35 +864,16 @@ int block_sweeps_t(T* w, const int64_t* blocks, int n_blocks, const int32_t* sup
   }
 }
 
-template <typename T, typename T32>
+template <typename T>
 int qr_t(const void* a, void* work, void* work32, const int64_t* blocks, int n_blocks, int64_t* state, double* scale,
          int64_t* qctrl, int qctrl_words, cudaStream_t s) {
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, yb::svd_qr_kernel<T, T32>, yb::kThreads, 0);
-  if (e != cudaSuccess) { yb::set_cuda_error((int)e); return YB_ERR_CUDA; }
-  const int capacity = sms * (per_sm < 1 ? 1 : per_sm);
-  int group = capacity / n_blocks;
-  group = group < 1 ? 1 : (group > 64 ? 64 : group);
-  int n_groups = capacity / group;
-  if (n_groups > n_blocks) n_groups = n_blocks;
-  if ((int64_t)n_groups * yb::C_REC + n_blocks > qctrl_words) n_groups = (qctrl_words - n_blocks) / yb::C_REC;
-  if (n_groups < 1) return YB_ERR_INVALID;
-  if (state) yb::block_fro_kernel<T><<<n_blocks, 256, 0, s>>>((const T*)a, blocks, nullptr, scale, state);
-  yb::svd_qr_load_kernel<T><<<dim3(64, (unsigned)n_blocks), 256, 0, s>>>((const T*)a, (T*)work, blocks);
-  e = cudaMemsetAsync(qctrl, 0, sizeof(int64_t) * ((size_t)n_groups * yb::C_REC + n_blocks), s);
-  if (e != cudaSuccess) { yb::set_cuda_error((int)e); return YB_ERR_CUDA; }
-  T* w = (T*)work;
-  T32* w32 = (T32*)work32;
-  unsigned long long* qc = (unsigned long long*)qctrl;
-  void* args[] = {&w, &w32, &blocks, &n_blocks, &group, &qc, &scale};
-  e = cudaLaunchCooperativeKernel((const void*)yb::svd_qr_kernel<T, T32>, dim3(n_groups * group), dim3(yb::kThreads),
-                                  args, 0, s);
-  if (e != cudaSuccess) { yb::set_cuda_error((int)e); return YB_ERR_CUDA; }
-  if (state) yb::svd_state_reset_kernel<<<n_blocks, 32, 0, s>>>(state);
-  return yb::check_launch();
+  if (state) block_fro_kernel<T><<<n_blocks, 256, 0, s>>>((const T*)a, blocks, nullptr, scale, state);
+  svd_qr_load_kernel<T><<<dim3(64, (unsigned)n_blocks), 256, 0, s>>>((const T*)a, (T*)work, blocks);
+  const int st = Num<T>::cplx ? qr_factor_c128(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, s)
+                              : qr_factor_f64(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, s);
+  if (st != YB_OK) return st;
+  if (state) svd_state_reset_kernel<<<n_blocks, 32, 0, s>>>(state);
+  return check_launch();
 }
 
 template <typename T>
@@ -1092,8 +920,8 @@ int yb_svd_qr(const void* a, void* work64, void* work32, const int64_t* blocks, 
   if (!a || !work64 || !work32 || !blocks || !state || !scale || !qctrl) return YB_ERR_INVALID;
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype == YB_F64)
-    return yb::qr_t<double, float>(a, work64, work32, blocks, n_blocks, state, scale, qctrl, qctrl_words, s);
-  return yb::qr_t<double2, float2>(a, work64, work32, blocks, n_blocks, state, scale, qctrl, qctrl_words, s);
+    return yb::qr_t<double>(a, work64, work32, blocks, n_blocks, state, scale, qctrl, qctrl_words, s);
+  return yb::qr_t<double2>(a, work64, work32, blocks, n_blocks, state, scale, qctrl, qctrl_words, s);
 }
 
 int yb_fill_candidates(void* G, const int64_t* recs, int n_recs, int dtype, void* stream) {
@@ -1116,11 +944,11 @@ int yb_qr(const void* a, void* Q, void* R, void* work64, const int64_t* blocks, 
   const dim3 grid(64, (unsigned)n_blocks);
   int st;
   if (dtype == YB_F64) {
-    st = yb::qr_t<double, float>(a, work64, nullptr, blocks, n_blocks, nullptr, nullptr, qctrl, qctrl_words, s);
+    st = yb::qr_t<double>(a, work64, nullptr, blocks, n_blocks, nullptr, nullptr, qctrl, qctrl_words, s);
     if (st != YB_OK) return st;
     yb::qr_finalize_kernel<double><<<grid, 256, 0, s>>>((const double*)work64, (double*)Q, (double*)R, blocks);
   } else {
-    st = yb::qr_t<double2, float2>(a, work64, nullptr, blocks, n_blocks, nullptr, nullptr, qctrl, qctrl_words, s);
+    st = yb::qr_t<double2>(a, work64, nullptr, blocks, n_blocks, nullptr, nullptr, qctrl, qctrl_words, s);
     if (st != YB_OK) return st;
     yb::qr_finalize_kernel<double2><<<grid, 256, 0, s>>>((const double2*)work64, (double2*)Q, (double2*)R, blocks);
   }
