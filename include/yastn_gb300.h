@@ -339,6 +339,13 @@ int yb_svd_row_sweeps(void* work, const int64_t* blocks, int n_blocks, const int
                       int64_t* state, int64_t* aux, int64_t aux_words, void* stream);
 int yb_svd_widen(const void* work32, void* work64, const int64_t* blocks, int n_blocks, int dtype,
                  int64_t* state, void* stream);
+/* T <- 1.5 I - 0.5 T for every block, T (k x k) at t_delta elements after W in the FP64 workspace:
+ * the right factor of the Newton-Schulz step W (1.5 I - 0.5 W^H W). */
+int yb_svd_ns_prep(void* work64, const int64_t* blocks, int n_blocks, int dtype, int64_t t_delta, void* stream);
+/* T = W D and Wn = D^-1 R (at t_delta and 2 t_delta elements after W) for blocks with a QR start, D
+ * the powers of two of a two-sided equilibration of R: the operands of X = W R for a product whose
+ * digits are scaled per row and column. X's storage is scratch. Three launches. */
+int yb_svd_scale_wr(void* work64, const int64_t* blocks, int n_blocks, int dtype, int64_t t_delta, void* stream);
 int yb_svd_shift_prefill(void* work64, const int64_t* blocks, int n_blocks, int dtype,
                          const double* shift, void* stream);
 /* yb_svd_qr: the QR-preconditioned start (every block of the records has [16] = 1), in

@@ -786,6 +786,95 @@ def ozaki_dot_plan(meta_dot, s, cplx=False):
     return CACHE.get((meta_dot,), ('ozaki_dot', s, bool(cplx)), build)
 
 
+class EmulatedGemm:
+    """Grouped products C = op(A) op(B) (one term per output, C assigned) on the BF16 tensor cores:
+    split records, output records and tiles of one kernel (``tile_n`` 64 or 32: tcgen05; 0:
+    mma.sync), and the products that stay native FP64 (short K, skinny outputs)."""
+
+    def __init__(self, **kw):
+        self.__dict__.update(kw)
+        self._dev = {}
+
+
+def emulated_gemm(out_list, s, cplx=False):
+    """``out_list`` as for ``_pack_gemm`` with one term per output, flags 0 or 1 (op(A) conjugated);
+    offsets and strides in elements. A complex product is two real ones of doubled K: A's rows
+    as [re | im] (conjugated: [re | -im]), B's columns as [re | -im] and [im | re]."""
+    f = 2 if cplx else 1
+    where, blocks, refs, small = {}, [], [], []
+    flops = 0
+
+    def operand(op, off, rows, K, rs, ks, mode):
+        key = (op, off, rows, K, rs, ks, mode)
+        if key not in where:
+            where[key] = len(blocks)
+            blocks.append((op, off, rows, f * K, rs, ks, mode, (f * K + 15) // 16 * 16))
+        return where[key]
+
+    for c_off, m, n, ldc, terms in out_list:
+        (a_off, b_off, K, ars, acs, brs, bcs, fl), = terms
+        if m == 0 or n == 0:
+            continue
+        if K < OZAKI_MIN_DIM or (m <= OZAKI_SKINNY_ROWS and n > GEMM_TILE):
+            small.append((c_off, m, n, ldc, terms))
+            continue
+        ai = operand(0, a_off, m, K, ars, acs, (2 if fl & 1 else 1) if cplx else 0)
+        for part, mode in enumerate((2, 3) if cplx else (0,)):
+            bi = operand(1, b_off, n, K, bcs, brs, mode)
+            refs.append((f * c_off + part, m, n, f * ldc, ai, bi, f * K, (f * K + 15) // 16 * 16, f))
+        flops += (8 if cplx else 2) * m * n * K
+
+    def padded(tm, tn):
+        return sum(-(-m // tm) * tm * -(-n // tn) * tn * Kp for _, m, n, _, _, _, _, Kp, _ in refs)
+    w64, w128, w32 = padded(64, 64), padded(OZAKI_TC_M, 64), padded(OZAKI_TC_M, 32)
+    tile_n = (32 if w32 < w128 else 64) if min(w32, w128) <= 1.6 * w64 else 0
+    tm, tn = (OZAKI_TC_M, tile_n) if tile_n else (64, 64)
+    recs, groups, asz, bsz, aex, bex, at = _split_layout(blocks, s, tm if tile_n else 0, tn if tile_n else 0)
+    outs = np.array([(c, m, n, ld, at[ai][0], at[ai][1], at[bi][0], at[bi][1], Kr, Kp, cs, 0, 0, 0, 0, 0)
+                     for c, m, n, ld, ai, bi, Kr, Kp, cs in refs], dtype=np.int64).reshape(-1, 16)
+    tiles = [(int(o[8]), oi, tr, tc) for oi, o in enumerate(outs)
+             for tr in range(-(-int(o[1]) // tm)) for tc in range(-(-int(o[2]) // tn))]
+    tiles.sort(key=lambda x: -x[0])
+    tiles = np.array([(oi, tr, tc, 0) for _, oi, tr, tc in tiles], dtype=np.int32).reshape(-1, 4)
+    sfx = {64: '_tc', 32: '_tc32', 0: ''}[tile_n]
+    return EmulatedGemm(**{'tile_n': tile_n, 'slices': s, 'recs': recs, 'groups': groups, 'a_size': asz, 'b_size': bsz,
+                           'a_exps': aex, 'b_exps': bex, 'flops': flops, 'native': _pack_gemm(small),
+                           'outs' + sfx: outs, 'tiles' + sfx: tiles, 'n_tiles': len(tiles)})
+
+
+def svd_emulated(plan, s, cplx):
+    """The products of the block SVD's FP64 steps as emulated GEMMs, from the records of ``plan``:
+    T = W^H W and W' = W (1.5 - 0.5 T) from W and back from Wn, X = W X_0 (QR start: W R; else W A
+    into T, ``xa``), and the factor that comes from Q."""
+    got = plan.__dict__.get('_emulated')
+    if got is not None:
+        return got
+    w0, t0, n0, ws = plan.w_range
+    gram, ns, gram2, ns2, xr, xa, qu, qv = [], [], [], [], [], [], [], []
+    cj = int(cplx)
+    for r in plan.blocks:
+        a0, m, n, u0, v0, x0, W, k, tall = (int(r[i]) for i in (0, 1, 2, 3, 5, 6, 7, 9, 12))
+        T, Wn = W + ws, W + 2 * ws
+        gram.append((T, k, k, k, [(W, W, k, 1, k, k, 1, cj)]))
+        ns.append((Wn, k, k, k, [(W, T, k, k, 1, k, 1, 0)]))
+        gram2.append((T, k, k, k, [(Wn, Wn, k, 1, k, k, 1, cj)]))
+        ns2.append((W, k, k, k, [(Wn, T, k, k, 1, k, 1, 0)]))
+        if int(r[16]) == 1:
+            LQ, Z, WS = (int(r[i]) for i in (17, 18, 22))
+            xr.append((x0, k, k, k, [(T, Wn, k, k, 1, k, 1, 0)]))  # W R scaled (yb_svd_scale_wr)
+            if tall:
+                qu.append((u0, m, k, k, [(Z, WS, k, 1, LQ, 1, k, cj)]))
+            else:
+                qv.append((v0, k, n, n, [(WS, Z, k, k, 1, LQ, 1, 0)]))
+        elif m == n:
+            xa.append((T, k, k, k, [(W, a0, k, k, 1, n, 1, 0)]))
+    got = {name: emulated_gemm(lst, s, cplx)
+           for name, lst in (('gram', gram), ('ns', ns), ('gram2', gram2), ('ns2', ns2), ('xr', xr), ('xa', xa),
+                             ('qu', qu), ('qv', qv))}
+    plan._emulated = got
+    return got
+
+
 # ----------------------------------------------------------------------------- SVD
 
 class SvdPlan:
@@ -1010,13 +1099,14 @@ class CompletionPlan:
     projections C = V_g^H G (g1) and G -= V_g C (g2), the QR records of the candidates, and
     the copy of the orthonormalised candidates into the factor."""
 
-    def __init__(self, to_u, g1, g2, meta, fill, copy, sizes):
+    def __init__(self, to_u, g1, g2, meta, fill, copy, sizes, e1=None, e2=None):
+        self.e1, self.e2 = e1, e2  # the same products (g2's without the subtraction) emulated
         self.to_u, self.g1, self.g2, self.meta, self.fill, self.copy = to_u, g1, g2, meta, fill, copy
         self.G, self.C, self.Q, self.R = sizes
         self._dev = {}
 
 
-def completion_plans(blocks, nz, cplx=False):
+def completion_plans(blocks, nz, cplx=False, slices=8):
     """Completion plans of svd records ``blocks`` (SVD_REC) for the per-block counts ``nz`` of
     vectors to complete (the last nz of each block's k). The vectors built from X's rows are
     U's columns for tall blocks started from A's rows and for wide blocks started from R's,
@@ -1051,7 +1141,8 @@ def completion_plans(blocks, nz, cplx=False):
         out.append(CompletionPlan(to_u, _pack_gemm(t['g1']), _pack_gemm(t['g2']), tuple(t['meta']),
                                   np.array(t['fill'], dtype=np.int64).reshape(-1, 2),
                                   CopyPlan(t['copies'], sum(int(np.prod(c[2])) for c in t['copies']), 0),
-                                  (t['G'], t['C'], t['Q'], t['R'])))
+                                  (t['G'], t['C'], t['Q'], t['R']),
+                                  emulated_gemm(t['g1'], slices, cplx), emulated_gemm(t['g2'], slices, cplx)))
     return out
 
 

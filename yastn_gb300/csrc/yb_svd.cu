@@ -115,6 +115,97 @@ __global__ void svd_widen_kernel(const T32* __restrict__ work32, T64* __restrict
   if (blockIdx.x == 0 && threadIdx.x < ST_THR32) state[blockIdx.y * ST_REC + threadIdx.x] = 0;
 }
 
+// T <- 1.5 I - 0.5 T for every block, T = W^H W at t_delta elements after W: the right factor of a
+// Newton-Schulz step W' = W (1.5 I - 0.5 W^H W).
+template <typename T64>
+__global__ void svd_ns_prep_kernel(T64* __restrict__ work64, const int64_t* __restrict__ blocks, int64_t t_delta) {
+  const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
+  const int64_t k = r[R_K];
+  T64* T = work64 + r[R_W] + t_delta;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < k * k; e += (int64_t)gridDim.x * blockDim.x) {
+    const T64 v = rscale(T[e], -0.5);
+    T[e] = e / k == e % k ? add_real(v, 1.5) : v;
+  }
+}
+
+// Operands of X = W R scaled along the contracted index: T = W D, Wn = D^-1 R, D the powers of two
+// of a two-sided equilibration of R: with c_j the exponent of the largest entry of column j, row l
+// gets the exponent max_j (exponent of R_lj - c_j), in [-200, 0]. The small rows of a graded R go
+// with entries of W that are small for the large ones, so the entries of a row of T and of a column
+// of Wn have one size each, and digits scaled per row of T and per column of Wn keep the relative
+// accuracy that an FP64 sum of the products has, for R graded by rows, by columns or both.
+// X's storage holds c (k values) and D (the next k) meanwhile (k = 1: no scaling).
+__device__ __forceinline__ int top_exponent(double v) {  // -2000 for zero
+  const int e = (int)((__double_as_longlong(v) >> 52) & 0x7ff);
+  return e ? e - 1023 : -2000;
+}
+__device__ __forceinline__ int top_exponent(double2 v) { return max(top_exponent(v.x), top_exponent(v.y)); }
+__device__ __forceinline__ double real_of(double v) { return v; }
+__device__ __forceinline__ double real_of(double2 v) { return v.x; }
+__device__ __forceinline__ void set_real(double& d, double v) { d = v; }
+__device__ __forceinline__ void set_real(double2& d, double v) { d = make_double2(v, 0.0); }
+
+template <typename T64>
+__global__ void svd_col_exponents_kernel(T64* __restrict__ work64, const int64_t* __restrict__ blocks) {
+  const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
+  if (!r[R_QR]) return;
+  const int64_t k = r[R_K];
+  const T64* R = work64 + r[R_RR];
+  __shared__ int red[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int64_t j0 = (int64_t)blockIdx.x * 32; j0 < k; j0 += (int64_t)gridDim.x * 32) {
+    const int64_t j = j0 + lane;
+    int e = -2000;
+    for (int64_t l = warp; l < k && l < j0 + 32; l += 8)
+      if (j < k && l <= j) e = max(e, top_exponent(R[l * k + j]));
+    red[warp][lane] = e;
+    __syncthreads();
+    if (warp == 0 && j < k) {
+      for (int w = 1; w < 8; ++w) e = max(e, red[w][lane]);
+      set_real(work64[r[R_X] + j], (double)e);
+    }
+    __syncthreads();
+  }
+}
+
+template <typename T64>
+__global__ void svd_row_scales_kernel(T64* __restrict__ work64, const int64_t* __restrict__ blocks) {
+  const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
+  const int64_t k = r[R_K];
+  if (!r[R_QR] || k < 2) return;
+  const T64* R = work64 + r[R_RR];
+  T64* c = work64 + r[R_X];
+  const int lane = threadIdx.x & 31, nw = (int)(gridDim.x * blockDim.x) >> 5;
+  for (int64_t l = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; l < k; l += nw) {
+    int e = -200;
+    for (int64_t j = l + lane; j < k; j += 32) {
+      const int v = top_exponent(R[l * k + j]);
+      if (v > -2000) e = max(e, v - (int)real_of(c[j]));
+    }
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (lane == 0) set_real(c[k + l], __longlong_as_double((long long)(1023 + e) << 52));
+  }
+}
+
+template <typename T64>
+__global__ void svd_scale_wr_kernel(T64* __restrict__ work64, const int64_t* __restrict__ blocks, int64_t t_delta) {
+  const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
+  if (!r[R_QR]) return;
+  const int64_t k = r[R_K];
+  const T64* W = work64 + r[R_W];
+  const T64* R = work64 + r[R_RR];
+  const T64* d = work64 + r[R_X] + k;
+  T64* Ws = work64 + r[R_W] + t_delta;
+  T64* Rs = work64 + r[R_W] + 2 * t_delta;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < k * k; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = e / k, j = e - i * k;
+    Ws[e] = k < 2 ? W[e] : rscale(W[e], real_of(d[j]));
+    // the inverse of a power of two: its exponent negated
+    Rs[e] = k < 2 ? R[e]
+                  : rscale(R[e], __longlong_as_double(((long long)2046 << 52) - __double_as_longlong(real_of(d[i]))));
+  }
+}
+
 // X = shift_b * W (eigh: the FP64 phase then adds W A with the grouped GEMM, X = W (A + shift I)).
 template <typename T64>
 __global__ void svd_shift_prefill_kernel(T64* __restrict__ work64, const int64_t* __restrict__ blocks,
@@ -1017,6 +1108,36 @@ int yb_svd_widen(const void* work32, void* work64, const int64_t* blocks, int n_
                                                                state);
   else
     return YB_ERR_INVALID;
+  return yb::check_launch();
+}
+
+int yb_svd_ns_prep(void* work64, const int64_t* blocks, int n_blocks, int dtype, int64_t t_delta, void* stream) {
+  if (n_blocks == 0) return YB_OK;
+  if (!work64 || !blocks || t_delta <= 0) return YB_ERR_INVALID;
+  const dim3 grid(64, (unsigned)n_blocks);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (dtype == YB_F64) yb::svd_ns_prep_kernel<double><<<grid, 256, 0, s>>>((double*)work64, blocks, t_delta);
+  else if (dtype == YB_C128) yb::svd_ns_prep_kernel<double2><<<grid, 256, 0, s>>>((double2*)work64, blocks, t_delta);
+  else return YB_ERR_INVALID;
+  return yb::check_launch();
+}
+
+int yb_svd_scale_wr(void* work64, const int64_t* blocks, int n_blocks, int dtype, int64_t t_delta, void* stream) {
+  if (n_blocks == 0) return YB_OK;
+  if (!work64 || !blocks || t_delta <= 0) return YB_ERR_INVALID;
+  const dim3 grid(64, (unsigned)n_blocks);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (dtype == YB_F64) {
+    yb::svd_col_exponents_kernel<double><<<grid, 256, 0, s>>>((double*)work64, blocks);
+    yb::svd_row_scales_kernel<double><<<grid, 256, 0, s>>>((double*)work64, blocks);
+    yb::svd_scale_wr_kernel<double><<<grid, 256, 0, s>>>((double*)work64, blocks, t_delta);
+  } else if (dtype == YB_C128) {
+    yb::svd_col_exponents_kernel<double2><<<grid, 256, 0, s>>>((double2*)work64, blocks);
+    yb::svd_row_scales_kernel<double2><<<grid, 256, 0, s>>>((double2*)work64, blocks);
+    yb::svd_scale_wr_kernel<double2><<<grid, 256, 0, s>>>((double2*)work64, blocks, t_delta);
+  } else {
+    return YB_ERR_INVALID;
+  }
   return yb::check_launch();
 }
 

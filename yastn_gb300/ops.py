@@ -409,6 +409,36 @@ def _ozaki_run(plan, A, B, out, slices, tc):
                len(arrs[3]), slices, st)
 
 
+def run_emulated(eg, a, b, c):
+    """The products of ``eg`` (P.EmulatedGemm) from the flat tensors a and b into c: one split
+    launch, one GEMM launch, and a native FP64 launch for the short ones."""
+    if eg.native.outs.size:
+        run_gemm(eg.native, a, b, c)
+    if eg.n_tiles == 0:
+        return c
+    dev, st = c.device, _stream()
+    tc = eg.tile_n
+    if tc:
+        tiles, offs = P.ozaki_tc_schedule(eg, _sm_count(dev), tc)
+        arrs = (eg.recs, eg.groups, getattr(eg, 'outs_tc' if tc == 64 else 'outs_tc32'), tiles, offs)
+    else:
+        arrs = (eg.recs, eg.groups, eg.outs, eg.tiles)
+    d = _dev(eg, 'emulated', arrs, dev)
+    a_sl = torch.empty(max(eg.a_size, 1), dtype=torch.bfloat16, device=dev)
+    b_sl = torch.empty(max(eg.b_size, 1), dtype=torch.bfloat16, device=dev)
+    ex = torch.empty(eg.a_exps + eg.b_exps, dtype=torch.int32, device=dev)
+    b_ex = ex[eg.a_exps:]
+    N.call('yb_ozaki_split', _ptr(a), _ptr(b), _ptr(a_sl), _ptr(b_sl), _ptr(ex), _ptr(b_ex), _ptr(d[0]), _ptr(d[1]),
+           len(eg.groups), eg.slices, st)
+    if tc:
+        N.call('yb_ozaki_gemm_tc', _ptr(a_sl), _ptr(ex), _ptr(b_sl), _ptr(b_ex), _ptr(c), _ptr(d[2]), _ptr(d[3]),
+               eg.n_tiles, _ptr(d[4]), len(arrs[4]) - 1, tc, eg.slices, st)
+    else:
+        N.call('yb_ozaki_gemm', _ptr(a_sl), _ptr(ex), _ptr(b_sl), _ptr(b_ex), _ptr(c), _ptr(d[2]), _ptr(d[3]),
+               eg.n_tiles, eg.slices, st)
+    return c
+
+
 _SMS = {}
 
 
@@ -508,6 +538,7 @@ BLOCKED_FP32 = [True]  # FP32 phase on super-vectors in shared memory (False: on
 BLOCKED_FP64 = [True]  # FP64 phase likewise, on 4-row super-vectors (False: one pair per warp)
 ROWS_PER_SUPER = [None]  # super-vector height (None: largest of 16, 8, 4 that fits)
 NS_STEPS = 2          # Newton-Schulz steps: non-orthogonality ~1e-6 -> 1e-12 -> ~eps
+SVD_EMULATED = [True]  # FP64 products inside svd / eigh on the tensor cores (False: the native grouped GEMM)
 SVD_QR = [True]       # svd: Jacobi on the rows of R of a Householder QR (few FP64 sweeps on graded spectra)
 
 
@@ -572,22 +603,46 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
     else:
         N.call('yb_svd_sweeps', _ptr(w32), _ptr(dblocks), nb, _ptr(dpairs), len(plan.pair_items), plan.max_rounds,
                32, code, MAX_SWEEPS32, TOL_STOP32, _ptr(state), st)
-    _svd_state_check(state, nb, 'FP32', False)
+    host = state.cpu()
+    _svd_state_check(host, nb, 'FP32', False)
+    thr64 = np.ascontiguousarray(host.numpy()[5:SVD_STATE_REC * nb:SVD_STATE_REC]).view(np.float64)
     if qctrl is not None and bool(qctrl[nb + 2::4].any()):
         raise RuntimeError("yastn_gb300 svd: QR group barrier timed out")
     N.call('yb_svd_widen', _ptr(w32), _ptr(w64), _ptr(dblocks), nb, code, _ptr(state), st)
     w0, t0, n0, ws = plan.w_range
-    W, Wn = w64[w0:w0 + ws], w64[n0:n0 + ws]
-    for _ in range(NS_STEPS):
-        Wn.copy_(W)
-        run_gemm(plan.gram, w64, w64, w64)
-        run_gemm(plan.ns, w64, w64, w64, alpha=-0.5, beta=1.5)
-        W.copy_(Wn)
+    # The FP64 products of the block SVD run on the tensor cores (57-bit digits per row and column,
+    # one rounding per 400 contracted indices; R's grading is taken out of X = W R first): their
+    # errors are no larger than the DFMA kernel's, which the FP64 pipe bounds: 2.7 against 0.46 ms
+    # for all products of two 432 x 432 blocks, 55 against 3.7 ms for two 1296 x 1296, 0.64 against
+    # 0.10 ms in the eigh of five blocks up to 110. Short products (K < 16) stay native, and so does
+    # a call with a block of non-finite norm, whose NaN and Inf propagate.
+    emu = None
+    if SVD_EMULATED[0] and np.isfinite(thr64).all():
+        emu = P.svd_emulated(plan, OZAKI_SLICES, cplx)
+        for gram, ns in (('gram', 'ns'), ('gram2', 'ns2')):
+            run_emulated(emu[gram], w64, w64, w64)
+            N.call('yb_svd_ns_prep', _ptr(w64), _ptr(dblocks), nb, code, ws, st)
+            run_emulated(emu[ns], w64, w64, w64)
+    else:
+        W, Wn = w64[w0:w0 + ws], w64[n0:n0 + ws]
+        for _ in range(NS_STEPS):
+            Wn.copy_(W)
+            run_gemm(plan.gram, w64, w64, w64)
+            run_gemm(plan.ns, w64, w64, w64, alpha=-0.5, beta=1.5)
+            W.copy_(Wn)
     if plan.qr:
-        run_gemm(plan.xform, w64, w64, w64)  # X = W R
+        if emu:
+            N.call('yb_svd_scale_wr', _ptr(w64), _ptr(dblocks), nb, code, ws, st, launches=3)
+            run_emulated(emu['xr'], w64, w64, w64)  # X = W R = T Wn
+        else:
+            run_gemm(plan.xform, w64, w64, w64)
     elif shift is not None:
         N.call('yb_svd_shift_prefill', _ptr(w64), _ptr(dblocks), nb, code, _ptr(shift), st)
-        run_gemm(plan.xform, w64, data, w64, beta=1.0)
+        if emu:  # X = shift W + W A, W A by way of T (laid out like X: the blocks are square)
+            run_emulated(emu['xa'], w64, data, w64)
+            w64[:ws].add_(w64[t0:t0 + ws])
+        else:
+            run_gemm(plan.xform, w64, data, w64, beta=1.0)
     else:
         run_gemm(plan.xform, w64, data, w64)
     tol64 = TOL_STOP64_QR if plan.qr else (TOL_STOP64 if mode == 0 else TOL_STOP64_EIGH)
@@ -608,13 +663,17 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
     if n_small is not None:
         nz = n_small.cpu().numpy()
         if nz.any():
-            _complete(plan, U, V, nz, cplx)
+            _complete(plan, U, V, nz, cplx, emu is not None)
     if plan.qr:  # the factor that comes from Q: Vh = conj(W) Q^T (wide), U = conj(Q) W^T (tall)
-        run_gemm(plan.qfin_v, w64, w64, V)
-        run_gemm(plan.qfin_u, w64, w64, U)
+        if emu:
+            run_emulated(emu['qv'], w64, w64, V)
+            run_emulated(emu['qu'], w64, w64, U)
+        else:
+            run_gemm(plan.qfin_v, w64, w64, V)
+            run_gemm(plan.qfin_u, w64, w64, U)
 
 
-def _complete(plan, U, V, nz, cplx):
+def _complete(plan, U, V, nz, cplx, emulated=False):
     """Blocked completion of the vectors of small singular values (blocks left by
     yb_svd_finalize): per block, nz candidate vectors with entries uniform in [-1, 1)
     (yb_fill_candidates), projected twice off the k - nz earlier vectors by grouped GEMMs
@@ -632,8 +691,12 @@ def _complete(plan, U, V, nz, cplx):
         (dfill,) = _dev(cp, 'fill', (cp.fill,), dev)
         N.call('yb_fill_candidates', _ptr(G), _ptr(dfill), len(cp.fill), _dtype_code(F.dtype), _stream())
         for _ in range(2):
-            run_gemm(cp.g1, F, G, C)
-            run_gemm(cp.g2, F, C, G, alpha=-1.0, beta=1.0)
+            if emulated and getattr(cp, 'e1', None) is not None:
+                run_emulated(cp.e1, F, G, C)
+                G.sub_(run_emulated(cp.e2, F, C, torch.zeros_like(G)))
+            else:
+                run_gemm(cp.g1, F, G, C)
+                run_gemm(cp.g2, F, C, G, alpha=-1.0, beta=1.0)
         Qc, _ = qr(G, cp.meta, (max(cp.Q, 1), max(cp.R, 1)))
         run_copy(cp.copy, Qc, F)
 
