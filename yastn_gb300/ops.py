@@ -342,7 +342,8 @@ def _autotune_ozaki(plan, A, B, out, slices):
     """Kernel choice for one dot metadata: the mma.sync kernel and the tcgen05 kernel with
     128 x 64 or 128 x 32 tiles produce the same bits, so the first call times the three (CUDA
     events; skipped during stream capture, where the tile-padding estimate decides) and the
-    plan keeps the fastest."""
+    plan keeps the fastest. Inside ``hold_constant_operands`` both operands are split every time,
+    as in a first application."""
     if not OZAKI_AUTOTUNE[0] or torch.cuda.is_current_stream_capturing():
         return plan.prefer_tc
     times = {}
@@ -350,14 +351,14 @@ def _autotune_ozaki(plan, A, B, out, slices):
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         torch.cuda._sleep(2_000_000)  # hold the stream while the host enqueues: time the GPU, not the host
         e0.record()
-        _ozaki_run(plan, A, B, out, slices, tc)
+        _ozaki_run(plan, A, B, out, slices, tc, hold=False)
         e1.record()
         e1.synchronize()
         times[tc] = e0.elapsed_time(e1)  # the second (warm) measurement of each kernel is kept
     return min(times, key=times.get)
 
 
-def _ozaki_run(plan, A, B, out, slices, tc):
+def _ozaki_run(plan, A, B, out, slices, tc, hold=True):
     """Both operands split by one yb_ozaki_split launch (B's blocks read by columns in
     place), then the emulated GEMM: tcgen05 (tile layout) or mma.sync (digit planes). Inside
     ``hold_constant_operands`` an operand split before, unchanged, keeps its digit planes and
@@ -380,26 +381,26 @@ def _ozaki_run(plan, A, B, out, slices, tc):
     # the per-operand group lists travel with the plan's arrays (no upload during a capture)
     darr = _dev(plan, key, arrs + tuple(by_op), dev)
     drec, dgrp, dout, dtl = darr[:4]
-    held_a = _held('split', (id(plan), 0, tile_n, slices), A)
-    held_b = _held('split', (id(plan), 1, tile_n, slices), B)
+    held_a = _held('split', (id(plan), 0, tile_n, slices), A) if hold else None
+    held_b = _held('split', (id(plan), 1, tile_n, slices), B) if hold else None
     hit_a, hit_b = _hit(held_a, A), _hit(held_b, B)
     a_sl, a_ex = hit_a if hit_a else (torch.empty(max(asz, 1), dtype=torch.bfloat16, device=dev),
                                       torch.empty(max(plan.a_exps, 1), dtype=torch.int32, device=dev))
     b_sl, b_ex = hit_b if hit_b else (torch.empty(max(bsz, 1), dtype=torch.bfloat16, device=dev),
                                       torch.empty(max(plan.b_exps, 1), dtype=torch.int32, device=dev))
-    if not hit_a and not hit_b:
+    if hit_a is None and hit_b is None:
         groups, n_groups = dgrp, len(arrs[1])
-    elif hit_a != hit_b:
-        side = 1 if hit_a else 0  # split only the operand that is not held
+    elif hit_a is None or hit_b is None:
+        side = 1 if hit_b is None else 0  # split only the operand that is not held
         groups, n_groups = darr[len(arrs) + side], len(by_op[side])
     else:
         groups, n_groups = None, 0
     if n_groups:
         N.call('yb_ozaki_split', _ptr(A), _ptr(B), _ptr(a_sl), _ptr(b_sl), _ptr(a_ex), _ptr(b_ex), _ptr(drec),
                _ptr(groups), n_groups, slices, st)
-    if held_a is not None and not hit_a:
+    if held_a is not None and hit_a is None:
         _store(held_a, A, (a_sl, a_ex))
-    if held_b is not None and not hit_b:
+    if held_b is not None and hit_b is None:
         _store(held_b, B, (b_sl, b_ex))
     if tile_n:
         N.call('yb_ozaki_gemm_tc', _ptr(a_sl), _ptr(a_ex), _ptr(b_sl), _ptr(b_ex), _ptr(out), _ptr(dout), _ptr(dtl),
