@@ -24,6 +24,7 @@
 // complex rows the phase u = g/|g| of g = <x_p, x_q> = sum_l x_p[l] conj(x_q[l]) is first
 // moved onto x_q, which makes the pair's inner product real, and the real rotation of
 // (|x_p|^2, |x_q|^2, |g|) follows: x_p <- c x_p - s u x_q, x_q <- s x_p + c u x_q (unitary).
+#include <cooperative_groups.h>
 #include "yb_svd_common.cuh"
 
 namespace yb {
@@ -33,39 +34,54 @@ namespace {
 // and scale[b], a power of two that brings the FP32 copy of the block (shift included)
 // below 1 in magnitude, so that FP32 squares and dot products neither overflow nor lose
 // the block to underflow. The rotations, and so W, do not depend on the scale.
+// A cluster of kFroCtas CTAs per block (one SM's FP64 pipe needs 0.5 ms for the 1.7 M squares of a
+// 1296 x 1296 block); the partial sums are added in CTA order.
+constexpr int kFroCtas = 8;
+
 template <typename TI>
-__global__ void block_fro_kernel(const TI* __restrict__ A, const int64_t* __restrict__ blocks,
-                                 double* __restrict__ shift, double* __restrict__ scale,
-                                 int64_t* __restrict__ state) {
+__global__ void __cluster_dims__(kFroCtas, 1, 1)
+    block_fro_kernel(const TI* __restrict__ A, const int64_t* __restrict__ blocks, double* __restrict__ shift,
+                     double* __restrict__ scale, int64_t* __restrict__ state) {
   // QR-preconditioned blocks start the FP32 phase from the rows of R, where small singular
   // values are explicit row norms rather than cancellations: its noise norm is FP64's
   __shared__ double red[32];
-  const int64_t* r = blocks + (int64_t)blockIdx.x * YB_SVD_REC;
+  __shared__ double part;
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
   const int64_t cnt = r[R_M] * r[R_N];
   const TI* a = A + r[R_A];
   double acc = 0.0;
-  for (int64_t e = threadIdx.x; e < cnt; e += blockDim.x) acc += cabs2(a[e]);
+#pragma unroll 4
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < cnt; e += (int64_t)kFroCtas * blockDim.x)
+    acc += cabs2(a[e]);
   acc = warp_sum(acc);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();
   if (threadIdx.x == 0) {
     double tot = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += red[w];
+    part = tot;
+  }
+  cluster.sync();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    double tot = 0.0;
+    for (int c = 0; c < kFroCtas; ++c) tot += *cluster.map_shared_rank(&part, c);
     // ||A||_2 <= ||A||_F: A + shift I is positive definite; +1 keeps an all-zero block regular
     const double fro = sqrt(tot);
     double bound = fro;
     if (shift != nullptr) {
-      shift[blockIdx.x] = fro + 1.0;
+      shift[blockIdx.y] = fro + 1.0;
       bound = 2.0 * fro + 1.0;
     }
     int e = 0;
     if (bound > 0.0 && bound <= 1.0e300) frexp(bound, &e);
-    scale[blockIdx.x] = ldexp(1.0, -e);
+    scale[blockIdx.y] = ldexp(1.0, -e);
     // the FP32 phase works on scale * A, the FP64 phase on A itself
     const double t32 = (r[R_QR] ? kNoise64 : kNoise32) * fro * ldexp(1.0, -e), t64 = kNoise64 * fro;
-    state[(int64_t)blockIdx.x * ST_REC + ST_THR32] = __double_as_longlong(t32 * t32);
-    state[(int64_t)blockIdx.x * ST_REC + ST_THR64] = __double_as_longlong(t64 * t64);
+    state[(int64_t)blockIdx.y * ST_REC + ST_THR32] = __double_as_longlong(t32 * t32);
+    state[(int64_t)blockIdx.y * ST_REC + ST_THR64] = __double_as_longlong(t64 * t64);
   }
+  cluster.sync();  // every CTA's shared memory stays until it has been read
 }
 
 // X32 = scale_b (A or A^H) (+ shift on the diagonal) in FP32, W32 = I; resets the state.
@@ -567,8 +583,8 @@ int launch_block_sweeps(T* work, const int64_t* blocks, int n_blocks, const int3
   return YB_OK;
 }
 
-// One CTA per block: singular values = row norms, sort descending (index tie-break),
-// write U, S, Vh; vectors of zero norm are completed to an orthonormal set.
+// Finalisation: singular values = row norms, sorted descending (index tie-break), U, S, Vh
+// written; vectors of zero norm are completed to an orthonormal set.
 // mode 0: SVD. mode 1/2: Hermitian eigendecomposition of a block shifted by shift[b]
 // (lambda = sigma - shift), eigenvectors = columns of W^H, ordered ascending (1) or by
 // |lambda| descending (2); Vh is not written.
@@ -652,123 +668,167 @@ __global__ void qr_finalize_kernel(const T* __restrict__ work, T* __restrict__ Q
   }
 }
 
+// The finalisation takes three launches: the rows' norms (a warp per row, all SMs) into S, unsorted;
+// the vectors, each CTA gathering 32 positions of the descending order through shared memory (both
+// the reads of X's and W's rows and the writes of U's columns coalesce); S sorted in place and the
+// rows at noise level counted, with their completion, by one CTA per block. Positions are ranks,
+// counted on integer keys (FP64 compares would take the FP64 pipe). As one CTA per block it took
+// 5.3 ms for two 1296 x 1296 blocks.
+
+// Sort key of a value of S (larger keys first): singular values as they are, eigenvalues ascending
+// (mode 1) or by magnitude (mode 2).
+__device__ __forceinline__ unsigned long long final_key(double v, int mode) {
+  const double x = mode == 1 ? 0.0 - v : (mode == 2 ? fabs(v) : v + 0.0);
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  return (long long)b < 0 ? ~b : b | 0x8000000000000000ull;
+}
+
+// Position of key i among the k keys: descending, ties by index.
+__device__ __forceinline__ int final_rank(const unsigned long long* __restrict__ key, int k, int i) {
+  const unsigned long long v = key[i];
+  int rank = 0;
+#pragma unroll 8
+  for (int j = 0; j < i; ++j) rank += key[j] >= v;
+#pragma unroll 8
+  for (int j = i + 1; j < k; ++j) rank += key[j] > v;
+  return rank;
+}
+
 template <typename T>
-__global__ void __launch_bounds__(1024) svd_finalize_kernel(T* __restrict__ work, T* __restrict__ U,
-                                                            double* __restrict__ S, T* __restrict__ Vh,
-                                                            const int64_t* __restrict__ blocks, int pow2,
-                                                            int mode, const double* __restrict__ shift,
-                                                            const int64_t* __restrict__ state,
-                                                            int64_t* __restrict__ n_small) {
-  extern __shared__ unsigned char smem_raw[];
-  // [sig: pow2 doubles][complex: pow2 doubles][idx: pow2 ints]
-  double* sig = reinterpret_cast<double*>(smem_raw);
-  double* cim = sig + pow2;
-  int* idx = reinterpret_cast<int*>(cim + (Num<T>::cplx ? pow2 : 0));
-  __shared__ int n_zero;
-  __shared__ double kmin;
-  const int64_t* r = blocks + (int64_t)blockIdx.x * YB_SVD_REC;
-  const int64_t m = r[R_M], n = r[R_N], k = r[R_K], L = r[R_L];
-  const bool tall = m > n;
+__global__ void svd_norms_kernel(const T* __restrict__ work, double* __restrict__ S, const int64_t* __restrict__ blocks,
+                                 int mode, const double* __restrict__ shift) {
+  const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
+  const int64_t k = r[R_K], L = r[R_L];
   const T* X = work + r[R_X];
-  const T* W = work + r[R_W];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  if (threadIdx.x == 0) n_zero = 0;
-  for (int i = threadIdx.x; i < pow2; i += blockDim.x) {
-    sig[i] = -1.0;  // padding sorts last
-    idx[i] = i;
-  }
-  __syncthreads();
-  for (int64_t i = warp; i < k; i += nw) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = (int64_t)gridDim.x * blockDim.x >> 5;
+  for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < k; i += nw) {
     double acc = 0.0;
+#pragma unroll 4
     for (int64_t l = lane; l < L; l += 32) acc += cabs2(X[i * L + l]);
     acc = warp_sum(acc);
-    if (lane == 0) {
-      const double sv = sqrt(acc);
-      sig[i] = (mode == 0) ? sv : (mode == 1 ? -(sv - shift[blockIdx.x]) : fabs(sv - shift[blockIdx.x]));
+    if (lane == 0) S[r[R_S] + i] = mode == 0 ? sqrt(acc) : sqrt(acc) - shift[blockIdx.y];
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) svd_vectors_kernel(T* __restrict__ work, T* __restrict__ U,
+                                                          const double* __restrict__ S, T* __restrict__ Vh,
+                                                          const int64_t* __restrict__ blocks, int mode,
+                                                          const int64_t* __restrict__ state) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned long long* key = reinterpret_cast<unsigned long long*>(smem_raw);  // [k]
+  __shared__ int row[32];
+  __shared__ double inv[32];
+  __shared__ T tile[32][33];
+  const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
+  const int64_t m = r[R_M], n = r[R_N], k = r[R_K], L = r[R_L];
+  const bool tall = m > n, qr = r[R_QR] != 0;
+  const T* X = work + r[R_X];
+  const T* W = work + r[R_W];
+  T* WS = work + r[R_WS];
+  T* Ub = U + r[R_U];
+  T* Vb = mode == 0 ? Vh + r[R_V] : nullptr;
+  const double* Sb = S + r[R_S];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if ((int64_t)blockIdx.x * 32 >= k) return;
+  const double zthr = mode == 0 && state ? sqrt(__longlong_as_double((long long)state[(int64_t)blockIdx.y * ST_REC + ST_THR64])) : 0.0;
+  for (int i = threadIdx.x; i < k; i += 256) key[i] = final_key(Sb[i], mode);
+  __syncthreads();
+  const int j0 = (int)blockIdx.x * 32, nj = min(32, (int)k - j0);
+  for (int i = threadIdx.x; i < k; i += 256) {
+    const int p = final_rank(key, (int)k, i);
+    if (p >= j0 && p < j0 + 32) {
+      const double sv = Sb[i];
+      row[p - j0] = i;
+      inv[p - j0] = (sv > zthr && sv > 0.0) ? 1.0 / sv : 0.0;
     }
   }
   __syncthreads();
-  if (mode != 0) {
-    // eigh sort keys may be negative: shift them so that the -1 padding still sorts last
-    if (threadIdx.x == 0) {
-      double mn = 0.0;
-      for (int64_t i = 0; i < k; ++i) mn = fmin(mn, sig[i]);
-      kmin = mn;
-    }
-    __syncthreads();
-    for (int64_t i = threadIdx.x; i < k; i += blockDim.x) sig[i] -= kmin;
-    __syncthreads();
-  }
-  // bitonic sort, descending by value, ascending index on ties
-  for (int size = 2; size <= pow2; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < pow2; i += blockDim.x) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const bool up = ((i & size) == 0);
-          const double vi = sig[i], vj = sig[j];
-          const int ii = idx[i], ij = idx[j];
-          const bool i_first = (vi > vj) || (vi == vj && ii < ij);
-          if (up != i_first) {
-            sig[i] = vj; sig[j] = vi;
-            idx[i] = ij; idx[j] = ii;
-          }
-        }
-      }
+  // 32 rows (positions) x 32 entries of a k x len matrix M through the tile: row jj of the tile by
+  // load(jj, l); store(jj, l, v) coalesced along jj (by_column) or along l
+  auto pass = [&](int64_t len, bool by_column, auto load, auto store) {
+    for (int64_t l0 = 0; l0 < len; l0 += 32) {
       __syncthreads();
+      for (int jj = warp; jj < nj; jj += 8)
+        if (l0 + lane < len) tile[jj][lane] = load(jj, l0 + lane);
+      __syncthreads();
+      for (int a = warp; a < 32; a += 8) {
+        const int jj = by_column ? lane : a;
+        const int64_t l = l0 + (by_column ? a : lane);
+        if (jj < nj && l < len) store(jj, l, tile[jj][l - l0]);
+      }
     }
-  }
-  double* Sb = S + r[R_S];
-  T* Ub = U + r[R_U];
-  T* Vb = Vh + r[R_V];
-  if (mode != 0) {
-    for (int64_t j = warp; j < k; j += nw) {
-      const int64_t i = idx[j];
-      double acc = 0.0;
-      for (int64_t l = lane; l < L; l += 32) acc += cabs2(X[i * L + l]);
-      acc = warp_sum(acc);
-      if (lane == 0) Sb[j] = sqrt(acc) - shift[blockIdx.x];
-    }
-    for (int64_t e = threadIdx.x; e < k * k; e += blockDim.x) {
-      const int64_t j = e / k, c = e - j * k;
-      Ub[c * k + j] = cconj_(W[(int64_t)idx[j] * k + c]);
-    }
+  };
+  if (mode != 0) {  // eigenvectors: columns of W^H
+    pass(k, true, [&](int jj, int64_t l) { return cconj_(W[(int64_t)row[jj] * k + l]); },
+         [&](int jj, int64_t l, T v) { Ub[l * k + j0 + jj] = v; });
     return;
-  }
-  // rows at the rounding-noise level were not rotated: their vectors are completed like
-  // those of zero values (the values themselves are kept)
-  const double zthr = state ? sqrt(__longlong_as_double((long long)state[(int64_t)blockIdx.x * ST_REC + ST_THR64]))
-                            : 0.0;
-  for (int j = threadIdx.x; j < k; j += blockDim.x) {
-    Sb[j] = sig[j];
-    if (!(sig[j] > zthr && sig[j] > 0.0)) atomicAdd(&n_zero, 1);
   }
   // wide (X_0 = A): Vh rows = x_j / s_j, U = W^H; tall (X_0 = A^H): U columns = conj(x_j) / s_j,
   // Vh = W. QR-preconditioned (X_0 = R): wide: U columns = x_j / s_j, and the sorted conj(W)
   // goes to WS for Vh = conj(W) Q^T; tall: Vh rows = conj(x_j) / s_j, WS = sorted W for
-  // U = conj(Q) W^T (both products follow as grouped GEMMs).
-  const bool qr = r[R_QR] != 0;
+  // U = conj(Q) W^T (both products follow as GEMMs). Rows at the rounding-noise level were not
+  // rotated: their vectors are zero here and completed like those of zero values.
   const bool to_u = tall != qr;  // the factor built from the rows of X
-  for (int64_t e = threadIdx.x; e < k * L; e += blockDim.x) {
-    const int64_t j = e / L, l = e - j * L;
-    const double sv = sig[j];
-    const T x = X[(int64_t)idx[j] * L + l];
-    T v = (sv > zthr && sv > 0.0) ? rscale(x, 1.0 / sv) : rscale(x, 0.0);
-    if (tall) v = cconj_(v);
-    if (to_u) Ub[l * k + j] = v; else Vb[j * n + l] = v;
-  }
-  T* WS = work + r[R_WS];
-  for (int64_t e = threadIdx.x; e < k * k; e += blockDim.x) {
-    const int64_t j = e / k, c = e - j * k;
-    const T w = W[(int64_t)idx[j] * k + c];
-    if (qr) WS[e] = tall ? w : cconj_(w);
-    else if (tall) Vb[j * n + c] = w;
-    else Ub[c * k + j] = cconj_(w);
+  pass(L, to_u,
+       [&](int jj, int64_t l) {
+         const T v = rscale(X[(int64_t)row[jj] * L + l], inv[jj]);
+         return tall ? cconj_(v) : v;
+       },
+       [&](int jj, int64_t l, T v) {
+         if (to_u) Ub[l * k + j0 + jj] = v; else Vb[(int64_t)(j0 + jj) * n + l] = v;
+       });
+  pass(k, !qr && !tall,
+       [&](int jj, int64_t l) {
+         const T w = W[(int64_t)row[jj] * k + l];
+         return tall ? w : cconj_(w);
+       },
+       [&](int jj, int64_t l, T v) {
+         if (qr) WS[(int64_t)(j0 + jj) * k + l] = v;
+         else if (tall) Vb[(int64_t)(j0 + jj) * n + l] = v;
+         else Ub[l * k + j0 + jj] = v;
+       });
+}
+
+// S sorted in place; for an SVD the rows at noise level counted and small completions done here.
+template <typename T>
+__global__ void __launch_bounds__(1024) svd_finalize_kernel(T* __restrict__ U, double* __restrict__ S,
+                                                            T* __restrict__ Vh, const int64_t* __restrict__ blocks,
+                                                            int mode, const int64_t* __restrict__ state,
+                                                            int64_t* __restrict__ n_small) {
+  extern __shared__ unsigned char smem_raw[];
+  const int64_t* r = blocks + (int64_t)blockIdx.x * YB_SVD_REC;
+  const int64_t m = r[R_M], n = r[R_N], k = r[R_K], L = r[R_L];
+  // [key / real coefficients: k words][values / imaginary coefficients: k doubles]
+  unsigned long long* key = reinterpret_cast<unsigned long long*>(smem_raw);
+  double* sig = reinterpret_cast<double*>(smem_raw);
+  double* cim = sig + k;
+  __shared__ int n_zero;
+  const bool tall = m > n;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  double* Sb = S + r[R_S];
+  T* Ub = U + r[R_U];
+  T* Vb = Vh + r[R_V];
+  if (threadIdx.x == 0) n_zero = 0;
+  for (int i = threadIdx.x; i < k; i += blockDim.x) {
+    const double v = Sb[i];
+    cim[i] = v;
+    key[i] = final_key(v, mode);
   }
   __syncthreads();
-  if (n_zero == 0) return;
+  const double zthr = mode == 0 && state ? sqrt(__longlong_as_double((long long)state[(int64_t)blockIdx.x * ST_REC + ST_THR64]))
+                                         : 0.0;
+  for (int i = threadIdx.x; i < k; i += blockDim.x) {
+    const double v = cim[i];
+    Sb[final_rank(key, (int)k, i)] = v;
+    if (!(v > zthr && v > 0.0)) atomicAdd(&n_zero, 1);
+  }
+  __syncthreads();
+  if (mode != 0 || n_zero == 0) return;
+  const bool to_u = tall != (r[R_QR] != 0);  // the factor built from the rows of X
   // large completions (n_zero k L above 2^22) are left to the host's blocked completion
-  // (random candidates projected with grouped GEMMs and orthonormalised by yb_qr): the count
+  // (random candidates projected with GEMMs and orthonormalised by yb_qr): the count
   // goes to n_small[b] and the vectors stay as written
   if (n_small != nullptr && (double)n_zero * (double)k * (double)L > 4194304.0) {
     if (threadIdx.x == 0) n_small[blockIdx.x] = n_zero;
@@ -958,7 +1018,7 @@ int block_sweeps_t(T* w, const int64_t* blocks, int n_blocks, const int32_t* sup
 template <typename T>
 int qr_t(const void* a, void* work, void* work32, const int64_t* blocks, int n_blocks, int64_t* state, double* scale,
          int64_t* qctrl, int qctrl_words, cudaStream_t s) {
-  if (state) block_fro_kernel<T><<<n_blocks, 256, 0, s>>>((const T*)a, blocks, nullptr, scale, state);
+  if (state) block_fro_kernel<T><<<dim3(kFroCtas, (unsigned)n_blocks), 256, 0, s>>>((const T*)a, blocks, nullptr, scale, state);
   svd_qr_load_kernel<T><<<dim3(64, (unsigned)n_blocks), 256, 0, s>>>((const T*)a, (T*)work, blocks);
   const int st = Num<T>::cplx ? qr_factor_c128(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, s)
                               : qr_factor_f64(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, s);
@@ -968,17 +1028,22 @@ int qr_t(const void* a, void* work, void* work32, const int64_t* blocks, int n_b
 }
 
 template <typename T>
-int finalize_t(void* work, void* U, double* S, void* Vh, const int64_t* blocks, int n_blocks, int pow2,
+int finalize_t(void* work, void* U, double* S, void* Vh, const int64_t* blocks, int n_blocks, int max_k,
                       int mode, const double* shift, const int64_t* state, int64_t* n_small, cudaStream_t s) {
-  const size_t smem = (size_t)pow2 * (sizeof(double) * (Num<T>::cplx ? 2 : 1) + sizeof(int));
-  if (smem > 32 * 1024) {  // with the kernel's static shared memory the total passes 48 KB earlier
-    cudaError_t e = cudaFuncSetAttribute(yb::svd_finalize_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) { yb::set_cuda_error((int)e); return YB_ERR_CUDA; }
+  const size_t keys = (size_t)max_k * sizeof(double), smem = 2 * keys;
+  auto vec = svd_vectors_kernel<T>;
+  auto fin = svd_finalize_kernel<T>;
+  cudaError_t e = cudaSuccess;
+  if (keys > 24 * 1024) {  // with the static shared memory the total may pass 48 KB
+    e = cudaFuncSetAttribute(vec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)keys);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   }
-  yb::svd_finalize_kernel<T><<<n_blocks, 1024, smem, s>>>((T*)work, (T*)U, S, (T*)Vh, blocks, pow2, mode,
-                                                          shift, state, n_small);
-  return yb::check_launch();
+  if (e != cudaSuccess) { set_cuda_error((int)e); return YB_ERR_CUDA; }
+  const unsigned tiles = (unsigned)((max_k + 31) / 32), nb = (unsigned)n_blocks;
+  svd_norms_kernel<T><<<dim3(tiles * 4 < 128 ? tiles * 4 : 128, nb), 256, 0, s>>>((const T*)work, S, blocks, mode, shift);
+  vec<<<dim3(tiles, nb), 256, keys, s>>>((T*)work, (T*)U, S, (T*)Vh, blocks, mode, state);
+  fin<<<nb, 1024, smem, s>>>((T*)U, S, (T*)Vh, blocks, mode, state, n_small);
+  return check_launch();
 }
 
 }  // namespace yb
@@ -993,11 +1058,11 @@ int yb_svd_init(const void* a, void* work32, const int64_t* blocks, int n_blocks
   cudaStream_t s = (cudaStream_t)stream;
   dim3 grid(64, (unsigned)n_blocks);
   if (dtype == YB_F64) {
-    yb::block_fro_kernel<double><<<n_blocks, 256, 0, s>>>((const double*)a, blocks, shift, scale, state);
+    yb::block_fro_kernel<double><<<dim3(yb::kFroCtas, (unsigned)n_blocks), 256, 0, s>>>((const double*)a, blocks, shift, scale, state);
     yb::svd_init_kernel<double, float><<<grid, 256, 0, s>>>((const double*)a, (float*)work32, blocks, state, shift,
                                                             scale);
   } else {
-    yb::block_fro_kernel<double2><<<n_blocks, 256, 0, s>>>((const double2*)a, blocks, shift, scale, state);
+    yb::block_fro_kernel<double2><<<dim3(yb::kFroCtas, (unsigned)n_blocks), 256, 0, s>>>((const double2*)a, blocks, shift, scale, state);
     yb::svd_init_kernel<double2, float2><<<grid, 256, 0, s>>>((const double2*)a, (float2*)work32, blocks, state,
                                                               shift, scale);
   }
@@ -1163,12 +1228,11 @@ int yb_svd_finalize(void* work, void* U, double* S, void* Vh, const int64_t* blo
   if (dtype != YB_F64 && dtype != YB_C128) return YB_ERR_INVALID;
   if (mode < 0 || mode > 2 || (mode != 0 && shift == nullptr)) return YB_ERR_INVALID;
   if (max_k > 8192) return YB_ERR_TOO_LARGE;
-  int pow2 = 1;
-  while (pow2 < max_k) pow2 <<= 1;
+  if (max_k <= 0) return YB_OK;
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype == YB_F64)
-    return yb::finalize_t<double>(work, U, S, Vh, blocks, n_blocks, pow2, mode, shift, state, n_small, s);
-  return yb::finalize_t<double2>(work, U, S, Vh, blocks, n_blocks, pow2, mode, shift, state, n_small, s);
+    return yb::finalize_t<double>(work, U, S, Vh, blocks, n_blocks, max_k, mode, shift, state, n_small, s);
+  return yb::finalize_t<double2>(work, U, S, Vh, blocks, n_blocks, max_k, mode, shift, state, n_small, s);
 }
 
 }  // extern "C"

@@ -660,7 +660,7 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
     _svd_state_check(state, nb, 'FP64', True)
     n_small = torch.zeros(nb, dtype=torch.int64, device=dev) if mode == 0 else None
     N.call('yb_svd_finalize', _ptr(w64), _ptr(U), _ptr(S), _vp(V.data_ptr() if V is not None else 0), _ptr(dblocks),
-           nb, code, plan.max_k, mode, sp, _ptr(state), _vp(n_small.data_ptr() if n_small is not None else 0), st)
+           nb, code, plan.max_k, mode, sp, _ptr(state), _vp(n_small.data_ptr() if n_small is not None else 0), st, launches=3)
     if n_small is not None:
         nz = n_small.cpu().numpy()
         if nz.any():
