@@ -87,12 +87,21 @@ int yb_last_cuda_error(void);
 #define YB_CP_DSTR 24
 #define YB_CP_MAGIC 32
 #define YB_CP_SHIFT 40
+#define YB_BOX_REC 64
 #define YB_COPY_ITEM_UNITS 2048
 #define YB_COPY_TILE 32
 #define YB_COPY_ITEM_TILES 2
 int yb_block_copy(const void* src, void* dst, int unit_bytes,
                   const int64_t* tasks, int n_tasks,
                   const int64_t* items, int n_items, void* stream);
+
+/* Box copies: blocks permuted through shared memory in boxes of t_d elements along each dim, read
+ * in source order and written in destination order. tasks: records of YB_BOX_REC int64, boxes:
+ * int64 triples (source offset, destination offset, clip word) (both: csrc/yb_copy.cu); items:
+ * n_items int32 quadruples (task, first box, number of boxes >= 1, 0), 16-byte aligned, one CTA
+ * each. A box has at most 2048 elements (1024 of 16 bytes). Elements as in yb_block_copy. */
+int yb_box_copy(const void* src, void* dst, int unit_bytes, const int64_t* tasks, const int64_t* boxes,
+                const int32_t* items, int n_items, void* stream);
 
 /* Composed copy: one pass for a chain of block copies (merges, unmerges, transposes, block
  * negations, conjugation) between two GEMMs of a double-layer PEPS contraction.

@@ -228,6 +228,132 @@ def _transpose_task(so, do, sizes, ss, ds):
     return rec
 
 
+BOX_REC = 64
+BOX_MAX_T = 255      # coordinates within a box are bytes
+BOX_PER_CTA = 16     # boxes of one CTA, fewer where that leaves less than BOX_CTAS CTAs
+BOX_CTAS = 608       # four per SM (two at a time)
+BOX_MIN_MIXED = 1 << 20
+BOX_MIN_SCATTER = 1 << 22
+
+
+def _box_elements(elem):
+    """Elements of a box at most (4 per thread of a CTA, 2 of 16 bytes)."""
+    return 2048 if elem < 16 else 1024
+
+
+def _box_task(so, do, sizes, ss, ds, elem):
+    """Box record and table of boxes (source offset, destination offset, clip word) of a collapsed
+    task (yb_box_copy); None if it has no such form. The box grows
+    along the source-contiguous and the destination-contiguous dims until both runs are 256 bytes
+    or the dims end, then on while it fits; extents are evened out."""
+    nd = len(sizes)
+    cap = _box_elements(elem)
+    by_src = sorted(range(nd), key=lambda i: (-ss[i], i))
+    by_dst = sorted(range(nd), key=lambda i: (-ds[i], i))
+
+    def extents(run):
+        t = [1] * nd
+        for order in (by_src, by_dst):
+            got = 1
+            for i in reversed(order):
+                if got >= run:
+                    break
+                t[i] = max(t[i], min(sizes[i], BOX_MAX_T, -(-run // got)))
+                got *= t[i]
+                if t[i] < sizes[i]:
+                    break
+        return t
+    def runs(t):
+        out = []
+        for order in (by_src, by_dst):
+            got = 1
+            for i in reversed(order):
+                got *= t[i]
+                if t[i] < sizes[i]:
+                    break
+            out.append(got)
+        return out
+    # of the boxes for growing run targets the one that moves least: a 32-byte sector more per run on
+    # each side, and the lanes of a pass that stay idle
+    targets = {4, 8, 16, 32, 64}
+    for order in (by_src, by_dst):
+        got = 1
+        for i in reversed(order):
+            targets.update(got * f for f in (1, 2, 3, 4, 6, 8) if f <= sizes[i])
+            got *= sizes[i]
+            targets.add(got)
+    best = None
+    for target in sorted(x for x in targets if 1 < x <= cap):
+        t = [-(-n // -(-n // x)) for n, x in zip(sizes, extents(target))]
+        count = int(np.prod(t, dtype=np.int64))
+        if count <= cap:
+            full = np.prod([-(-n // x) for n, x in zip(sizes, t)], dtype=np.int64) * (-(-count // 512) * 512)
+            cost = sum(32 / (r * elem) for r in runs(t)) + 0.5 * float(full) / float(np.prod(sizes, dtype=np.int64))
+            if best is None or cost < best[0]:
+                best = (cost, t)
+    if best is None:
+        return None
+    t = best[1]
+    clipped = [i for i in range(nd) if sizes[i] % t[i]]
+    if np.prod(t, dtype=np.int64) > cap or len(clipped) > 4 or \
+            any(sum((x - 1) * abs(b) for x, b in zip(t, st)) >= 2 ** 31 for st in (ss, ds)):
+        return None
+    sm, at = [0] * nd, 1
+    for i in reversed(by_src):
+        sm[i], at = at, at * t[i]
+    rec = np.zeros(BOX_REC, dtype=np.int64)
+    rec[0], rec[1] = nd, np.prod(t, dtype=np.int64)
+    for d, i in enumerate(by_src):
+        m, sh = fast_div_consts(t[i])
+        rec[8 + d], rec[16 + d], rec[24 + d], rec[32 + d], rec[40 + d] = t[i], ss[i], ds[i], sm[i], m | (sh << 32)
+        rec[48 + d] = clipped.index(i) if i in clipped else -1
+    for p, i in enumerate(by_dst):
+        rec[56 + p] = by_src.index(i)
+    nt = [-(-sizes[i] // t[i]) for i in by_src]
+    # neighbouring boxes of the table, run by neighbouring CTAs, are neighbours in the source
+    grid = np.indices(nt).reshape(nd, -1) if nd else np.zeros((0, 1), dtype=np.int64)
+    org = grid * np.array([t[i] for i in by_src])[:, None]
+    clip = np.zeros(org.shape[1], dtype=np.int64)
+    for b in range(4):  # bytes without a dim never clip (coordinate 0)
+        lim = np.full(org.shape[1], 255, dtype=np.int64)
+        if b < len(clipped):
+            d = by_src.index(clipped[b])
+            lim = np.minimum(t[clipped[b]], sizes[clipped[b]] - org[d])
+        clip |= lim << (8 * b)
+    table = np.stack([so + (org * np.array([ss[i] for i in by_src])[:, None]).sum(0),
+                      do + (org * np.array([ds[i] for i in by_src])[:, None]).sum(0), clip], axis=1)
+    return rec, table.astype(np.int64)
+
+
+def _by_destination(task):
+    """The task with its dims ordered by the destination's strides (the task itself if they are)."""
+    so, do, sizes, ss, ds = task
+    o = sorted(range(len(sizes)), key=lambda i: (-ds[i], i))
+    if o == list(range(len(sizes))):
+        return task
+    return (so, do) + tuple(_collapse([sizes[i] for i in o], [ss[i] for i in o], [ds[i] for i in o]))
+
+
+def _wants_box(sizes, ss, ds, elem):
+    """Whether a collapsed task goes by boxes: a transposition whose 32 x 32 tiles over its innermost
+    source and destination dims (extents y and x) would be less than half full. Measured, 24 M FP64
+    elements in blocks of (shape, order): (15, 14, 13, 13, 12) 43210 as tiles 408, boxes 154 us; (5, 6,
+    5, 7, 6) 43210 2254 and 197; (19, 18, 17, 20) 3210 252 and 123; but (100, 3, 100, 3) 3210 109 and
+    121, (513, 511) 10 98 and 113. Common innermost runs, and dims of fewer than 4, are copied unit by
+    unit: (15, 14, 13, 13, 12) 02314 68, boxes 148 us."""
+    last = len(sizes) - 1
+    if last < 1 or len(sizes) > CP_MAXD or ds[last] != 1 or ss[last] == 1 or sizes[last] < 4:
+        return False
+    ys = [j for j in range(last) if ss[j] == 1 and sizes[j] >= 4]
+    if not ys:
+        return False
+    x, y, T = sizes[last], sizes[ys[-1]], COPY_TILE
+    tiles = -(-x // T) * -(-y // T)
+    # a block of a single box pays the box's set-up for itself: only where a tile holds little
+    return x * y < 0.5 * T * T * tiles and (x * y < 300 * tiles or
+                                            np.prod(sizes, dtype=np.int64) >= 4 * _box_elements(elem))
+
+
 class CopyPlan:
     """Host copy of a family-(a) plan: tasks, items, element coverage."""
 
@@ -246,9 +372,47 @@ class CopyPlan:
 
     def packed(self, vec_ok):
         """(tasks int64 [n, COPY_REC], items int64 [m, 2]) with 16-byte units where allowed."""
-        if vec_ok in self._packed:
-            return self._packed[vec_ok]
-        recs, items = [], []
+        if vec_ok not in self._packed:
+            self._packed[vec_ok] = self._pack(self._expanded(), vec_ok)
+        return self._packed[vec_ok]
+
+    def packed_with_boxes(self, vec_ok, elem):
+        """(tasks, items, box tasks [n, BOX_REC], boxes [m, 3], box items [l, 4]): the tasks that ``_wants_box`` apart, the others as in ``packed``."""
+        key = ('boxes', vec_ok, elem)
+        if key not in self._packed:
+            rest, recs, tables = [], [], []
+            tasks = self._expanded()
+            # an inverse copy lists its dims in its source's order: unit by unit it reads runs and
+            # scatters them, which beats boxes up to tens of MB (32 MB of FP64; 219 MB: 248 and 150 us)
+            by_dst = [_by_destination(t) for t in tasks]
+            scatter = [t is not u for t, u in zip(tasks, by_dst)]
+            large = sum(int(np.prod(t[2], dtype=np.int64)) for t, x in zip(tasks, scatter) if x) >= BOX_MIN_SCATTER
+            for task, ordered, x in zip(tasks, by_dst, scatter):
+                box = _box_task(*ordered, elem) if (large or not x) and _wants_box(*ordered[2:], elem) else None
+                if box is None:
+                    rest.append(task)
+                    continue
+                recs.append(box[0])
+                tables.append(box[1])
+            # a second launch for the rest is worth it from about a million elements on (below, both
+            # are latency: 8 + 6 us against 8..14)
+            if rest and sum(int(r[1]) * len(x) for r, x in zip(recs, tables)) < BOX_MIN_MIXED:
+                rest, recs, tables = self._expanded(), [], []
+            total = sum(len(x) for x in tables)
+            per = max(1, min(BOX_PER_CTA, total // BOX_CTAS))
+            items, first = [], 0
+            for ti, table in enumerate(tables):
+                for f in range(0, len(table), per):
+                    items.append((ti, first + f, min(per, len(table) - f), 0))
+                first += len(table)
+            if first >= 2 ** 31:
+                raise PlanError("copy plan with more than 2^31 boxes")
+            boxes = np.stack(recs) if recs else np.zeros((0, BOX_REC), dtype=np.int64)
+            tables = np.concatenate(tables) if tables else np.zeros((0, 3), dtype=np.int64)
+            self._packed[key] = self._pack(rest, vec_ok) + (boxes, tables, np.array(items, dtype=np.int32).reshape(-1, 4))
+        return self._packed[key]
+
+    def _expanded(self):
         expanded = []
         for (so, do, sizes, ss, ds) in self.tasks_list:
             sizes, ss, ds = _collapse(sizes, ss, ds)
@@ -262,6 +426,11 @@ class CopyPlan:
                 o_s = so + sum(int(i) * int(x) for i, x in zip(idx, ss[:lead]))
                 o_d = do + sum(int(i) * int(x) for i, x in zip(idx, ds[:lead]))
                 expanded.append((o_s, o_d, sizes[lead:], ss[lead:], ds[lead:]))
+        return expanded
+
+    @staticmethod
+    def _pack(expanded, vec_ok):
+        recs, items = [], []
         for (so, do, sizes, ss, ds) in expanded:
             ti = len(recs)
             tr = _transpose_task(so, do, sizes, ss, ds)
@@ -289,9 +458,7 @@ class CopyPlan:
             recs.append(rec)
             items.extend((ti, f) for f in range(0, count, COPY_ITEM_UNITS))
         tasks = np.stack(recs) if recs else np.zeros((0, COPY_REC), dtype=np.int64)
-        items = np.array(items, dtype=np.int64).reshape(-1, 2)
-        self._packed[vec_ok] = (tasks, items)
-        return self._packed[vec_ok]
+        return tasks, np.array(items, dtype=np.int64).reshape(-1, 2)
 
 
 # ----------------------------------------------------------------------------- merge / unmerge

@@ -90,12 +90,14 @@ def _dev(plan, key, arrays, device):
 def run_copy(plan, src, dst):
     """Run a CopyPlan from ``src`` into ``dst`` (both 1-D, same dtype)."""
     vec_ok = src.dtype == torch.float64 and src.data_ptr() % 16 == 0 and dst.data_ptr() % 16 == 0
-    tasks, items = plan.packed(vec_ok)
-    if len(items) == 0:
-        return dst
-    dt, di = _dev(plan, ('copy', vec_ok), (tasks, items), src.device)
-    N.call('yb_block_copy', _ptr(src), _ptr(dst), src.element_size(), _ptr(dt), len(tasks), _ptr(di), len(items),
-           _stream())
+    elem = src.element_size()
+    tasks, items, box_tasks, boxes, box_items = plan.packed_with_boxes(vec_ok, elem)
+    if len(items):
+        dt, di = _dev(plan, ('copy', vec_ok, elem), (tasks, items), src.device)
+        N.call('yb_block_copy', _ptr(src), _ptr(dst), elem, _ptr(dt), len(tasks), _ptr(di), len(items), _stream())
+    if len(box_items):
+        dt, db, di = _dev(plan, ('boxes', vec_ok, elem), (box_tasks, boxes, box_items), src.device)
+        N.call('yb_box_copy', _ptr(src), _ptr(dst), elem, _ptr(dt), _ptr(db), _ptr(di), len(box_items), _stream())
     return dst
 
 
