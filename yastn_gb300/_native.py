@@ -104,11 +104,16 @@ def lib():
 LAUNCHES = [0]
 
 
+_functions = {}
+
+
 def call(name, *args, launches=1):
     """Call an entry point and raise NativeError on a non-zero status."""
-    L = lib()
-    st = getattr(L, name)(*args)
+    f = _functions.get(name)
+    if f is None:
+        f = _functions[name] = getattr(lib(), name)
+    st = f(*args)
     if st != YB_OK:
-        raise NativeError(name, st, L.yb_last_cuda_error() if st == YB_ERR_CUDA else 0)
+        raise NativeError(name, st, lib().yb_last_cuda_error() if st == YB_ERR_CUDA else 0)
     LAUNCHES[0] += launches
     return st

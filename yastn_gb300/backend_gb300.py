@@ -24,6 +24,7 @@ from functools import reduce
 
 import numpy as np
 import torch
+import torch.autograd.forward_ad as _fwd_ad
 from torch.utils.checkpoint import checkpoint as _checkpoint
 
 from . import ops
@@ -302,34 +303,54 @@ class _FixSigns(torch.autograd.Function):
         return gUi, gVi, None
 
 
+def _apply(fn, tensors, *args):
+    """``fn.apply(*tensors, *args)`` at the host cost that the call needs: Function.apply binds its
+    arguments through inspect.signature (30 us with a merge's metadata). With plain tensors, no
+    torch.func transform, forward-mode level or trace active, what it goes on to do is called
+    directly: the forward alone where nothing requires grad (backend.dot 51 -> 16 us on the host),
+    else the autograd node's own apply. Everything else (wrapped or subclassed tensors included)
+    takes Function.apply."""
+    if (torch._C._are_functorch_transforms_active() or _fwd_ad._current_level >= 0
+            or torch._C._get_tracing_state() is not None):
+        return fn.apply(*tensors, *args)
+    grad = False
+    for t in tensors:
+        if type(t) is not torch.Tensor or torch._C._functorch.is_functorch_wrapped_tensor(t):
+            return fn.apply(*tensors, *args)
+        grad = grad or t.requires_grad
+    if grad and torch.is_grad_enabled():
+        return super(torch.autograd.Function, fn).apply(*tensors, *args)
+    return fn.forward(*tensors, *args)
+
+
 def transpose_and_merge(data, order, meta_new, meta_mrg, Dsize):
-    return _TransposeAndMerge.apply(data, order, meta_new, meta_mrg, Dsize)
+    return _apply(_TransposeAndMerge, (data,), order, meta_new, meta_mrg, Dsize)
 
 
 def unmerge(data, meta):
-    return _Unmerge.apply(data, meta)
+    return _apply(_Unmerge, (data,), meta)
 
 
 def transpose(data, axes, meta_transpose):
-    return _Transpose.apply(data, axes, meta_transpose)
+    return _apply(_Transpose, (data,), axes, meta_transpose)
 
 
 def dot(Adata, Bdata, meta_dot, Dsize):
-    return _Dot.apply(Adata, Bdata, meta_dot, Dsize)
+    return _apply(_Dot, (Adata, Bdata), meta_dot, Dsize)
 
 
 def transpose_dot_sum(Adata, Bdata, meta_dot, Areshape, Breshape, Aorder, Border, Dsize):
-    return _TransposeDotSum.apply(Adata, Bdata, meta_dot, Areshape, Breshape, Aorder, Border, Dsize)
+    return _apply(_TransposeDotSum, (Adata, Bdata), meta_dot, Areshape, Breshape, Aorder, Border, Dsize)
 
 
 def apply_mask(Adata, mask, meta, Dsize, axis, a_ndim):
-    return _ApplyMask.apply(Adata, mask, meta, Dsize, axis, a_ndim)
+    return _apply(_ApplyMask, (Adata,), mask, meta, Dsize, axis, a_ndim)
 
 
 def svd(data, meta, sizes, fullrank_uv=False, ad_decomp_reg=1.0e-12, diagnostics=None, **kwargs):
     if fullrank_uv:
         raise NotImplementedError("yastn_gb300 svd computes the thin SVD (fullrank_uv=False)")
-    return _Svd.apply(data, meta, sizes, fullrank_uv, ad_decomp_reg, diagnostics)
+    return _apply(_Svd, (data,), meta, sizes, fullrank_uv, ad_decomp_reg, diagnostics)
 
 
 def svdvals(data, meta, sizeS, **kwargs):
@@ -341,7 +362,7 @@ def svdvals(data, meta, sizeS, **kwargs):
 
 
 def fix_svd_signs(Udata, Vhdata, meta):
-    return _FixSigns.apply(Udata, Vhdata, meta)
+    return _apply(_FixSigns, (Udata, Vhdata), meta)
 
 
 # ============================================================================ cold bookkeeping
@@ -661,7 +682,7 @@ class _Qr(torch.autograd.Function):
 
 
 def qr(data, meta, sizes):
-    return _Qr.apply(data, meta, sizes)
+    return _apply(_Qr, (data,), meta, sizes)
 
 
 def pinv(A, rcond=None, hermitian=False, out=None, atol=None, rtol=None):
@@ -677,9 +698,9 @@ def eigh(data, meta=None, sizes=(1, 1), order_by_magnitude=False, ad_decomp_reg=
         if data.dim() != 2 or data.shape[1] != D:
             raise ValueError("eigh of a dense matrix needs a square 2-D tensor")
         meta1 = (((0, D * D), (D, D), (0, D * D), (D, D), (0, D)),)
-        S, U = _Eigh.apply(data.reshape(-1), meta1, (D, D * D), order_by_magnitude, ad_decomp_reg)
+        S, U = _apply(_Eigh, (data.reshape(-1),), meta1, (D, D * D), order_by_magnitude, ad_decomp_reg)
         return S, U.reshape(D, D)
-    return _Eigh.apply(data, meta, sizes, order_by_magnitude, ad_decomp_reg)
+    return _apply(_Eigh, (data,), meta, sizes, order_by_magnitude, ad_decomp_reg)
 
 
 @torch.no_grad()

@@ -25,7 +25,7 @@ def _vp(x):
 def _ptr(t):
     if t.is_conj() or t.is_neg():  # a lazy view: its memory is not what the kernels would read
         raise ValueError("yastn_gb300: a conjugate/negative view reached a kernel unresolved")
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _plain(t):
@@ -38,7 +38,9 @@ def _plain(t):
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current device's current stream, as torch.cuda.current_stream().cuda_stream (which wraps
+    it in a Stream object: 3 us on the host against 0.2)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _dtype_code(dtype):
@@ -89,16 +91,30 @@ def _dev(plan, key, arrays, device):
 
 def run_copy(plan, src, dst):
     """Run a CopyPlan from ``src`` into ``dst`` (both 1-D, same dtype)."""
-    vec_ok = src.dtype == torch.float64 and src.data_ptr() % 16 == 0 and dst.data_ptr() % 16 == 0
-    elem = src.element_size()
-    tasks, items, box_tasks, boxes, box_items = plan.packed_with_boxes(vec_ok, elem)
-    if len(items):
-        dt, di = _dev(plan, ('copy', vec_ok, elem), (tasks, items), src.device)
-        N.call('yb_block_copy', _ptr(src), _ptr(dst), elem, _ptr(dt), len(tasks), _ptr(di), len(items), _stream())
-    if len(box_items):
-        dt, db, di = _dev(plan, ('boxes', vec_ok, elem), (box_tasks, boxes, box_items), src.device)
-        N.call('yb_box_copy', _ptr(src), _ptr(dst), elem, _ptr(dt), _ptr(db), _ptr(di), len(box_items), _stream())
+    sp, dp, elem = _ptr(src), _ptr(dst), src.element_size()
+    vec_ok = src.dtype == torch.float64 and (sp | dp) % 16 == 0
+    key = ('copy', vec_ok, elem, src.device)
+    launches = plan._dev.get(key)
+    if launches is None:
+        launches = plan._dev[key] = _copy_launches(plan, vec_ok, elem, src.device)
+    st = _stream()
+    for name, args, _ in launches:
+        N.call(name, sp, dp, elem, *args, st)
     return dst
+
+
+def _copy_launches(plan, vec_ok, elem, device):
+    """(entry point, arguments between the element size and the stream, the device arrays they point
+    into) of a CopyPlan's launches; kept on the plan."""
+    tasks, items, box_tasks, boxes, box_items = plan.packed_with_boxes(vec_ok, elem)
+    out = []
+    if len(items):
+        d = _dev(plan, ('records', vec_ok, elem), (tasks, items), device)
+        out.append(('yb_block_copy', (_ptr(d[0]), len(tasks), _ptr(d[1]), len(items)), d))
+    if len(box_items):
+        d = _dev(plan, ('boxes', vec_ok, elem), (box_tasks, boxes, box_items), device)
+        out.append(('yb_box_copy', (_ptr(d[0]), _ptr(d[1]), _ptr(d[2]), len(box_items)), d))
+    return out
 
 
 def map_gather(src, gmap, conj=False):
@@ -240,23 +256,47 @@ def transpose_backward(data_b, axes, meta_transpose):
 
 # ----------------------------------------------------------------------------- family (b)
 
-def run_gemm(plan, a, b, c, alpha=1.0, beta=0.0):
+def run_gemm(plan, a, b, c, alpha=1.0, beta=0.0, stream=None, keep=None):
+    """C_o = alpha sum op(A) op(B) + beta C_o of a GemmPlan on the current stream, or on ``stream`` (a
+    raw handle): ``keep`` then receives the workspace, to be held until that stream has been waited
+    for."""
     code = _dtype_code(c.dtype)
+    alpha, beta = float(alpha), float(beta)
+    key = ('gemm', a.device)
+    got = plan._dev.get(key)
+    if got is None:
+        got = plan._dev[key] = _gemm_launches(plan, a.device)
+    direct, split, _ = got
+    st = _stream() if stream is None else stream
+    if direct:
+        N.call(direct[0], _ptr(a), _ptr(b), _ptr(c), code, *direct[1], alpha, beta, st)
+    if split:
+        # split-K: chunk products into a workspace, then the ordered sum into C
+        parts, red, size = split
+        ws = torch.empty(size, dtype=c.dtype, device=c.device)
+        if keep is not None:
+            keep.append(ws)
+        N.call('yb_grouped_gemm', _ptr(a), _ptr(b), _ptr(ws), code, *parts, 1.0, 0.0, st)
+        N.call('yb_gemm_reduce', _ptr(c), _ptr(ws), code, *red, alpha, beta, st)
+    return c
+
+
+def _gemm_launches(plan, device):
+    """The launches of a GemmPlan with the addresses of its device arrays (kept on the plan with
+    them): (entry point, records and tiles) or None, the split-K parts or None, the arrays."""
+    direct = split = None
+    keep = []
     if len(plan.tiles):
-        do, dtm, dti = _dev(plan, 'gemm', (plan.outs, plan.terms, plan.tiles), a.device)
-        N.call('yb_grouped_gemm_short' if plan.all_short else 'yb_grouped_gemm', _ptr(a), _ptr(b), _ptr(c), code,
-               _ptr(do), _ptr(dtm), _ptr(dti), len(plan.tiles), float(alpha), float(beta), _stream())
+        d = _dev(plan, 'gemm', (plan.outs, plan.terms, plan.tiles), device)
+        direct = ('yb_grouped_gemm_short' if plan.all_short else 'yb_grouped_gemm',
+                  (_ptr(d[0]), _ptr(d[1]), _ptr(d[2]), len(plan.tiles)))
+        keep.append(d)
     sp = plan.split
     if sp is not None:
-        # split-K: chunk products into a workspace, then the ordered sum into C
-        ws = torch.empty(sp.ws, dtype=c.dtype, device=c.device)
-        do, dtm, dti, dred, dtask = _dev(plan, 'gemm_split', (sp.outs, sp.terms, sp.tiles, sp.red, sp.tasks),
-                                         a.device)
-        N.call('yb_grouped_gemm', _ptr(a), _ptr(b), _ptr(ws), code, _ptr(do), _ptr(dtm), _ptr(dti),
-               len(sp.tiles), 1.0, 0.0, _stream())
-        N.call('yb_gemm_reduce', _ptr(c), _ptr(ws), code, _ptr(dred), _ptr(dtask), len(sp.tasks), float(alpha),
-               float(beta), _stream())
-    return c
+        d = _dev(plan, 'gemm_split', (sp.outs, sp.terms, sp.tiles, sp.red, sp.tasks), device)
+        split = ((_ptr(d[0]), _ptr(d[1]), _ptr(d[2]), len(sp.tiles)), (_ptr(d[3]), _ptr(d[4]), len(sp.tasks)), sp.ws)
+        keep.append(d)
+    return direct, split, keep
 
 
 def promote(A, B):
@@ -319,13 +359,13 @@ def dot_ozaki(A, B, meta_dot, Dsize, slices=OZAKI_SLICES):
     # emulated GEMM, and the current stream waits for them (a fork and join inside a CUDA graph)
     fork = len(plan.native.tiles) > 0 or plan.native.split is not None
     if fork:
-        main, side = torch.cuda.current_stream(A.device), _side_stream(A.device)
+        main, side, keep = torch.cuda.current_stream(A.device), _side_stream(A.device), []
         side.wait_stream(main)
-        with torch.cuda.stream(side):
-            run_gemm(plan.native, A, B, out)
+        run_gemm(plan.native, A, B, out, stream=side.cuda_stream, keep=keep)
     _ozaki_run(plan, A, B, out, slices, tc)
     if fork:
         main.wait_stream(side)
+        del keep  # after the wait: its memory may be given to later work of the main stream
     return out
 
 
@@ -368,48 +408,49 @@ def _ozaki_run(plan, A, B, out, slices, tc, hold=True):
     dev = A.device
     st = _stream()
     tile_n = 0 if not tc else (32 if tc == 32 else 64)
-    if tile_n:
-        # tiles grouped by CTA (one CTA per SM) with balanced work
-        sfx = '_tc' if tile_n == 64 else '_tc32'
-        tiles, offs = P.ozaki_tc_schedule(plan, _sm_count(dev), tile_n)
-        key, arrs = 'ozaki' + sfx, (getattr(plan, 'split_recs' + sfx), getattr(plan, 'split_groups' + sfx),
-                                    getattr(plan, 'outs' + sfx), tiles, offs)
-        asz, bsz = getattr(plan, 'a_size' + sfx), getattr(plan, 'b_size' + sfx)
-        by_op = getattr(plan, 'split_groups' + sfx + '_ab')
-    else:
-        key, arrs = 'ozaki', (plan.split_recs, plan.split_groups, plan.outs, plan.tiles)
-        asz, bsz = plan.a_size, plan.b_size
-        by_op = plan.split_groups_ab
-    # the per-operand group lists travel with the plan's arrays (no upload during a capture)
-    darr = _dev(plan, key, arrs + tuple(by_op), dev)
-    drec, dgrp, dout, dtl = darr[:4]
+    key = ('ozaki', tile_n, dev)
+    rec = plan._dev.get(key)
+    if rec is None:
+        rec = plan._dev[key] = _ozaki_arrays(plan, tile_n, dev)
+    recs, groups_of, gemm, asz, bsz, _ = rec
     held_a = _held('split', (id(plan), 0, tile_n, slices), A) if hold else None
     held_b = _held('split', (id(plan), 1, tile_n, slices), B) if hold else None
     hit_a, hit_b = _hit(held_a, A), _hit(held_b, B)
-    a_sl, a_ex = hit_a if hit_a else (torch.empty(max(asz, 1), dtype=torch.bfloat16, device=dev),
+    a_sl, a_ex = hit_a if hit_a else (torch.empty(asz, dtype=torch.bfloat16, device=dev),
                                       torch.empty(max(plan.a_exps, 1), dtype=torch.int32, device=dev))
-    b_sl, b_ex = hit_b if hit_b else (torch.empty(max(bsz, 1), dtype=torch.bfloat16, device=dev),
+    b_sl, b_ex = hit_b if hit_b else (torch.empty(bsz, dtype=torch.bfloat16, device=dev),
                                       torch.empty(max(plan.b_exps, 1), dtype=torch.int32, device=dev))
-    if hit_a is None and hit_b is None:
-        groups, n_groups = dgrp, len(arrs[1])
-    elif hit_a is None or hit_b is None:
-        side = 1 if hit_b is None else 0  # split only the operand that is not held
-        groups, n_groups = darr[len(arrs) + side], len(by_op[side])
-    else:
-        groups, n_groups = None, 0
+    # both operands, or only the one that is not held
+    groups, n_groups = groups_of[(hit_a is None) + 2 * (hit_b is None)]
+    pa, pae, pb, pbe = _ptr(a_sl), _ptr(a_ex), _ptr(b_sl), _ptr(b_ex)
     if n_groups:
-        N.call('yb_ozaki_split', _ptr(A), _ptr(B), _ptr(a_sl), _ptr(b_sl), _ptr(a_ex), _ptr(b_ex), _ptr(drec),
-               _ptr(groups), n_groups, slices, st)
+        N.call('yb_ozaki_split', _ptr(A), _ptr(B), pa, pb, pae, pbe, recs, groups, n_groups, slices, st)
     if held_a is not None and hit_a is None:
         _store(held_a, A, (a_sl, a_ex))
     if held_b is not None and hit_b is None:
         _store(held_b, B, (b_sl, b_ex))
+    N.call('yb_ozaki_gemm_tc' if tile_n else 'yb_ozaki_gemm', pa, pae, pb, pbe, _ptr(out), *gemm, slices, st)
+
+
+def _ozaki_arrays(plan, tile_n, dev):
+    """Addresses of an emulated dot's device arrays, kept on the plan with them: the split records,
+    the split groups (none; of A; of B; of both) with their counts, the GEMM's arguments between
+    the output and the slice count, and the digit planes' sizes."""
     if tile_n:
-        N.call('yb_ozaki_gemm_tc', _ptr(a_sl), _ptr(a_ex), _ptr(b_sl), _ptr(b_ex), _ptr(out), _ptr(dout), _ptr(dtl),
-               len(arrs[3]), _ptr(darr[4]), len(arrs[4]) - 1, tile_n, slices, st)
+        # tiles grouped by CTA (one CTA per SM) with balanced work
+        sfx = '_tc' if tile_n == 64 else '_tc32'
+        tiles, offs = P.ozaki_tc_schedule(plan, _sm_count(dev), tile_n)
+        sizes = getattr(plan, 'a_size' + sfx), getattr(plan, 'b_size' + sfx)
     else:
-        N.call('yb_ozaki_gemm', _ptr(a_sl), _ptr(a_ex), _ptr(b_sl), _ptr(b_ex), _ptr(out), _ptr(dout), _ptr(dtl),
-               len(arrs[3]), slices, st)
+        sfx, tiles, offs = '', plan.tiles, np.zeros(1, dtype=np.int32)
+        sizes = plan.a_size, plan.b_size
+    ab = getattr(plan, 'split_groups' + sfx + '_ab')
+    arrs = (getattr(plan, 'split_recs' + sfx), getattr(plan, 'split_groups' + sfx), ab[0], ab[1],
+            getattr(plan, 'outs' + sfx), tiles, offs)
+    d = _dev(plan, 'ozaki' + sfx, arrs, dev)
+    groups = ((None, 0), (_ptr(d[2]), len(arrs[2])), (_ptr(d[3]), len(arrs[3])), (_ptr(d[1]), len(arrs[1])))
+    gemm = (_ptr(d[4]), _ptr(d[5]), len(tiles)) + ((_ptr(d[6]), len(offs) - 1, tile_n) if tile_n else ())
+    return _ptr(d[0]), groups, gemm, max(sizes[0], 1), max(sizes[1], 1), d
 
 
 def run_emulated(eg, a, b, c):
