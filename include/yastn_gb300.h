@@ -147,6 +147,12 @@ int yb_map_gather(const void* src, void* dst, int dtype, const int32_t* map, int
 int yb_grouped_gemm(const void* a, const void* b, void* c, int dtype,
                     const int64_t* outs, const int64_t* terms, const int32_t* tiles, int n_tiles,
                     double alpha, double beta, void* stream);
+/* yb_grouped_gemm_fine: the grouped GEMM on 32 x 32 tiles (output, tile row, tile column, 0), for
+ * plans with few 64 x 64 tiles. Output records with [6] = 1 are partial products, written to ws at
+ * [0] without alpha and beta (ws may be null if there is none); yb_gemm_reduce sums them. */
+int yb_grouped_gemm_fine(const void* a, const void* b, void* c, void* ws, int dtype, const int64_t* outs,
+                         const int64_t* terms, const int32_t* tiles, int n_tiles, double alpha, double beta,
+                         void* stream);
 /* yb_grouped_gemm_short: yb_grouped_gemm for plans whose tiles are all of kind 2 (the
  * contractions of a tensor with a small MPO block): a kernel of its own with few registers,
  * eight warps per SM scheduler, all loads of a thread's columns issued before its FMAs. */

@@ -693,7 +693,7 @@ def _pack_gemm(out_list, allow_split=True):
     too few tiles for the GPU, outputs with a long K are split into K chunks computed into
     a workspace and summed by a reduction pass (split-K; not with ``allow_split=False``)."""
     ck = _split_chunk_k(out_list) if allow_split else None
-    split = None
+    split, whole = None, out_list
     if ck is not None:
         direct, parts, red, tasks, ws = [], [], [], [], 0
         for c_off, m, n, ldc, tl in out_list:
@@ -718,7 +718,84 @@ def _pack_gemm(out_list, allow_split=True):
     if split is not None:
         flops += sum(2 * int(o[1]) * int(o[2]) * int(t[2]) for o in split.outs
                      for t in split.terms[int(o[4]):int(o[5])])
-    return GemmPlan(outs, terms, _tiles_for(outs, terms), flops, split)
+    plan = GemmPlan(outs, terms, _tiles_for(outs, terms), flops, split)
+    if allow_split:
+        plan.out_list = whole
+    return plan
+
+
+FINE_TILE = 32           # tiles of yb_grouped_gemm_fine
+FINE_UNITS = 2432        # fine tiles x chunks aimed at (16 per SM: the last ones to finish are short)
+FINE_MIN_K = 24          # shortest K chunk (16 us of an SM at 32 x 32; 13 sectors of 10..129: 32 gives 48 us,
+                         # 24 gives 40, 16 gives 44 with its larger reduction)
+FINE_MIN_LONGEST = 24    # plans whose longest K is shorter are one 64 x 64 step per 16 us: left alone
+
+
+class FineGemm:
+    """The 64 x 64 outputs of a plan on 32 x 32 tiles with K chunks (records, partial-product workspace
+    and reduction), and the plan of the outputs with tiles of other kinds (or None)."""
+
+    def __init__(self, rest, outs, terms, tiles, red, tasks, ws):
+        self.rest, self.outs, self.terms, self.tiles = rest, outs, terms, tiles
+        self.red, self.tasks, self.ws = red, tasks, ws
+        self._dev = {}
+
+
+def fine_gemm(plan):
+    """The FineGemm of ``plan``, or None where it has no 64 x 64 tiles or only short products.
+    Measured against the 64 x 64 tiles (us): sectors of 10..129 140 -> 40, up to 240 251 -> 95, up to
+    422 558 -> 319, up to 704 2246 -> 1994, complex128 up to 129 531 -> 113."""
+    got = plan.__dict__.get('_fine', 0)
+    if got != 0:
+        return got
+    plan._fine = None
+    out_list = plan.__dict__.get('out_list')
+    if out_list is None:
+        return None
+    rest, mine = [], []
+    for o in out_list:
+        kind0 = o[1] and o[2] and tile_kind(o[1], o[2], [t[2] for t in o[4]]) == 0
+        (mine if kind0 else rest).append(o)
+    if max((sum(t[2] for t in o[4]) for o in mine), default=0) < FINE_MIN_LONGEST:
+        return None
+
+    def padded(outputs):  # FMAs as issued: warps of 8 rows x 16 columns
+        return sum(-(-o[1] // 8) * 8 * -(-o[2] // 16) * 16 * sum(t[2] for t in o[4]) for o in outputs)
+    if padded(rest) <= padded(mine) // 4:  # cheaper here than a launch of their own
+        rest, mine = [], [o for o in out_list if o[1] and o[2]]
+
+    def n_tiles(o):
+        return -(-o[1] // FINE_TILE) * -(-o[2] // FINE_TILE)
+    work = sum(n_tiles(o) * sum(t[2] for t in o[4]) for o in mine)
+    ck = max(FINE_MIN_K, -(-work // FINE_UNITS) + 15 & ~15)
+    outs, terms, red, tasks, tiles, ws = [], [], [], [], [], 0
+
+    def add(c_off, m, n, ldc, tl, partial):
+        oi, t0 = len(outs), len(terms)
+        terms.extend(tl)
+        outs.append((c_off, m, n, ldc, t0, len(terms), int(partial), 0))
+        kk = sum(t[2] for t in tl)
+        tiles.extend((kk, oi, tr, tc) for tr in range(-(-m // FINE_TILE)) for tc in range(-(-n // FINE_TILE)))
+    for c_off, m, n, ldc, tl in mine:
+        kk = sum(t[2] for t in tl)
+        nch = max(1, (2 * kk + ck) // (2 * ck))
+        if nch == 1:
+            add(c_off, m, n, ldc, tl, False)
+            continue
+        ch = _chunks(tl, -(-kk // nch) + 15 & ~15)
+        for ci, cl in enumerate(ch):
+            add(ws + ci * m * n, m, n, n, cl, True)
+        tasks.extend((len(red), it) for it in range(-(-m * n // GEMM_RED_ITEM)))
+        red.append((c_off, m, n, ldc, ws, len(ch), 0, 0))
+        ws += len(ch) * m * n
+    tiles.sort(key=lambda x: -x[0])
+    plan._fine = FineGemm(_pack_gemm(rest, allow_split=False) if rest else None,
+                          np.array(outs, dtype=np.int64).reshape(-1, GEMM_OUT_REC),
+                          np.array(terms, dtype=np.int64).reshape(-1, GEMM_TERM_REC),
+                          np.array([(oi, tr, tc, 0) for _, oi, tr, tc in tiles], dtype=np.int32).reshape(-1, 4),
+                          np.array(red, dtype=np.int64).reshape(-1, GEMM_RED_REC),
+                          np.array(tasks, dtype=np.int32).reshape(-1, 2), ws)
+    return plan._fine
 
 
 def dot_coverage(meta_dot):

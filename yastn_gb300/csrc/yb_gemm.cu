@@ -485,6 +485,139 @@ __global__ void __launch_bounds__(kThreads) grouped_gemm_kernel(const typename F
   }
 }
 
+// The general product: 32 x 32 tiles, K cut into chunks where the plan has few of them. An SM issues
+// one warp DFMA per 19 cycles whatever runs on it, so a 64 x 64 tile of K = 128 takes it 135 us: with a
+// few dozen of them most SMs idle, with a few hundred the last ones leave them idle; a fine tile takes
+// a quarter of that per K, and the chunks of a long K are summed afterwards by gemm_reduce_kernel. 256
+// threads, 2 x 2 outputs each (eight warps of 8 rows x 16 columns: warps outside a small sector skip
+// their FMAs), the next 16 k loaded into registers while the current ones are multiplied. Outputs
+// with [6] = 1 go to the workspace as they are (partial products), the others to C with alpha and
+// beta. Bound: the DFMA rate. Measured against 64 x 64 tiles: 13 sectors of 10..129 140 -> 40 us (16 us
+// of FMAs), of 16..704 2246 -> 1994 us, complex128 sectors of 10..129 531 -> 113 us.
+constexpr int kFine = 32;
+
+template <class F>
+__global__ void __launch_bounds__(kThreads) fine_gemm_kernel(const typename F::T* __restrict__ A,
+                                                              const typename F::T* __restrict__ B,
+                                                              typename F::T* __restrict__ C,
+                                                              typename F::T* __restrict__ ws,
+                                                              const int64_t* __restrict__ outs,
+                                                              const int64_t* __restrict__ terms,
+                                                              const int32_t* __restrict__ tiles, double alpha,
+                                                              double beta) {
+  using T = typename F::T;
+  constexpr int kL = kFine * kK / kThreads;  // elements of each operand a thread loads per step
+  __shared__ __align__(16) T As[2][kK][kFine + 2];
+  __shared__ __align__(16) T Bs[2][kK][kFine + 2];
+  const int4 tl = reinterpret_cast<const int4*>(tiles)[blockIdx.x];
+  const int64_t* orec = outs + (int64_t)tl.x * YB_GEMM_OUT_REC;
+  const int64_t c_off = orec[0], m = orec[1], n = orec[2], ldc = orec[3];
+  const int t0 = (int)orec[4], t1 = (int)orec[5];
+  const bool partial = orec[6] != 0;
+  const int64_t row0 = (int64_t)tl.y * kFine, col0 = (int64_t)tl.z * kFine;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ri = (warp >> 1) * 8 + (lane >> 3) * 2, ci = (warp & 1) * 16 + (lane & 7) * 2;
+  const bool active = (row0 + (warp >> 1) * 8 < m) && (col0 + (warp & 1) * 16 < n);
+  T acc[2][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) acc[i][j] = F::zero();
+
+  // step (t, k0): 16 contracted indices of term t from k0 on
+  int t = t0;
+  int64_t k0 = 0;
+  T ra[kL], rb[kL];
+  int kn = 0;        // valid indices of the step in registers
+  bool a_k = true, b_j = true;
+  auto fetch = [&] {
+    const int64_t* trec = terms + (int64_t)t * YB_GEMM_TERM_REC;
+    const int64_t K = trec[2], a_rs = trec[3], a_cs = trec[4], b_rs = trec[5], b_cs = trec[6];
+    const int flags = (int)trec[7];
+    const T* a = A + trec[0];
+    const T* b = B + trec[1];
+    kn = (int)min((int64_t)kK, K - k0);
+    a_k = a_cs == 1;
+    b_j = b_cs == 1 || b_rs != 1;
+#pragma unroll
+    for (int r = 0; r < kL; ++r) {
+      const int e = threadIdx.x + r * kThreads;
+      {
+        const int l = a_k ? e % kK : e / kFine, i = a_k ? e / kK : e % kFine;
+        const bool ok = row0 + i < m && l < kn;
+        ra[r] = ok ? a[(row0 + i) * a_rs + (k0 + l) * a_cs] : F::zero();
+        if (flags & 1) ra[r] = F::conj(ra[r]);
+      }
+      {
+        const int j = b_j ? e % kFine : e / kK, l = b_j ? e / kFine : e % kK;
+        const bool ok = col0 + j < n && l < kn;
+        rb[r] = ok ? b[(k0 + l) * b_rs + (col0 + j) * b_cs] : F::zero();
+        if (flags & 2) rb[r] = F::conj(rb[r]);
+      }
+    }
+    k0 += kK;
+    if (k0 >= K) {
+      k0 = 0;
+      ++t;
+    }
+  };
+  // terms of length zero contribute nothing
+  auto skip_empty = [&] {
+    while (t < t1 && terms[(int64_t)t * YB_GEMM_TERM_REC + 2] <= 0) ++t;
+  };
+  skip_empty();
+  int buf = 0;
+  bool more = t < t1;
+  if (more) fetch();
+  while (more) {
+    const int steps = kn;
+#pragma unroll
+    for (int r = 0; r < kL; ++r) {
+      const int e = threadIdx.x + r * kThreads;
+      if (a_k) As[buf][e % kK][e / kK] = ra[r]; else As[buf][e / kFine][e % kFine] = ra[r];
+      if (b_j) Bs[buf][e / kFine][e % kFine] = rb[r]; else Bs[buf][e % kK][e / kK] = rb[r];
+    }
+    __syncthreads();
+    skip_empty();
+    more = t < t1;
+    if (more) fetch();
+    if (active) {
+#pragma unroll
+      for (int l = 0; l < kK; ++l) {
+        if (l >= steps) break;
+        T a[2], b[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) a[i] = As[buf][l][ri + i];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) b[j] = Bs[buf][l][ci + j];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) F::fma(acc[i][j], a[i], b[j]);
+      }
+    }
+    buf ^= 1;  // the other buffer's readers passed the barrier above
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int64_t gi = row0 + ri + i;
+    if (gi >= m) continue;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int64_t gj = col0 + ci + j;
+      if (gj >= n) continue;
+      if (partial) {
+        ws[c_off + gi * ldc + gj] = acc[i][j];
+      } else {
+        T* p = C + c_off + gi * ldc + gj;
+        T v = alpha == 1.0 ? acc[i][j] : F::scale(acc[i][j], alpha);
+        if (beta != 0.0) v = F::add(v, F::scale(*p, beta));
+        *p = v;
+      }
+    }
+  }
+}
+
 // Split-K reduction: C_o = alpha * sum_{c < chunks} P[p_off + c m n + i n + j] + beta * C_o,
 // the partial products summed in chunk order (deterministic). One CTA per task of
 // YB_GEMM_RED_ITEM consecutive elements of one output.
@@ -526,6 +659,24 @@ extern "C" int yb_gemm_reduce(void* c, const void* p, int dtype, const int64_t* 
   } else if (dtype == YB_C128) {
     yb::gemm_reduce_kernel<yb::Cplx><<<n_tasks, yb::kThreads, 0, s>>>((double2*)c, (const double2*)p, recs,
                                                                       tasks, alpha, beta);
+  } else {
+    return YB_ERR_INVALID;
+  }
+  return yb::check_launch();
+}
+
+extern "C" int yb_grouped_gemm_fine(const void* a, const void* b, void* c, void* ws, int dtype, const int64_t* outs,
+                                    const int64_t* terms, const int32_t* tiles, int n_tiles, double alpha,
+                                    double beta, void* stream) {
+  if (n_tiles == 0) return YB_OK;
+  if (!a || !b || !c || !outs || !terms || !tiles || n_tiles < 0) return YB_ERR_INVALID;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (dtype == YB_F64) {
+    yb::fine_gemm_kernel<yb::Real><<<n_tiles, yb::kThreads, 0, s>>>((const double*)a, (const double*)b, (double*)c,
+                                                                    (double*)ws, outs, terms, tiles, alpha, beta);
+  } else if (dtype == YB_C128) {
+    yb::fine_gemm_kernel<yb::Cplx><<<n_tiles, yb::kThreads, 0, s>>>((const double2*)a, (const double2*)b, (double2*)c,
+                                                                    (double2*)ws, outs, terms, tiles, alpha, beta);
   } else {
     return YB_ERR_INVALID;
   }

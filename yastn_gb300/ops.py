@@ -266,8 +266,19 @@ def run_gemm(plan, a, b, c, alpha=1.0, beta=0.0, stream=None, keep=None):
     got = plan._dev.get(key)
     if got is None:
         got = plan._dev[key] = _gemm_launches(plan, a.device)
-    direct, split, _ = got
+    rest, fine, direct, split, _ = got
     st = _stream() if stream is None else stream
+    if rest is not None:
+        run_gemm(rest, a, b, c, alpha, beta, st, keep)
+    if fine:
+        args, red, size = fine
+        ws = torch.empty(size, dtype=c.dtype, device=c.device) if size else None
+        wp = _ptr(ws) if size else 0
+        N.call('yb_grouped_gemm_fine', _ptr(a), _ptr(b), _ptr(c), wp, code, *args, alpha, beta, st)
+        if size:
+            if keep is not None:
+                keep.append(ws)
+            N.call('yb_gemm_reduce', _ptr(c), wp, code, *red, alpha, beta, st)
     if direct:
         N.call(direct[0], _ptr(a), _ptr(b), _ptr(c), code, *direct[1], alpha, beta, st)
     if split:
@@ -283,9 +294,16 @@ def run_gemm(plan, a, b, c, alpha=1.0, beta=0.0, stream=None, keep=None):
 
 def _gemm_launches(plan, device):
     """The launches of a GemmPlan with the addresses of its device arrays (kept on the plan with
-    them): (entry point, records and tiles) or None, the split-K parts or None, the arrays."""
+    them): the plan of the outputs beside the fine tiles, the fine tiles' arguments, their reduction and
+    workspace; or (entry point, records and tiles) and the split-K parts; the arrays. None where
+    there is none of it."""
     direct = split = None
     keep = []
+    f = P.fine_gemm(plan)
+    if f is not None:
+        d = _dev(f, 'fine', (f.outs, f.terms, f.tiles, f.red, f.tasks), device)
+        return f.rest, ((_ptr(d[0]), _ptr(d[1]), _ptr(d[2]), len(f.tiles)), (_ptr(d[3]), _ptr(d[4]), len(f.tasks)),
+                        f.ws), None, None, [d]
     if len(plan.tiles):
         d = _dev(plan, 'gemm', (plan.outs, plan.terms, plan.tiles), device)
         direct = ('yb_grouped_gemm_short' if plan.all_short else 'yb_grouped_gemm',
@@ -296,7 +314,7 @@ def _gemm_launches(plan, device):
         d = _dev(plan, 'gemm_split', (sp.outs, sp.terms, sp.tiles, sp.red, sp.tasks), device)
         split = ((_ptr(d[0]), _ptr(d[1]), _ptr(d[2]), len(sp.tiles)), (_ptr(d[3]), _ptr(d[4]), len(sp.tasks)), sp.ws)
         keep.append(d)
-    return direct, split, keep
+    return None, None, direct, split, keep
 
 
 def promote(A, B):
