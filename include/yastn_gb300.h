@@ -359,8 +359,13 @@ int yb_svd_widen(const void* work32, void* work64, const int64_t* blocks, int n_
 int yb_svd_ns_prep(void* work64, const int64_t* blocks, int n_blocks, int dtype, int64_t t_delta, void* stream);
 /* T = W D and Wn = D^-1 R (at t_delta and 2 t_delta elements after W) for blocks with a QR start, D
  * the powers of two of a two-sided equilibration of R: the operands of X = W R for a product whose
- * digits are scaled per row and column. X's storage is scratch. Three launches. */
-int yb_svd_scale_wr(void* work64, const int64_t* blocks, int n_blocks, int dtype, int64_t t_delta, void* stream);
+ * digits are scaled per row and column. X's storage is scratch. Three launches. The FP64 noise
+ * norm in state of a block whose R is not finite becomes NaN: yb_svd_poison then writes NaN to its
+ * X (which 0, U = the workspace) or to the factor that comes from Q (which 1). */
+int yb_svd_scale_wr(void* work64, const int64_t* blocks, int n_blocks, int dtype, int64_t t_delta,
+                    int64_t* state, void* stream);
+int yb_svd_poison(void* U, void* V, const int64_t* blocks, int n_blocks, int dtype, const int64_t* state,
+                  int which, void* stream);
 int yb_svd_shift_prefill(void* work64, const int64_t* blocks, int n_blocks, int dtype,
                          const double* shift, void* stream);
 /* yb_svd_qr: the QR-preconditioned start (every block of the records has [16] = 1), in

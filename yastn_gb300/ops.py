@@ -642,14 +642,17 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
     dblocks, dpairs = _dev(plan, 'svd', (plan.blocks, plan.pair_items), dev)
     w64 = torch.empty(plan.n64, dtype=torch.complex128 if cplx else torch.float64, device=dev)
     w32 = torch.empty(plan.n32, dtype=torch.complex64 if cplx else torch.float32, device=dev)
-    state = torch.zeros(SVD_STATE_REC * nb + 4, dtype=torch.int64, device=dev)
+    # control words: [state][state after the FP32 phase][completion counts][QR flags], read once at the
+    # end: the host never waits between the phases
+    n_st, n_qr = SVD_STATE_REC * nb + 4, (nb + 4 * min(nb, 4096)) if plan.qr else 0
+    ctl = torch.zeros(2 * n_st + nb + n_qr, dtype=torch.int64, device=dev)
+    state, qctrl = ctl[:n_st], ctl[2 * n_st + nb:]
+    n_small = ctl[2 * n_st:2 * n_st + nb] if mode == 0 else None
     aux = torch.empty(2 * nb, dtype=torch.float64, device=dev)  # [scale | shift]
     shift = aux[nb:] if mode != 0 else None
     sp = _vp(shift.data_ptr() if shift is not None else 0)
     st = _stream()
-    qctrl = None
     if plan.qr:
-        qctrl = torch.zeros(nb + 4 * min(nb, 4096), dtype=torch.int64, device=dev)
         N.call('yb_svd_qr', _ptr(data), _ptr(w64), _ptr(w32), _ptr(dblocks), nb, code, _ptr(state), _ptr(aux[:nb]),
                _ptr(qctrl), qctrl.numel(), st, launches=4)
     else:
@@ -665,21 +668,17 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
     else:
         N.call('yb_svd_sweeps', _ptr(w32), _ptr(dblocks), nb, _ptr(dpairs), len(plan.pair_items), plan.max_rounds,
                32, code, MAX_SWEEPS32, TOL_STOP32, _ptr(state), st)
-    host = state.cpu()
-    _svd_state_check(host, nb, 'FP32', False)
-    thr64 = np.ascontiguousarray(host.numpy()[5:SVD_STATE_REC * nb:SVD_STATE_REC]).view(np.float64)
-    if qctrl is not None and bool(qctrl[nb + 2::4].any()):
-        raise RuntimeError("yastn_gb300 svd: QR group barrier timed out")
+    ctl[n_st:2 * n_st].copy_(state)
     N.call('yb_svd_widen', _ptr(w32), _ptr(w64), _ptr(dblocks), nb, code, _ptr(state), st)
     w0, t0, n0, ws = plan.w_range
     # The FP64 products of the block SVD run on the tensor cores (57-bit digits per row and column,
     # one rounding per 400 contracted indices; R's grading is taken out of X = W R first): their
     # errors are no larger than the DFMA kernel's, which the FP64 pipe bounds: 2.7 against 0.46 ms
     # for all products of two 432 x 432 blocks, 55 against 3.7 ms for two 1296 x 1296, 0.64 against
-    # 0.10 ms in the eigh of five blocks up to 110. Short products (K < 16) stay native, and so does
-    # a call with a block of non-finite norm, whose NaN and Inf propagate.
+    # 0.10 ms in the eigh of five blocks up to 110. Short products (K < 16) stay native; the results of a
+    # block with a non-finite entry, which digits cannot hold, are made NaN (yb_svd_poison).
     emu = None
-    if SVD_EMULATED[0] and np.isfinite(thr64).all():
+    if SVD_EMULATED[0]:
         emu = P.svd_emulated(plan, OZAKI_SLICES, cplx)
         for gram, ns in (('gram', 'ns'), ('gram2', 'ns2')):
             run_emulated(emu[gram], w64, w64, w64)
@@ -694,8 +693,9 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
             W.copy_(Wn)
     if plan.qr:
         if emu:
-            N.call('yb_svd_scale_wr', _ptr(w64), _ptr(dblocks), nb, code, ws, st, launches=3)
+            N.call('yb_svd_scale_wr', _ptr(w64), _ptr(dblocks), nb, code, ws, _ptr(state), st, launches=3)
             run_emulated(emu['xr'], w64, w64, w64)  # X = W R = T Wn
+            N.call('yb_svd_poison', _ptr(w64), 0, _ptr(dblocks), nb, code, _ptr(state), 0, st)
         else:
             run_gemm(plan.xform, w64, w64, w64)
     elif shift is not None:
@@ -718,21 +718,24 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
     else:
         N.call('yb_svd_sweeps', _ptr(w64), _ptr(dblocks), nb, _ptr(dpairs), len(plan.pair_items), plan.max_rounds,
                64, code, max_sweeps, tol64, _ptr(state), st)
-    _svd_state_check(state, nb, 'FP64', True)
-    n_small = torch.zeros(nb, dtype=torch.int64, device=dev) if mode == 0 else None
-    N.call('yb_svd_finalize', _ptr(w64), _ptr(U), _ptr(S), _vp(V.data_ptr() if V is not None else 0), _ptr(dblocks),
-           nb, code, plan.max_k, mode, sp, _ptr(state), _vp(n_small.data_ptr() if n_small is not None else 0), st, launches=3)
-    if n_small is not None:
-        nz = n_small.cpu().numpy()
-        if nz.any():
-            _complete(plan, U, V, nz, cplx, emu is not None)
+    N.call('yb_svd_finalize', _ptr(w64), _ptr(U), _ptr(S), _ptr(V) if V is not None else 0, _ptr(dblocks), nb, code,
+           plan.max_k, mode, sp, _ptr(state), _ptr(n_small) if n_small is not None else 0, st, launches=3)
     if plan.qr:  # the factor that comes from Q: Vh = conj(W) Q^T (wide), U = conj(Q) W^T (tall)
         if emu:
             run_emulated(emu['qv'], w64, w64, V)
             run_emulated(emu['qu'], w64, w64, U)
+            N.call('yb_svd_poison', _ptr(U), _ptr(V), _ptr(dblocks), nb, code, _ptr(state), 1, st)
         else:
             run_gemm(plan.qfin_v, w64, w64, V)
             run_gemm(plan.qfin_u, w64, w64, U)
+    host = ctl.cpu()
+    _svd_state_check(host[n_st:2 * n_st], nb, 'FP32', False)
+    if plan.qr and bool(host[2 * n_st + nb:][nb + 2::4].any()):
+        raise RuntimeError("yastn_gb300 svd: QR group barrier timed out")
+    _svd_state_check(host[:n_st], nb, 'FP64', True)
+    nz = host[2 * n_st:2 * n_st + nb].numpy()
+    if nz.any():
+        _complete(plan, U, V, nz, cplx, emu is not None)
 
 
 def _complete(plan, U, V, nz, cplx, emulated=False):
@@ -795,7 +798,7 @@ def qr(data, meta, sizes):
     N.call('yb_qr', _ptr(data), _ptr(Q), _ptr(R), _ptr(work), _ptr(dblocks), nb, _dtype_code(data.dtype),
            _ptr(qctrl), qctrl.numel(), _stream(), launches=4)
     run_gemm(plan.right, Q, data, R)
-    if bool(qctrl[nb + 2::4].any()):
+    if bool(qctrl.cpu()[nb + 2::4].any()):
         raise RuntimeError("yastn_gb300 qr: QR group barrier timed out")
     return Q, R
 
