@@ -18,8 +18,8 @@
 // scalars (done by all eight they cost more than the panel's FMAs at L = 100).
 //
 // Measured (GB300; before: a warp per column, one reflector at a time, published by itself): yb_qr
-// of two 540 x 432 blocks 7.8 -> 3.2 ms; yb_svd_qr of two 432 x 432 blocks 6.2 -> 2.8 ms, two
-// 1296 x 1296 62 -> 21 ms (10.6 ms at the DFMA rate), nine of 24..93 0.73 -> 0.47 ms, five complex
+// of two 540 x 432 blocks 7.8 -> 3.1 ms; yb_svd_qr of two 432 x 432 blocks 6.2 -> 2.7 ms, two
+// 1296 x 1296 62 -> 19 ms (10.6 ms at the DFMA rate), nine of 24..93 0.73 -> 0.47 ms, five complex
 // ones of 31 x 24 .. 78 x 60 0.68 -> 0.54 ms; 595 blocks of 42..60 2.6 -> 1.4 ms.
 #pragma once
 #include "yb_svd_common.cuh"
@@ -565,13 +565,13 @@ __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const i
   for (int64_t e = gt; e < k; e += ngt) tau[e] = ldcg_t(V + e * L + e);  // T's diagonal
   if (!grid_barrier(ctrl, group)) return false;
   // Q's columns: row c of Z becomes (H_0 ... H_c e_c)^T, the panels backwards
-  const int64_t gw = (int64_t)rank * kWarps + warp, nwg = (int64_t)group * kWarps;
-  const int64_t c_lo = (int64_t)rank * kWarps;  // this CTA's warps hold columns c_lo + n nwg + (0 .. kWarps - 1)
-  const int64_t top = c_lo < k ? min(k - 1, c_lo + (k - 1 - c_lo) / nwg * nwg + kWarps - 1) : -1;
+  // Columns rank, rank + group, .. of a CTA, dealt to its warps in turn: every CTA has columns of all
+  // panels (with 8 neighbouring columns a CTA, the last of 54 did all 108 panels of k = 432 alone).
+  const int64_t top = rank < k ? rank + (k - 1 - rank) / group * group : -1;
   for (int64_t q = np - 1; q >= 0; --q) {
     if (top < q * kPanel) continue;  // no column of this CTA from this panel on
     const QrPanel<T, VS> p = qr_load_panel<T, VS>(V, L, q, width(q), Vs, sh);
-    for (int64_t c = gw; c < k; c += nwg) {
+    for (int64_t c = rank + (int64_t)group * warp; c < k; c += (int64_t)group * kWarps) {
       if (c < q * kPanel) continue;
       T* x = Z + c * L;
       if (c / kPanel == q) {
