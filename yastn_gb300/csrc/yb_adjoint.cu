@@ -186,41 +186,108 @@ __global__ void qr_copyltu_kernel(double* __restrict__ M, const int64_t* __restr
 }
 
 // B <- B R^{-H} row by row (R upper triangular with a real diagonal): x R^H = b, i.e.
-// x_j = (b_j - sum_{l > j} x_l conj(R_jl)) / R_jj by back substitution, one warp per row, in
-// place. Entries of x already solved are re-read from L2 (written by lane 0 of the same warp,
-// ordered by __syncwarp).
+// x_j = (b_j - sum_{l > j} x_l conj(R_jl)) / R_jj by back substitution, in place. A warp takes a row, a
+// CTA eight; 32 unknowns at a time: lane j sums over the solved ones (32 x 32 tiles of R shared by the
+// CTA's rows, the next tile's loads in flight), then the 32 are solved among themselves, each
+// broadcast to the lanes below it. Bound: the FP64 issue of an SM (rows k^2 / 2 FMAs and, in the
+// chain of 32 solves, four instructions each by all eight warps: 0.35 ms at two blocks of
+// 540 x 432) and the chain's latency. Measured there: 0.73 ms; one unknown at a time, a sum over
+// global memory and a division each, 2.5 ms.
 template <bool Cx>
-__global__ void trsm_rt_kernel(double* __restrict__ B, const double* __restrict__ Rm, const int64_t* __restrict__ recs) {
-  constexpr int W = Cx ? 2 : 1;
+struct TrsmVal {
+  using T = double;
+};
+template <>
+struct TrsmVal<true> {
+  using T = double2;
+};
+__device__ __forceinline__ double trsm_shfl(double v, int s) { return __shfl_sync(0xffffffffu, v, s); }
+__device__ __forceinline__ double2 trsm_shfl(double2 v, int s) {
+  return make_double2(__shfl_sync(0xffffffffu, v.x, s), __shfl_sync(0xffffffffu, v.y, s));
+}
+// acc += x conj(r)
+__device__ __forceinline__ void trsm_fma(double& acc, double x, double r) { acc = fma(x, r, acc); }
+__device__ __forceinline__ void trsm_fma(double2& acc, double2 x, double2 r) {
+  acc.x = fma(x.x, r.x, fma(x.y, r.y, acc.x));
+  acc.y = fma(x.y, r.x, fma(-x.x, r.y, acc.y));
+}
+// v -= x conj(r)
+__device__ __forceinline__ void trsm_fms(double& v, double x, double r) { v = fma(-x, r, v); }
+__device__ __forceinline__ void trsm_fms(double2& v, double2 x, double2 r) {
+  v.x = fma(-x.x, r.x, fma(-x.y, r.y, v.x));
+  v.y = fma(-x.y, r.x, fma(x.x, r.y, v.y));
+}
+__device__ __forceinline__ double trsm_sub(double a, double b) { return a - b; }
+__device__ __forceinline__ double2 trsm_sub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double trsm_re(double a) { return a; }
+__device__ __forceinline__ double trsm_re(double2 a) { return a.x; }
+// v / d from ri = 1 / d: the product corrected by its residual; the division itself where 1 / d leaves
+// the normal numbers (d zero or subnormal, infinite or close to it) and for an infinite quotient
+__device__ __forceinline__ double trsm_div(double v, double d, double ri) {
+  if (!(fabs(ri) < 0x1p1000 && fabs(ri) > 0x1p-1000)) return v / d;
+  const double q = v * ri;
+  return isinf(q) ? q : fma(fma(-q, d, v), ri, q);
+}
+__device__ __forceinline__ double2 trsm_div(double2 v, double d, double ri) {
+  return make_double2(trsm_div(v.x, d, ri), trsm_div(v.y, d, ri));
+}
+
+template <bool Cx>
+__global__ void __launch_bounds__(256) trsm_rt_kernel(double* __restrict__ B, const double* __restrict__ Rm,
+                                                      const int64_t* __restrict__ recs) {
+  using T = typename TrsmVal<Cx>::T;
+  __shared__ T tile[2][32][33];  // [l][j]: R_{J0 + j, l0 + l}
   const int64_t* r = recs + (int64_t)blockIdx.y * YB_QRADJ_REC;
   const int64_t k = r[1], rows = r[3], ldb = r[4], ldr = r[6];
-  double* b = B + W * r[2];
-  const double* R = Rm + W * r[5];
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t row = warp; row < rows; row += nwarps) {
-    double* x = b + W * row * ldb;
-    for (int64_t j = k - 1; j >= 0; --j) {
-      double ar = 0.0, ai = 0.0;
-      for (int64_t l = j + 1 + lane; l < k; l += 32) {
-        if (Cx) {  // x_l conj(R_jl)
-          const double rr = R[2 * (j * ldr + l)], ri = R[2 * (j * ldr + l) + 1];
-          const double xr = __ldcg(x + 2 * l), xi = __ldcg(x + 2 * l + 1);
-          ar = fma(xr, rr, fma(xi, ri, ar));
-          ai = fma(xi, rr, fma(-xr, ri, ai));
-        } else {
-          ar = fma(R[j * ldr + l], __ldcg(x + l), ar);
+  T* b = reinterpret_cast<T*>(B) + r[2];
+  const T* R = reinterpret_cast<const T*>(Rm) + r[5];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const T zero = T{};
+  for (int64_t g0 = (int64_t)blockIdx.x * 8; g0 < rows; g0 += (int64_t)gridDim.x * 8) {
+    const bool live = g0 + warp < rows;
+    T* x = b + (live ? g0 + warp : 0) * ldb;
+    for (int64_t J0 = (k - 1) / 32 * 32; J0 >= 0; J0 -= 32) {
+      const int w = (int)min((int64_t)32, k - J0);
+      // tiles l0 = J0 (the diagonal one, used last) and from J0 + 32 on
+      T reg[4], xn = zero;
+      auto fetch = [&](int64_t l0) {
+        xn = live && l0 + lane < k ? __ldcg(x + l0 + lane) : zero;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int j = warp + 8 * u;
+          reg[u] = (j < w && l0 + lane < k) ? R[(J0 + j) * ldr + l0 + lane] : zero;
         }
+      };
+      auto put = [&](int buf) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) tile[buf][lane][warp + 8 * u] = reg[u];
+      };
+      T acc = zero;
+      int buf = 0;
+      int64_t l0 = J0 + 32 < k ? J0 + 32 : J0;
+      fetch(l0);
+      for (;;) {
+        put(buf);
+        __syncthreads();
+        if (l0 == J0) break;
+        const T xv = xn;
+        l0 = l0 + 32 < k ? l0 + 32 : J0;
+        fetch(l0);
+#pragma unroll 8
+        for (int l = 0; l < 32; ++l) trsm_fma(acc, trsm_shfl(xv, l), tile[buf][l][lane]);
+        buf ^= 1;  // the other buffer's readers passed the barrier above
       }
-      ar = warp_sum(ar);
-      if (Cx) ai = warp_sum(ai);
-      if (lane == 0) {
-        const double d = R[W * (j * ldr + j)];  // real and positive
-        x[W * j] = (__ldcg(x + W * j) - ar) / d;
-        if (Cx) x[2 * j + 1] = (__ldcg(x + 2 * j + 1) - ai) / d;
+      T v = trsm_sub(xn, acc);  // the right-hand side came with the diagonal tile
+      const double d = lane < w ? trsm_re(tile[buf][lane][lane]) : 1.0, ri = 1.0 / d;
+      T sol = zero;
+      for (int j = w - 1; j >= 0; --j) {
+        const T q = trsm_div(v, d, ri);
+        if (lane == j) sol = q;
+        const T xj = trsm_shfl(q, j);
+        if (lane < j) trsm_fms(v, xj, tile[buf][j][lane]);  // R_{J0 + lane, J0 + j}
       }
-      __syncwarp();
+      if (live && lane < w) x[J0 + lane] = sol;
+      __syncthreads();  // the tile's readers, and the row's solved part for its own warp
     }
   }
 }
@@ -242,7 +309,7 @@ extern "C" int yb_qr_adjoint_sym(void* M, const int64_t* recs, int n_blocks, int
 extern "C" int yb_trsm_rt(void* B, const void* R, const int64_t* recs, int n_blocks, int dtype, void* stream) {
   if (n_blocks == 0) return YB_OK;
   if (!B || !R || !recs) return YB_ERR_INVALID;
-  const dim3 grid(32, (unsigned)n_blocks);
+  const dim3 grid(128, (unsigned)n_blocks);
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype == YB_F64) yb::trsm_rt_kernel<false><<<grid, 256, 0, s>>>((double*)B, (const double*)R, recs);
   else if (dtype == YB_C128) yb::trsm_rt_kernel<true><<<grid, 256, 0, s>>>((double*)B, (const double*)R, recs);
