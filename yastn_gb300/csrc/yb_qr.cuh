@@ -1,33 +1,72 @@
 // Blocked Householder QR of all blocks in one cooperative launch (yb_svd_qr, yb_qr).
 //
 // Z holds the columns of M as rows. Groups of CTAs take a block at a time; panels of kPanel
-// columns belong to the CTAs of a group in turn. When panel q is published, every CTA brings its
-// V and T to shared memory and applies I - V T^H V^H to its own later panels; the owner of panel
-// q + 1 takes that one first: its columns live in registers (256 threads, a row of the panel per
-// thread and pass), are updated by panel q, factored, and published through the block's ready
-// counter. The waits are bounded (error word of the group). After the factorisation (a group
-// barrier) R's rows and the FP32 start are written, and every warp forms its own columns of Q by
-// the panels backwards.
+// columns belong to the owners of a group in turn: an owner is a CTA, or for columns of more than
+// kPairRows rows a cluster of two. When panel q is published, every CTA brings its V and T to shared
+// memory and applies I - V T^H V^H to its own later panels; the owner of panel q + 1 takes that one
+// first: its columns live in registers (256 threads a CTA, a row of the panel per thread and pass,
+// V's entries of those rows straight from global memory), are updated by panel q, factored, and
+// published through the block's ready counter. The waits are bounded (error word of the group). After
+// the factorisation (a group barrier) R's rows and the FP32 start are written, and every warp forms
+// its own columns of Q by the panels backwards.
 //
-// What bounds it: the path through the panels (each update and factorisation runs on one SM,
-// whose FP64 pipe issues a warp instruction every 19 cycles, 64 for a single warp) and, for large
-// blocks, the FP64 work of the updates. A panel of w columns costs that path a fixed part (publish,
-// wait, V's load, w reductions and scalars) and FMAs that grow with w^2: w = 4 is the shortest per
-// column by the count of instructions from L = 100 to 2000. A reflector's norm, its inner products
-// with the panel's other columns and those that T needs are one reduction, and one warp does the
-// scalars (done by all eight they cost more than the panel's FMAs at L = 100).
+// What bounds it: the path through the panels (each update and factorisation runs on one or two SMs,
+// whose FP64 pipes issue a warp instruction every 19 cycles, 64 for a single warp: at k = 432 a panel
+// takes 33 k cycles, a quarter each for its steps' inner products, their scalars, and the update
+// before) and, for large blocks, the FP64 work of the updates. A panel of w columns costs that path a
+// fixed part (publish, wait, V's load, w reductions and scalars) and FMAs that grow with w^2: w = 4 is
+// the shortest per column by the count of instructions from L = 100 to 2000. A reflector's norm, its
+// inner products with the panel's other columns and those that T needs are one reduction, and one warp
+// does the scalars (done by all eight they cost more than the panel's FMAs at L = 100).
+//
+// Why kPairRows = 256: a second CTA helps where it has rows to take (the first 256 are the first
+// CTA's), and its barriers cost what it saves around 432 rows: clusters against single CTAs, yb_svd_qr
+// of two 432 x 432 blocks 2.37 / 2.36 ms, yb_qr of two 216 x 432 ones 1.34 / 1.40, two 540 x 432
+// 2.64 / 2.73, yb_svd_qr of two 1296 x 1296 16.6 / 17.0, yb_qr of two 648 x 1296 6.9 / 7.9.
 //
 // Measured (GB300; before: a warp per column, one reflector at a time, published by itself): yb_qr
-// of two 540 x 432 blocks 7.8 -> 3.1 ms; yb_svd_qr of two 432 x 432 blocks 6.2 -> 2.7 ms, two
-// 1296 x 1296 62 -> 19 ms (10.6 ms at the DFMA rate), nine of 24..93 0.73 -> 0.47 ms, five complex
-// ones of 31 x 24 .. 78 x 60 0.68 -> 0.54 ms; 595 blocks of 42..60 2.6 -> 1.4 ms.
+// of two 540 x 432 blocks 7.8 -> 2.6 ms; yb_svd_qr of two 432 x 432 blocks 6.2 -> 2.4 ms, two
+// 1296 x 1296 62 -> 16.6 ms (10.6 ms at the DFMA rate), nine of 24..93 0.73 -> 0.41 ms, five complex
+// ones of 31 x 24 .. 78 x 60 0.68 -> 0.48 ms; 595 blocks of 42..60 2.6 -> 1.4 ms.
 #pragma once
+#include <cooperative_groups.h>
 #include "yb_svd_common.cuh"
 
 namespace yb {
 namespace {
 
 constexpr int kPanel = 4;
+constexpr int kMaxCl = 2;        // CTAs that factor a panel together
+constexpr int64_t kPairRows = 256;  // columns longer than this are taken by kMaxCl CTAs
+
+// The CL CTAs that share a panel are a cluster: barrier, and a store to the same place in all.
+template <int CL>
+__device__ __forceinline__ void qr_sync() {
+  if constexpr (CL == 1) __syncthreads();
+  else cooperative_groups::this_cluster().sync();
+}
+template <int CL, typename T>
+__device__ __forceinline__ void qr_put(T* at, T v) {
+  if constexpr (CL == 1) {
+    *at = v;
+  } else {
+#pragma unroll
+    for (int c = 0; c < CL; ++c) *cooperative_groups::this_cluster().map_shared_rank(at, c) = v;
+  }
+}
+// Whether every CTA of the cluster got through a barrier of the group.
+template <int CL>
+__device__ __forceinline__ bool qr_all(bool ok) {
+  if constexpr (CL > 1) {
+    __shared__ int all[CL];
+    if (threadIdx.x == 0) qr_put<CL>(all + cooperative_groups::this_cluster().block_rank(), (int)ok);
+    qr_sync<CL>();
+#pragma unroll
+    for (int c = 0; c < CL; ++c) ok = ok && all[c];
+    qr_sync<CL>();
+  }
+  return ok;
+}
 
 template <typename T>
 __device__ __forceinline__ T ldcg_t(const T* p) { return __ldcg(p); }
@@ -51,6 +90,25 @@ __device__ __forceinline__ T shfl_xor_t(T v, int o) {
   } else {
     return __shfl_xor_sync(0xffffffffu, v, o);
   }
+}
+
+// Sign and exponent of doubles by integer operations (an FP64 instruction takes a warp 64 cycles).
+__device__ __forceinline__ double neg_if(double v, bool n) {
+  return __longlong_as_double(__double_as_longlong(v) ^ (n ? (long long)(1ull << 63) : 0ll));
+}
+__device__ __forceinline__ double neg_t(double v) { return neg_if(v, true); }
+__device__ __forceinline__ double2 neg_t(double2 v) { return make_double2(neg_if(v.x, true), neg_if(v.y, true)); }
+__device__ __forceinline__ double times_pow2(double v, int e) {  // v normal and v 2^e normal, or v and the result 0
+  const long long b = __double_as_longlong(v);
+  const int x = (int)(b >> 52) & 0x7ff;
+  return x == 0 || x + e <= 0 ? 0.0 : __longlong_as_double(b + ((long long)e << 52));
+}
+// a positive normal double within FP32's range to FP32 (truncated) and back
+__device__ __forceinline__ float trunc32(double v) {
+  return __int_as_float((int)((__double_as_longlong(v) - (896ll << 52)) >> 29));
+}
+__device__ __forceinline__ double widen64(float v) {
+  return __longlong_as_double(((long long)__float_as_int(v) << 29) + (896ll << 52));
 }
 
 // Sums of N values over the warp, N = 4 or 16: the halves are exchanged while there is more than
@@ -96,7 +154,8 @@ __device__ __forceinline__ void qr_wait(const unsigned long long* flag, unsigned
 template <typename T>
 struct QrShared {
   T Tm[kPanel][kPanel];          // T of the panel in Vs: Tm[j][i], j <= i, zero below
-  T part[2][kWarps][kPanel * kPanel];
+  T part[2][kMaxCl * kWarps][kPanel * kPanel];
+  T sum[kPanel * kPanel];        // V^H x of the update before a panel's factorisation
   T row[2][kPanel];              // the panel's row j
   T add[2][kPanel], f[2][kPanel];  // a step's updates: row j of the later columns += add, below x_c += f_c x_i
   T sc[2], diag[2], tau[2];
@@ -144,21 +203,9 @@ __device__ __forceinline__ QrPanel<T, VS> qr_load_panel(const T* __restrict__ V,
   return p;
 }
 
-// x <- (I - V op(T) V^H) x on a row of Z from row kPanel q on; op(T) = T^H (factorisation) or T
-// (forming Q). One warp; nb reflectors (the others are zero in Vs, skipped in global memory).
-template <typename T, bool VS, bool ADJ>
-__device__ __forceinline__ void qr_apply_panel(T* __restrict__ x, const QrPanel<T, VS>& p, int nb, const QrShared<T>& sh,
-                                               int lane) {
-  T w[kPanel];
-#pragma unroll
-  for (int i = 0; i < kPanel; ++i) w[i] = Num<T>::zero();
-#pragma unroll 4
-  for (int l = lane; l < p.len; l += 32) {
-    const T xv = ldcg_t(x + l);
-#pragma unroll
-    for (int i = 0; i < kPanel; ++i)
-      if (VS || i < nb) w[i] = Num<T>::fmac(xv, p.v(i, l), w[i]);
-  }
+// y = - op(T) w for the sums w of a warp's lanes; op(T) = T^H or T.
+template <typename T, bool ADJ>
+__device__ __forceinline__ void qr_apply_t(T (&w)[kPanel], T (&ny)[kPanel], const QrShared<T>& sh, int lane) {
   const T mine = warp_sums<T, kPanel>(w, lane);  // lane l: value l >> 3
   const int i = lane >> 3;
   T y = Num<T>::zero();
@@ -168,12 +215,33 @@ __device__ __forceinline__ void qr_apply_panel(T* __restrict__ x, const QrPanel<
     const T t = ADJ ? Num<T>::conj(sh.Tm[j][i]) : sh.Tm[i][j];
     y = Num<T>::fma_(t, wj, y);
   }
-  T ny[kPanel];
 #pragma unroll
-  for (int j = 0; j < kPanel; ++j) ny[j] = Num<T>::scale(-1, shfl_t(y, 8 * j));
+  for (int j = 0; j < kPanel; ++j) ny[j] = neg_t(shfl_t(y, 8 * j));
+}
+
+// x <- (I - V op(T) V^H) x on a row of Z from row kPanel q on; op(T) = T^H (factorisation) or T
+// (forming Q). One warp; nb reflectors (the others are zero in Vs, skipped in global memory). xs: the
+// warp's room for the row in shared memory, from which the update reads it again (null: not enough):
+// read from global memory twice, the FP64 pipe waits twice (two 1296 x 1296 blocks 18.7 ms instead of
+// 16.6); in registers, the variants by length spill and miss the instruction cache (20.8 ms).
+template <typename T, bool VS, bool ADJ>
+__device__ __forceinline__ void qr_apply_panel(T* __restrict__ x, const QrPanel<T, VS>& p, int nb, const QrShared<T>& sh,
+                                               int lane, T* __restrict__ xs) {
+  T w[kPanel], ny[kPanel];
+#pragma unroll
+  for (int i = 0; i < kPanel; ++i) w[i] = Num<T>::zero();
 #pragma unroll 4
   for (int l = lane; l < p.len; l += 32) {
-    T xv = ldcg_t(x + l);
+    const T xv = ldcg_t(x + l);
+    if (VS && xs) xs[l] = xv;
+#pragma unroll
+    for (int i = 0; i < kPanel; ++i)
+      if (VS || i < nb) w[i] = Num<T>::fmac(xv, p.v(i, l), w[i]);
+  }
+  qr_apply_t<T, ADJ>(w, ny, sh, lane);
+#pragma unroll 4
+  for (int l = lane; l < p.len; l += 32) {
+    T xv = VS && xs ? xs[l] : ldcg_t(x + l);
 #pragma unroll
     for (int j = 0; j < kPanel; ++j)
       if (VS || j < nb) xv = Num<T>::fma_(ny[j], p.v(j, l), xv);
@@ -185,60 +253,70 @@ __device__ __forceinline__ void qr_apply_panel(T* __restrict__ x, const QrPanel<
 // The reflector of a column from alpha (its entry on the diagonal) and xn = |x below|^2 (LAPACK
 // larfg: beta real, tau = (beta - alpha) / beta, v = x / (alpha - beta) with v_0 = 1); a column
 // that is already reduced gets tau = 0, sc = 0. With s = |beta|: tau = 1 + |Re alpha| / s (and
-// sign(Re alpha) Im alpha / s), 1 / (alpha - beta) = conj(alpha - beta) / ((s + |Re alpha|)^2 + (Im alpha)^2).
-// The square root and the two reciprocals are refined from FP32 starts (about 20 FP64
-// instructions instead of 60; the FP64 pipe issues one per 64 cycles and warp); norms whose
-// squares leave 2^+-900 take the library's.
+// sign(Re alpha) Im alpha / s), 1 / (alpha - beta) = conj(alpha - beta) / ((s + |Re alpha|)^2 + (Im alpha)^2);
+// ts = conj(tau sc) = -1 / beta.
+// All panels wait for this chain: 12 FP64 instructions of 64 cycles for a real column (the square
+// root and the reciprocal by one third-order step each from an FP32 start, scalings and signs by
+// integers) instead of 28; 2.7 k -> 1.6 k cycles a column with the updates' factors. Norms whose squares
+// leave 2^+-900 take the library's functions.
 template <typename T>
-__device__ __forceinline__ void qr_scalars(T alpha, double xn, T& tau, T& sc, T& diag) {
+__device__ __forceinline__ void qr_scalars(T alpha, double xn, T& tau, T& sc, T& diag, double& ts) {
   double ar, ai;
   if constexpr (Num<T>::cplx) { ar = alpha.x; ai = alpha.y; } else { ar = alpha; ai = 0.0; }
   if (xn == 0.0 && ai == 0.0) {
     tau = Num<T>::zero();
     sc = Num<T>::zero();
     diag = alpha;
+    ts = 0.0;
     return;
   }
   const double n2 = Num<T>::cplx ? fma(ar, ar, fma(ai, ai, xn)) : fma(ar, ar, xn);
-  // s = sqrt(n2), 1 / s, 1 / (s + |ar|); complex: re and im = (s + |ar|, ai) / ((s + |ar|)^2 + ai^2)
-  double s, is, id, fi = 0.0;
+  const bool ng = __double_as_longlong(ar) < 0;  // the sign of Re alpha, of -0 too
+  // s = sqrt(n2), is = 1 / s, t1 = |ar| / s + 1, id = 1 / (s + |ar|); complex: id and fi = (s + |ar|, ai) / ((s + |ar|)^2 + ai^2)
+  double s, is, t1, id, fi = 0.0;
   const int ex = (int)((__double_as_longlong(n2) >> 52) & 0x7ff) - 1023;
   if (ex > -900 && ex < 900) {
     const int h = ex >> 1;  // n2 = m 4^h, m in [1, 4)
-    const double dn = __longlong_as_double((long long)(1023 - h) << 52), up = __longlong_as_double((long long)(1023 + h) << 52);
-    const double m = n2 * dn * dn;
-    const double y0 = (double)rsqrtf((float)m);
-    const double e = fma(-m * y0, y0, 1.0);
-    const double y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
-    double q = m * y;
-    q = fma(0.5 * y, fma(-q, q, m), q);
-    const double d1 = fma(fabs(ar), dn, q);  // in [1, 4)
-    const double im = ai * dn;
+    const double m = times_pow2(n2, -2 * h), a1 = times_pow2(neg_if(ar, ng), -h);
+    const double y0 = widen64(rsqrtf(trunc32(m)));
+    const double q0 = m * y0;
+    const double e = fma(-q0, y0, 1.0);
+    const double t = e * fma(e, 0.375, 0.5);
+    const double y = fma(y0, t, y0), q = fma(q0, t, q0);  // 1 / sqrt(m), sqrt(m)
+    const double d1 = q + a1;  // in [1, 4)
+    t1 = fma(a1, y, 1.0);
+    const double im = Num<T>::cplx ? times_pow2(ai, -h) : 0.0;
     const double d = Num<T>::cplx ? fma(d1, d1, im * im) : d1;
-    double z = (double)(1.f / (float)d);
-    z = fma(z, fma(-d, z, 1.0), z);
-    z = fma(z, fma(-d, z, 1.0), z);
-    s = q * up;
-    is = y * dn;
-    id = (Num<T>::cplx ? z * d1 : z) * dn;
-    fi = im * z * dn;
+    double z = widen64(__frcp_rn(trunc32(d)));
+    const double ez = fma(-d, z, 1.0);
+    z = fma(z, fma(ez, ez, ez), z);
+    s = times_pow2(q, h);
+    is = times_pow2(y, -h);
+    id = times_pow2(Num<T>::cplx ? z * d1 : z, -h);
+    if constexpr (Num<T>::cplx) fi = times_pow2(im * z, -h);
   } else {
     s = sqrt(n2);
     is = 1.0 / s;
+    t1 = fma(fabs(ar), is, 1.0);
     const double t = ai / (s + fabs(ar));
     id = 1.0 / ((s + fabs(ar)) * fma(t, t, 1.0));
     fi = t * id;
   }
-  const double sg = copysign(1.0, ar);
+  ts = neg_if(is, ng);
   if constexpr (Num<T>::cplx) {
-    tau = make_double2(fma(fabs(ar), is, 1.0), sg * ai * is);
-    sc = make_double2(sg * id, -fi);
-    diag = make_double2(-sg * s, 0.0);
+    tau = make_double2(t1, ai * ts);
+    sc = make_double2(neg_if(id, ng), neg_if(fi, true));
+    diag = make_double2(neg_if(s, !ng), 0.0);
   } else {
-    tau = fma(fabs(ar), is, 1.0);
-    sc = sg * id;
-    diag = -sg * s;
+    tau = t1;
+    sc = neg_if(id, ng);
+    diag = neg_if(s, !ng);
   }
+}
+
+__device__ __forceinline__ double qr_fma_re(double a, double x, double acc) { return fma(a, x, acc); }
+__device__ __forceinline__ double2 qr_fma_re(double a, double2 x, double2 acc) {
+  return make_double2(fma(a, x.x, acc.x), fma(a, x.y, acc.y));
 }
 
 // Column i of T from tau and S_ci = v_c^H v_i, c < i: T_ci = -tau sum_{c <= d < i} T_cd S_di.
@@ -251,7 +329,7 @@ __device__ __forceinline__ void qr_t_column(T (&Tm)[kPanel][kPanel], const T (&S
 #pragma unroll
     for (int d = 0; d < kPanel; ++d)
       if (d >= c && d < i) a = Num<T>::fma_(Tm[c][d], S[d], a);
-    Tm[c][i] = Num<T>::scale(-1, Num<T>::mul(tau, a));
+    Tm[c][i] = neg_t(Num<T>::mul(tau, a));
   }
   Tm[i][i] = tau;
 }
@@ -260,72 +338,95 @@ __device__ __forceinline__ void qr_t_column(T (&Tm)[kPanel][kPanel], const T (&S
 // rows from l0 on lie in registers: thread t holds rows l0 + t + 256 r, r < R (warps whose rows lie
 // beyond the column do no arithmetic: the FP64 pipe is shared). Writes R's entries to Z and the
 // reflectors and T to V. Warp 0 does a step's scalars, the last warp T's columns.
-template <typename T, bool VS, int R>
+template <typename T, bool VS, int R, int CL>
 __device__ __forceinline__ void qr_factor_panel(T* __restrict__ Z, T* __restrict__ V, int64_t L, int64_t next, int nb,
                                                 QrPanel<T, VS>& p, T* Vs, QrShared<T>& sh,
                                                 const unsigned long long* ready, unsigned long long* err) {
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  constexpr int kT = CL * kThreads, kW = CL * kWarps;
+  const int crank = CL == 1 ? 0 : (int)cooperative_groups::this_cluster().block_rank();
+  const int t = threadIdx.x + crank * kThreads, lane = t & 31, gwarp = t >> 5, warp = threadIdx.x >> 5;
   const bool has_p = next > 0;
   const int64_t c0 = next * kPanel, l0 = has_p ? c0 - kPanel : 0;
   const int off = (int)(c0 - l0), len = (int)(L - l0);
-  const int live = (len - 32 * warp + kThreads - 1) / kThreads;  // passes with rows of this warp (may be <= 0)
-  __syncthreads();  // the columns as this CTA's warps left them
+  const int live = (len - 32 * gwarp + kT - 1) / kT;  // passes with rows of this warp (may be <= 0)
+  qr_sync<CL>();  // the columns as the warps left them
   T x[R][kPanel];
 #pragma unroll
   for (int r = 0; r < R; ++r)
 #pragma unroll
     for (int c = 0; c < kPanel; ++c) {
-      const int l = t + kThreads * r;
+      const int l = t + kT * r;
       x[r][c] = (l < len && c < nb) ? ldcg_t(Z + (c0 + c) * L + l0 + l) : Num<T>::zero();
     }
   if (has_p) {
     qr_wait(ready, (unsigned long long)next, err);
-    p = qr_load_panel<T, VS>(V, L, next - 1, kPanel, Vs, sh);
+    // V's entries of the thread's rows in registers where they fit, else the panel in shared memory
+    // (else the caller brings it there afterwards)
+    constexpr bool kRegs = R * (int)sizeof(T) <= 48;
+    const T* g = V + l0 * (L + 1);
+    const int yi = (lane & 15) >> 2, yc = lane & 3;
+    T v[kRegs ? R : 1][kPanel], tm[kPanel];
+    if constexpr (kRegs) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int i = 0; i < kPanel; ++i) {
+          const int l = t + kT * r;
+          v[r][i] = l >= len || l < i ? Num<T>::zero() : l == i ? Num<T>::one() : __ldcg(g + i * L + l);
+        }
+    } else {
+      p = qr_load_panel<T, VS>(V, L, next - 1, kPanel, Vs, sh);
+    }
+#pragma unroll
+    for (int j = 0; j < kPanel; ++j) tm[j] = j <= yi ? __ldcg(g + yi * L + j) : Num<T>::zero();
+    auto entry = [&](int r, int i) {
+      if constexpr (kRegs) return v[r][i];
+      const int l = t + kT * r;
+      return l < len ? p.v(i, l) : Num<T>::zero();
+    };
     T w[kPanel * kPanel];
 #pragma unroll
     for (int e = 0; e < kPanel * kPanel; ++e) w[e] = Num<T>::zero();
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int l = t + kThreads * r;
+    for (int r = 0; r < R; ++r)
       if (r < live) {
 #pragma unroll
         for (int i = 0; i < kPanel; ++i) {
-          const T v = l < len ? p.v(i, l) : Num<T>::zero();
+          const T ve = entry(r, i);
 #pragma unroll
-          for (int c = 0; c < kPanel; ++c) w[i * kPanel + c] = Num<T>::fmac(x[r][c], v, w[i * kPanel + c]);
+          for (int c = 0; c < kPanel; ++c) w[i * kPanel + c] = Num<T>::fmac(x[r][c], ve, w[i * kPanel + c]);
         }
       }
-    }
     T mine = Num<T>::zero();
     if (live > 0) mine = warp_sums<T, kPanel * kPanel>(w, lane);  // lane l: value l >> 1
-    if (!(lane & 1)) sh.part[0][warp][lane >> 1] = mine;
+    if (!(lane & 1)) qr_put<CL>(&sh.part[0][gwarp][lane >> 1], mine);
+    qr_sync<CL>();
+    // the warps' sums: 32 / kW values a warp, then y_ic = sum_j conj(T_ji) w_jc at lane 4 i + c
+    if (warp < kW / 2) {
+      const int e = (lane + 32 * warp) / kW;
+      T s = sh.part[0][lane % kW][e];
+#pragma unroll
+      for (int o = kW / 2; o >= 1; o >>= 1) s = Num<T>::add(s, shfl_xor_t(s, o));
+      if (lane % kW == 0) sh.sum[e] = s;
+    }
     __syncthreads();
     if (live > 0) {
-      // lane l < 16 (and l + 16): value l, warps 4 h .. 4 h + 3
-      T s = Num<T>::zero();
-#pragma unroll
-      for (int u = 0; u < kWarps / 2; ++u) s = Num<T>::add(s, sh.part[0][(lane >> 4) * (kWarps / 2) + u][lane & 15]);
-      s = Num<T>::add(s, shfl_xor_t(s, 16));
-      // y_ic = sum_j conj(T_ji) w_jc at lane 4 i + c
-      const int i = (lane & 15) >> 2, c = lane & 3;
       T y = Num<T>::zero();
 #pragma unroll
-      for (int j = 0; j < kPanel; ++j) y = Num<T>::fma_(Num<T>::conj(sh.Tm[j][i]), shfl_t(s, 4 * j + c), y);
-      y = Num<T>::scale(-1, y);
+      for (int j = 0; j < kPanel; ++j) y = Num<T>::fma_(Num<T>::conj(tm[j]), sh.sum[4 * j + yc], y);
+      y = neg_t(y);
 #pragma unroll
       for (int j = 0; j < kPanel; ++j) {
         T ny[kPanel];
 #pragma unroll
         for (int cc = 0; cc < kPanel; ++cc) ny[cc] = shfl_t(y, 4 * j + cc);
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int l = t + kThreads * r;
+        for (int r = 0; r < R; ++r)
           if (r < live) {
-            const T v = l < len ? p.v(j, l) : Num<T>::zero();
+            const T ve = entry(r, j);
 #pragma unroll
-            for (int cc = 0; cc < kPanel; ++cc) x[r][cc] = Num<T>::fma_(ny[cc], v, x[r][cc]);
+            for (int cc = 0; cc < kPanel; ++cc) x[r][cc] = Num<T>::fma_(ny[cc], ve, x[r][cc]);
           }
-        }
       }
     }
   }
@@ -351,15 +452,17 @@ __device__ __forceinline__ void qr_factor_panel(T* __restrict__ Z, T* __restrict
       }
     if (t == off + i) {
 #pragma unroll
-      for (int c = 0; c < kPanel; ++c) sh.row[b][c] = x[0][c];
+      for (int c = 0; c < kPanel; ++c) qr_put<CL>(&sh.row[b][c], x[0][c]);
     }
     T mine = Num<T>::zero();
     if (live > 0) mine = warp_sums<T, kPanel>(a, lane);  // lane l: value l >> 3
-    if (!(lane & 7)) sh.part[b][warp][lane >> 3] = mine;
-    __syncthreads();
+    if (!(lane & 7)) qr_put<CL>(&sh.part[b][gwarp][lane >> 3], mine);
+    qr_sync<CL>();
     T s = Num<T>::zero();
     if (warp == 0 || warp == kWarps - 1) {
       s = sh.part[b][lane & 7][lane >> 3];
+#pragma unroll
+      for (int u = 1; u < CL; ++u) s = Num<T>::add(s, sh.part[b][(lane & 7) + u * kWarps][lane >> 3]);
 #pragma unroll
       for (int o = 4; o >= 1; o >>= 1) s = Num<T>::add(s, shfl_xor_t(s, o));  // lane l: total l >> 3
     }
@@ -368,10 +471,10 @@ __device__ __forceinline__ void qr_factor_panel(T* __restrict__ Z, T* __restrict
       double xn;
       if constexpr (Num<T>::cplx) xn = d.x; else xn = d;
       T tau, sc, diag;
-      qr_scalars<T>(sh.row[b][i], xn, tau, sc, diag);
+      double ts;
+      qr_scalars<T>(sh.row[b][i], xn, tau, sc, diag, ts);
       // x_c -= conj(tau) (v^H x_c) v, v = sc x_i below row j; lane 8 c
-      const T w = Num<T>::fma_(Num<T>::conj(sc), s, sh.row[b][lane >> 3]);
-      const T g = Num<T>::scale(-1, Num<T>::mul(Num<T>::conj(tau), w));
+      const T g = neg_t(qr_fma_re(ts, s, Num<T>::mul(Num<T>::conj(tau), sh.row[b][lane >> 3])));
       const T f = Num<T>::mul(g, sc);
       if (!(lane & 7)) {
         sh.add[b][lane >> 3] = g;
@@ -405,7 +508,7 @@ __device__ __forceinline__ void qr_factor_panel(T* __restrict__ Z, T* __restrict
       }
     }
   }
-  if (t == kThreads - 1) {
+  if (threadIdx.x == kThreads - 1) {
 #pragma unroll
     for (int i = 0; i < kPanel; ++i)
 #pragma unroll
@@ -416,7 +519,7 @@ __device__ __forceinline__ void qr_factor_panel(T* __restrict__ Z, T* __restrict
   for (int r = 0; r < R; ++r)
 #pragma unroll
     for (int c = 0; c < kPanel; ++c) {
-      const int l = t + kThreads * r;
+      const int l = t + kT * r;
       if (l >= len || c >= nb) continue;
       const int64_t at = (c0 + c) * L + l0 + l;
       if (r == 0 && t <= off + c) {
@@ -435,7 +538,7 @@ __device__ void qr_factor_panel_long(T* __restrict__ Z, T* __restrict__ V, int64
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t c0 = next * kPanel;
   T* z = Z + (c0 + warp) * L;
-  if (has_p && warp < nb) qr_apply_panel<T, VS, true>(z + c0 - kPanel, p, kPanel, sh, lane);
+  if (has_p && warp < nb) qr_apply_panel<T, VS, true>(z + c0 - kPanel, p, kPanel, sh, lane, (T*)nullptr);
   __syncthreads();
   T Tm[kPanel][kPanel];
 #pragma unroll
@@ -465,14 +568,15 @@ __device__ void qr_factor_panel_long(T* __restrict__ Z, T* __restrict__ V, int64
     const T ti = sh.part[0][0][i];
     if constexpr (Num<T>::cplx) xn = ti.x; else xn = ti;
     T tau, sc, diag, S[kPanel];
-    qr_scalars<T>(sh.row[0][i], xn, tau, sc, diag);
+    double ts;
+    qr_scalars<T>(sh.row[0][i], xn, tau, sc, diag, ts);
 #pragma unroll
     for (int c = 0; c < kPanel; ++c)
       S[c] = c < i ? Num<T>::fma_(sc, sh.part[0][0][c], Num<T>::conj(sh.row[0][c])) : Num<T>::zero();
     qr_t_column<T>(Tm, S, tau, i);
     if (warp > i && warp < nb) {
-      const T w = Num<T>::fma_(Num<T>::conj(sc), sh.part[0][0][warp], sh.row[0][warp]);
-      const T g = Num<T>::scale(-1, Num<T>::mul(Num<T>::conj(tau), w)), f = Num<T>::mul(g, sc);
+      const T g = neg_t(qr_fma_re(ts, sh.part[0][0][warp], Num<T>::mul(Num<T>::conj(tau), sh.row[0][warp])));
+      const T f = Num<T>::mul(g, sc);
       for (int64_t l = j + 1 + lane; l < L; l += 32) z[l] = Num<T>::fma_(f, ldcg_t(xi + l), ldcg_t(z + l));
       if (lane == 0) z[j] = Num<T>::add(sh.row[0][warp], g);
     }
@@ -495,10 +599,10 @@ __device__ void qr_factor_panel_long(T* __restrict__ Z, T* __restrict__ V, int64
 
 // All steps of block r for the CTAs of a group (VS: the panels' V fits in shared memory; MAXR:
 // passes of 256 rows a panel may take in registers). False after a barrier timeout.
-template <typename T, typename T32, int MAXR, bool VS>
+template <typename T, typename T32, int MAXR, bool VS, int CL>
 __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const int64_t* __restrict__ r, int group, int rank,
                          unsigned long long* ready, unsigned long long* ctrl, const double* scale_b, T* Vs,
-                         QrShared<T>& sh) {
+                         int smem_elems, QrShared<T>& sh) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t gt = (int64_t)rank * kThreads + threadIdx.x, ngt = (int64_t)group * kThreads;
   const int64_t k = r[R_K], L = r[R_LQ];
@@ -507,20 +611,24 @@ __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const i
   T* tau = work + r[R_TAU];
   T* RR = work + r[R_RR];
   const int64_t np = (k + kPanel - 1) / kPanel;
+  T* xs = VS && (kPanel + kWarps) * L <= smem_elems ? Vs + (kPanel + warp) * L : nullptr;
   auto width = [&](int64_t q) { return (int)min((int64_t)kPanel, k - q * kPanel); };
-  // factorisation: panel q applied to this CTA's later panels, panel q + 1 factored by its owner
+  // factorisation: panel q applied to the later panels of this owner (a cluster of CL CTAs), panel
+  // q + 1 factored by its owner
+  const int owner = rank / CL, owners = group / CL, crank = rank % CL;
   for (int64_t q = -1; q + 1 < np; ++q) {
     const int64_t next = q + 1;
-    const int64_t mine = next + ((rank - next) % group + group) % group;  // first own panel from `next` on
-    if (mine >= np) break;  // nothing of this CTA's is left
+    const int64_t mine = next + ((owner - next) % owners + owners) % owners;  // first own panel from `next` on
+    if (mine >= np) break;  // nothing of this owner's is left
     QrPanel<T, VS> p = {Vs, V, L, 0};
     if (mine == next) {
-      const int64_t passes = (L - (q >= 0 ? q * kPanel : 0) + kThreads - 1) / kThreads;
+      const int64_t passes = (L - (q >= 0 ? q * kPanel : 0) + CL * kThreads - 1) / (CL * kThreads);
       const int nb = width(next);
-#define YB_PANEL(R) qr_factor_panel<T, VS, (R <= MAXR ? R : 1)>(Z, V, L, next, nb, p, Vs, sh, ready, ctrl + C_ERR)
+#define YB_PANEL(R) qr_factor_panel<T, VS, (R <= MAXR ? R : 1), CL>(Z, V, L, next, nb, p, Vs, sh, ready, ctrl + C_ERR)
       if (passes <= 1) YB_PANEL(1);
-      else if (passes <= 2) YB_PANEL(2);
-      else if (MAXR >= 4 && passes <= 4) YB_PANEL(4);
+      else if (MAXR >= 2 && passes <= 2) YB_PANEL(2);
+      else if (CL > 1 && MAXR >= 3 && passes <= 3) YB_PANEL(3);
+      else if (CL == 1 && MAXR >= 4 && passes <= 4) YB_PANEL(4);
       else if (MAXR >= 6 && passes <= 6) YB_PANEL(6);
       else if (MAXR >= 11 && passes <= 11) YB_PANEL(11);
       else {
@@ -528,11 +636,12 @@ __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const i
           qr_wait(ready, (unsigned long long)next, ctrl + C_ERR);
           p = qr_load_panel<T, VS>(V, L, q, kPanel, Vs, sh);
         }
-        qr_factor_panel_long<T, VS>(Z, V, L, next, nb, q >= 0, p, sh);
+        qr_sync<CL>();
+        if (crank == 0) qr_factor_panel_long<T, VS>(Z, V, L, next, nb, q >= 0, p, sh);
       }
 #undef YB_PANEL
-      __syncthreads();
-      if (threadIdx.x == 0) {
+      qr_sync<CL>();
+      if (threadIdx.x == 0 && crank == 0) {
         __threadfence();
         atomicMax(ready, (unsigned long long)(next + 1));
       }
@@ -541,16 +650,28 @@ __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const i
       p = qr_load_panel<T, VS>(V, L, q, kPanel, Vs, sh);
     }
     if (q >= 0) {
-      // this CTA's later panels: a column per warp
-      const int64_t first = mine == next ? mine + group : mine;
-      for (int64_t e = warp;; e += kWarps) {
-        const int64_t pan = first + (e / kPanel) * group, c = pan * kPanel + e % kPanel;
-        if (pan >= np) break;
-        if (c < k) qr_apply_panel<T, VS, true>(Z + c * L + q * kPanel, p, kPanel, sh, lane);
+      if (mine == next && next + owners < np) p = qr_load_panel<T, VS>(V, L, q, kPanel, Vs, sh);
+      // this owner's later panels: a column per warp. In a cluster a column stays with its warp: CTA
+      // j % CL takes column j of a panel.
+      const int64_t first = mine == next ? mine + owners : mine;
+      if constexpr (CL == 1) {
+        for (int64_t e = warp;; e += kWarps) {
+          const int64_t pan = first + (e / kPanel) * owners, c = pan * kPanel + e % kPanel;
+          if (pan >= np) break;
+          if (c < k) qr_apply_panel<T, VS, true>(Z + c * L + q * kPanel, p, kPanel, sh, lane, xs);
+        }
+      } else {
+        constexpr int kCols = kPanel / CL, kTurn = kWarps / kCols;
+        const int64_t o = (first - owner) / owners, turn = warp / kCols;
+        const int j = crank + CL * (warp % kCols);
+        for (int64_t pan = first + ((turn - o) % kTurn + kTurn) % kTurn * owners; pan < np; pan += kTurn * owners) {
+          const int64_t c = pan * kPanel + j;
+          if (c < k) qr_apply_panel<T, VS, true>(Z + c * L + q * kPanel, p, kPanel, sh, lane, xs);
+        }
       }
     }
   }
-  if (!grid_barrier(ctrl, group)) return false;
+  if (!qr_all<CL>(grid_barrier(ctrl, group))) return false;
   // R rows, tau, the FP32 start
   const double sc = scale_b ? *scale_b : 0.0;  // no FP32 Jacobi start for yb_qr
   for (int64_t e = gt; e < k * k; e += ngt) {
@@ -563,7 +684,7 @@ __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const i
     }
   }
   for (int64_t e = gt; e < k; e += ngt) tau[e] = ldcg_t(V + e * L + e);  // T's diagonal
-  if (!grid_barrier(ctrl, group)) return false;
+  if (!qr_all<CL>(grid_barrier(ctrl, group))) return false;
   // Q's columns: row c of Z becomes (H_0 ... H_c e_c)^T, the panels backwards
   // Columns rank, rank + group, .. of a CTA, dealt to its warps in turn: every CTA has columns of all
   // panels (with 8 neighbouring columns a CTA, the last of 54 did all 108 panels of k = 432 alone).
@@ -578,13 +699,13 @@ __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const i
         for (int64_t l = lane; l < L; l += 32) x[l] = (l == c) ? Num<T>::one() : Num<T>::zero();
         __syncwarp();
       }
-      qr_apply_panel<T, VS, false>(x + q * kPanel, p, width(q), sh, lane);
+      qr_apply_panel<T, VS, false>(x + q * kPanel, p, width(q), sh, lane, xs);
     }
   }
-  return grid_barrier(ctrl, group);
+  return qr_all<CL>(grid_barrier(ctrl, group));
 }
 
-template <typename T, typename T32, int MAXR, int PER_SM>
+template <typename T, typename T32, int MAXR, int PER_SM, int CL>
 __global__ void __launch_bounds__(kThreads, PER_SM)
     svd_qr_kernel(T* __restrict__ work, T32* __restrict__ work32, const int64_t* __restrict__ blocks, int n_blocks,
                   int group, unsigned long long* __restrict__ qctrl, const double* __restrict__ scale, int smem_elems) {
@@ -593,34 +714,61 @@ __global__ void __launch_bounds__(kThreads, PER_SM)
   __shared__ QrShared<T> sh;
   const int g = blockIdx.x / group, rank = blockIdx.x % group;
   const int n_groups = gridDim.x / group;
-  if (g >= n_groups) return;
+  qr_sync<CL>();  // every CTA of the cluster runs before its shared memory is written
   // qctrl: [n_blocks ready counters][C_REC words per group]
   unsigned long long* ctrl = qctrl + n_blocks + (int64_t)g * C_REC;
   for (int b = g; b < n_blocks; b += n_groups) {
     const int64_t* r = blocks + (int64_t)b * YB_SVD_REC;
     if (!r[R_QR]) continue;
     const double* sb = scale ? scale + b : nullptr;
-    const bool ok = kPanel * r[R_LQ] <= smem_elems
-                        ? qr_block<T, T32, MAXR, true>(work, work32, r, group, rank, qctrl + b, ctrl, sb, Vs, sh)
-                        : qr_block<T, T32, MAXR, false>(work, work32, r, group, rank, qctrl + b, ctrl, sb, Vs, sh);
+    bool ok;
+#define YB_BLOCK(MAX, VS, C) \
+  qr_block<T, T32, MAX, VS, C>(work, work32, r, group, rank, qctrl + b, ctrl, sb, Vs, smem_elems, sh)
+    if constexpr (CL > 1) {
+      ok = r[R_LQ] <= kPairRows ? YB_BLOCK(1, true, 1)
+           : kPanel * r[R_LQ] <= smem_elems ? YB_BLOCK(MAXR, true, CL) : YB_BLOCK(MAXR, false, CL);
+      ok = qr_all<CL>(ok);
+    } else {
+      ok = kPanel * r[R_LQ] <= smem_elems ? YB_BLOCK(MAXR, true, 1) : YB_BLOCK(MAXR, false, 1);
+    }
+#undef YB_BLOCK
     if (!ok) return;
   }
 }
 
-// Up to one block per SM: one CTA per SM, panels of up to 11 (complex: 6) passes in registers,
-// 200 KB of shared memory. More blocks than SMs, one CTA each: two CTAs per SM (the pipe of one is
-// idle while the other waits) with fewer passes and half the shared memory.
-template <typename T, typename T32, int MAXR, int PER_SM>
+// Up to one block per eight SMs: clusters of CL CTAs, one CTA per SM, panels of up to 6 passes of
+// CL x 256 rows in registers, 200 KB of shared memory. Up to one block per SM: the same without
+// clusters, up to 11 (complex: 6) passes of 256 rows. More blocks than SMs, one CTA each: two CTAs
+// per SM (the pipe of one is idle while the other waits) with fewer passes and half the shared
+// memory. `launched` false: the clusters do not fit the device, nothing was launched.
+template <typename T, typename T32, int MAXR, int PER_SM, int CL>
 int qr_launch(void* work, void* work32, const int64_t* blocks, int n_blocks, double* scale, int64_t* qctrl,
-              int qctrl_words, int sms, cudaStream_t s) {
-  auto kernel = svd_qr_kernel<T, T32, MAXR, PER_SM>;
+              int qctrl_words, int sms, cudaStream_t s, bool* launched) {
+  auto kernel = svd_qr_kernel<T, T32, MAXR, PER_SM, CL>;
   const int smem = 200 * 1024 / PER_SM;
-  int per_sm = 0;
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim = {CL, 1, 1};
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(sms / CL * CL));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = CL > 1 ? 2 : 1;
+  *launched = false;
+  int resident = 0;  // CTAs of the device, clusters when CL > 1
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, smem);
+  if (e == cudaSuccess) {
+    if constexpr (CL > 1) e = cudaOccupancyMaxActiveClusters(&resident, kernel, &cfg);
+    else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kThreads, smem);
+  }
   if (e != cudaSuccess) { set_cuda_error((int)e); return YB_ERR_CUDA; }
-  const int capacity = sms * (per_sm < 1 ? 1 : per_sm);
-  int group = capacity / n_blocks;
+  const int capacity = CL > 1 ? CL * resident : sms * (resident < 1 ? 1 : resident);
+  int group = capacity / n_blocks / CL * CL;
+  if (CL > 1 && group * n_blocks * 8 < 7 * sms) return YB_OK;
   group = group < 1 ? 1 : group;
   int n_groups = capacity / group;
   if (n_groups > n_blocks) n_groups = n_blocks;
@@ -628,13 +776,11 @@ int qr_launch(void* work, void* work32, const int64_t* blocks, int n_blocks, dou
   if (n_groups < 1) return YB_ERR_INVALID;
   e = cudaMemsetAsync(qctrl, 0, sizeof(int64_t) * ((size_t)n_groups * C_REC + n_blocks), s);
   if (e != cudaSuccess) { set_cuda_error((int)e); return YB_ERR_CUDA; }
-  T* w = (T*)work;
-  T32* w32 = (T32*)work32;
-  unsigned long long* qc = (unsigned long long*)qctrl;
-  int elems = smem / (int)sizeof(T);
-  void* args[] = {&w, &w32, &blocks, &n_blocks, &group, &qc, &scale, &elems};
-  e = cudaLaunchCooperativeKernel((const void*)kernel, dim3(n_groups * group), dim3(kThreads), args, smem, s);
+  cfg.gridDim = dim3((unsigned)(n_groups * group));
+  e = cudaLaunchKernelEx(&cfg, kernel, (T*)work, (T32*)work32, blocks, n_blocks, group, (unsigned long long*)qctrl,
+                         (const double*)scale, smem / (int)sizeof(T));
   if (e != cudaSuccess) { set_cuda_error((int)e); return YB_ERR_CUDA; }
+  *launched = true;
   return YB_OK;
 }
 
@@ -646,9 +792,15 @@ int qr_factor(void* work, void* work32, const int64_t* blocks, int n_blocks, dou
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) { set_cuda_error((int)e); return YB_ERR_CUDA; }
+  bool launched = false;
+  if (n_blocks * 8 <= sms) {
+    const int st = qr_launch<T, T32, 6, 1, kMaxCl>(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, sms, s,
+                                                   &launched);
+    if (st != YB_OK || launched) return st;
+  }
   return n_blocks <= sms
-             ? qr_launch<T, T32, kFew, 1>(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, sms, s)
-             : qr_launch<T, T32, kMany, 2>(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, sms, s);
+             ? qr_launch<T, T32, kFew, 1, 1>(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, sms, s, &launched)
+             : qr_launch<T, T32, kMany, 2, 1>(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, sms, s, &launched);
 }
 
 }  // namespace
