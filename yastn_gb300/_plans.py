@@ -1295,6 +1295,16 @@ class QrPlan:
 QRADJ_REC = 8
 
 
+def _lower_strips(k):
+    """Row strips (i0, i1) of a k x k matrix of which the lower triangle is wanted: the columns up to
+    i1 are formed. Strips of 64 rows, two of the products' tiles (a last one of less than 32 would go
+    to the kernel of short products)."""
+    edges = list(range(0, k, 64)) + [k]
+    if len(edges) > 2 and edges[-1] - edges[-2] < 32:
+        del edges[-2]
+    return list(zip(edges[:-1], edges[1:]))
+
+
 def qr_plan(meta, cplx=False):
     """Reduced QR records (sl, D, slQ, DQ, slR, DR) of yastn/tensor/linalg.py:795-828, as
     computed by backend_np.py:511-520 (positive diagonal of R)."""
@@ -1323,8 +1333,9 @@ def qr_plan(meta, cplx=False):
                 right.append((r0 + m, k, n - m, n, [(q0, a0 + m, m, 1, k, n, 1, cj)]))
                 w1.append((q0, m, m, k, [(a0 + m, r0 + m, n - m, n, 1, 1, n, 2 * cj)]))  # gQ' += A[:, m:] gV^H
                 y1.append((a0 + m, m, n - m, n, [(q0, r0 + m, m, k, 1, n, 1, 0)]))      # dA[:, m:] = Q gV
-            m1.append((mo, k, k, k, [(r0, r0, k, n, 1, 1, n, 2 * cj)]))                  # M = U gU^H
-            m2.append((mo, k, k, k, [(q0, q0, m, 1, k, k, 1, cj)]))                      # M -= gQ'^H Q
+            for i0, i1 in _lower_strips(k):  # M = U gU^H, M -= gQ'^H Q
+                m1.append((mo + i0 * k, i1 - i0, i1, k, [(r0 + i0 * n + i0, r0 + i0, k - i0, n, 1, 1, n, 2 * cj)]))
+                m2.append((mo + i0 * k, i1 - i0, i1, k, [(q0 + i0, q0, m, 1, k, k, 1, cj)]))
             s1.append((q0, m, k, k, [(q0, mo, k, k, 1, k, 1, 0)]))                       # gQ' += Q copyltu(M)
             adj.append((mo, k, q0, m, k, r0, n, 0))
             copies.append((q0, a0, [m, k], [k, 1], [n, 1]))
