@@ -187,12 +187,13 @@ __global__ void qr_copyltu_kernel(double* __restrict__ M, const int64_t* __restr
 
 // B <- B R^{-H} row by row (R upper triangular with a real diagonal): x R^H = b, i.e.
 // x_j = (b_j - sum_{l > j} x_l conj(R_jl)) / R_jj by back substitution, in place. A warp takes a row, a
-// CTA eight; 32 unknowns at a time: lane j sums over the solved ones (32 x 32 tiles of R shared by the
+// CTA four; 32 unknowns at a time: lane j sums over the solved ones (32 x 32 tiles of R shared by the
 // CTA's rows, the next tile's loads in flight), then the 32 are solved among themselves, each
 // broadcast to the lanes below it. Bound: the FP64 issue of an SM (rows k^2 / 2 FMAs and, in the
-// chain of 32 solves, four instructions each by all eight warps: 0.35 ms at two blocks of
-// 540 x 432) and the chain's latency. Measured there: 0.73 ms; one unknown at a time, a sum over
-// global memory and a division each, 2.5 ms.
+// chain of 32 solves, four instructions each: 0.35 ms at two blocks of 540 x 432, with eight rows an
+// SM). Measured there: 0.385 ms; with eight rows a CTA 0.73 (all warps of an SM wait for the same
+// tile), with two 0.63 (twice the loads of R); one unknown at a time, a sum over global memory and a
+// division each, 2.5 ms.
 template <bool Cx>
 struct TrsmVal {
   using T = double;
@@ -232,8 +233,10 @@ __device__ __forceinline__ double2 trsm_div(double2 v, double d, double ri) {
   return make_double2(trsm_div(v.x, d, ri), trsm_div(v.y, d, ri));
 }
 
+constexpr int kTrsmRows = 4;  // rows (warps) of a CTA
+
 template <bool Cx>
-__global__ void __launch_bounds__(256) trsm_rt_kernel(double* __restrict__ B, const double* __restrict__ Rm,
+__global__ void __launch_bounds__(kTrsmRows * 32) trsm_rt_kernel(double* __restrict__ B, const double* __restrict__ Rm,
                                                       const int64_t* __restrict__ recs) {
   using T = typename TrsmVal<Cx>::T;
   __shared__ T tile[2][32][33];  // [l][j]: R_{J0 + j, l0 + l}
@@ -243,24 +246,24 @@ __global__ void __launch_bounds__(256) trsm_rt_kernel(double* __restrict__ B, co
   const T* R = reinterpret_cast<const T*>(Rm) + r[5];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const T zero = T{};
-  for (int64_t g0 = (int64_t)blockIdx.x * 8; g0 < rows; g0 += (int64_t)gridDim.x * 8) {
+  for (int64_t g0 = (int64_t)blockIdx.x * kTrsmRows; g0 < rows; g0 += (int64_t)gridDim.x * kTrsmRows) {
     const bool live = g0 + warp < rows;
     T* x = b + (live ? g0 + warp : 0) * ldb;
     for (int64_t J0 = (k - 1) / 32 * 32; J0 >= 0; J0 -= 32) {
       const int w = (int)min((int64_t)32, k - J0);
       // tiles l0 = J0 (the diagonal one, used last) and from J0 + 32 on
-      T reg[4], xn = zero;
+      T reg[32 / kTrsmRows], xn = zero;
       auto fetch = [&](int64_t l0) {
         xn = live && l0 + lane < k ? __ldcg(x + l0 + lane) : zero;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int j = warp + 8 * u;
+        for (int u = 0; u < 32 / kTrsmRows; ++u) {
+          const int j = warp + kTrsmRows * u;
           reg[u] = (j < w && l0 + lane < k) ? R[(J0 + j) * ldr + l0 + lane] : zero;
         }
       };
       auto put = [&](int buf) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) tile[buf][lane][warp + 8 * u] = reg[u];
+        for (int u = 0; u < 32 / kTrsmRows; ++u) tile[buf][lane][warp + kTrsmRows * u] = reg[u];
       };
       T acc = zero;
       int buf = 0;
@@ -309,10 +312,10 @@ extern "C" int yb_qr_adjoint_sym(void* M, const int64_t* recs, int n_blocks, int
 extern "C" int yb_trsm_rt(void* B, const void* R, const int64_t* recs, int n_blocks, int dtype, void* stream) {
   if (n_blocks == 0) return YB_OK;
   if (!B || !R || !recs) return YB_ERR_INVALID;
-  const dim3 grid(128, (unsigned)n_blocks);
+  const dim3 grid(256, (unsigned)n_blocks);
   cudaStream_t s = (cudaStream_t)stream;
-  if (dtype == YB_F64) yb::trsm_rt_kernel<false><<<grid, 256, 0, s>>>((double*)B, (const double*)R, recs);
-  else if (dtype == YB_C128) yb::trsm_rt_kernel<true><<<grid, 256, 0, s>>>((double*)B, (const double*)R, recs);
+  if (dtype == YB_F64) yb::trsm_rt_kernel<false><<<grid, yb::kTrsmRows * 32, 0, s>>>((double*)B, (const double*)R, recs);
+  else if (dtype == YB_C128) yb::trsm_rt_kernel<true><<<grid, yb::kTrsmRows * 32, 0, s>>>((double*)B, (const double*)R, recs);
   else return YB_ERR_INVALID;
   return yb::check_launch();
 }
