@@ -25,9 +25,9 @@
 // 2.64 / 2.73, yb_svd_qr of two 1296 x 1296 16.6 / 17.0, yb_qr of two 648 x 1296 6.9 / 7.9.
 //
 // Measured (GB300; before: a warp per column, one reflector at a time, published by itself): yb_qr
-// of two 540 x 432 blocks 7.8 -> 2.6 ms; yb_svd_qr of two 432 x 432 blocks 6.2 -> 2.4 ms, two
-// 1296 x 1296 62 -> 16.6 ms (10.6 ms at the DFMA rate), nine of 24..93 0.73 -> 0.41 ms, five complex
-// ones of 31 x 24 .. 78 x 60 0.68 -> 0.48 ms; 595 blocks of 42..60 2.6 -> 1.4 ms.
+// of two 540 x 432 blocks 7.8 -> 2.5 ms; yb_svd_qr of two 432 x 432 blocks 6.2 -> 2.25 ms, two
+// 1296 x 1296 62 -> 16.0 ms (10.6 ms at the DFMA rate), nine of 24..93 0.73 -> 0.39 ms, five complex
+// ones of 31 x 24 .. 78 x 60 0.68 -> 0.47 ms; 595 blocks of 42..60 2.6 -> 1.4 ms.
 #pragma once
 #include <cooperative_groups.h>
 #include "yb_svd_common.cuh"
@@ -154,6 +154,7 @@ __device__ __forceinline__ void qr_wait(const unsigned long long* flag, unsigned
 template <typename T>
 struct QrShared {
   T Tm[kPanel][kPanel];          // T of the panel in Vs: Tm[j][i], j <= i, zero below
+  T Tq[2][kPanel][kPanel];       // the same for the two panels at hand when Q is formed
   T part[2][kMaxCl * kWarps][kPanel * kPanel];
   T sum[kPanel * kPanel];        // V^H x of the update before a panel's factorisation
   T row[2][kPanel];              // the panel's row j
@@ -203,16 +204,40 @@ __device__ __forceinline__ QrPanel<T, VS> qr_load_panel(const T* __restrict__ V,
   return p;
 }
 
+// The same without waiting: V's copy to shared memory is left in flight, T in the returned entry
+// (threads below kPanel^2).
+template <typename T>
+__device__ __forceinline__ T qr_fetch_panel(const T* __restrict__ V, int64_t L, int64_t q, int nb, T* Vs) {
+  const int64_t j0 = q * kPanel;
+  const T* g = V + j0 * L + j0;
+  const int len = (int)(L - j0);
+  for (int i = 0; i < kPanel; ++i) {
+    const T* src = g + i * L;
+    T* dst = Vs + i * len;
+    for (int l = threadIdx.x; l < len; l += kThreads) {
+      if (i < nb && l > i)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst + l)),
+                     "l"(src + l), "n"(sizeof(T))
+                     : "memory");
+      else
+        dst[l] = i < nb && l == i ? Num<T>::one() : Num<T>::zero();
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  const int i = threadIdx.x % kPanel, j = threadIdx.x / kPanel;
+  return j <= i && i < nb ? __ldcg(g + i * L + j) : Num<T>::zero();
+}
+
 // y = - op(T) w for the sums w of a warp's lanes; op(T) = T^H or T.
 template <typename T, bool ADJ>
-__device__ __forceinline__ void qr_apply_t(T (&w)[kPanel], T (&ny)[kPanel], const QrShared<T>& sh, int lane) {
+__device__ __forceinline__ void qr_apply_t(T (&w)[kPanel], T (&ny)[kPanel], const T (&Tm)[kPanel][kPanel], int lane) {
   const T mine = warp_sums<T, kPanel>(w, lane);  // lane l: value l >> 3
   const int i = lane >> 3;
   T y = Num<T>::zero();
 #pragma unroll
   for (int j = 0; j < kPanel; ++j) {
     const T wj = shfl_t(mine, 8 * j);
-    const T t = ADJ ? Num<T>::conj(sh.Tm[j][i]) : sh.Tm[i][j];
+    const T t = ADJ ? Num<T>::conj(Tm[j][i]) : Tm[i][j];
     y = Num<T>::fma_(t, wj, y);
   }
 #pragma unroll
@@ -225,8 +250,8 @@ __device__ __forceinline__ void qr_apply_t(T (&w)[kPanel], T (&ny)[kPanel], cons
 // read from global memory twice, the FP64 pipe waits twice (two 1296 x 1296 blocks 18.7 ms instead of
 // 16.6); in registers, the variants by length spill and miss the instruction cache (20.8 ms).
 template <typename T, bool VS, bool ADJ>
-__device__ __forceinline__ void qr_apply_panel(T* __restrict__ x, const QrPanel<T, VS>& p, int nb, const QrShared<T>& sh,
-                                               int lane, T* __restrict__ xs) {
+__device__ __forceinline__ void qr_apply_panel(T* __restrict__ x, const QrPanel<T, VS>& p, int nb,
+                                               const T (&Tm)[kPanel][kPanel], int lane, T* __restrict__ xs) {
   T w[kPanel], ny[kPanel];
 #pragma unroll
   for (int i = 0; i < kPanel; ++i) w[i] = Num<T>::zero();
@@ -238,7 +263,7 @@ __device__ __forceinline__ void qr_apply_panel(T* __restrict__ x, const QrPanel<
     for (int i = 0; i < kPanel; ++i)
       if (VS || i < nb) w[i] = Num<T>::fmac(xv, p.v(i, l), w[i]);
   }
-  qr_apply_t<T, ADJ>(w, ny, sh, lane);
+  qr_apply_t<T, ADJ>(w, ny, Tm, lane);
 #pragma unroll 4
   for (int l = lane; l < p.len; l += 32) {
     T xv = VS && xs ? xs[l] : ldcg_t(x + l);
@@ -538,7 +563,7 @@ __device__ void qr_factor_panel_long(T* __restrict__ Z, T* __restrict__ V, int64
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t c0 = next * kPanel;
   T* z = Z + (c0 + warp) * L;
-  if (has_p && warp < nb) qr_apply_panel<T, VS, true>(z + c0 - kPanel, p, kPanel, sh, lane, (T*)nullptr);
+  if (has_p && warp < nb) qr_apply_panel<T, VS, true>(z + c0 - kPanel, p, kPanel, sh.Tm, lane, (T*)nullptr);
   __syncthreads();
   T Tm[kPanel][kPanel];
 #pragma unroll
@@ -658,7 +683,7 @@ __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const i
         for (int64_t e = warp;; e += kWarps) {
           const int64_t pan = first + (e / kPanel) * owners, c = pan * kPanel + e % kPanel;
           if (pan >= np) break;
-          if (c < k) qr_apply_panel<T, VS, true>(Z + c * L + q * kPanel, p, kPanel, sh, lane, xs);
+          if (c < k) qr_apply_panel<T, VS, true>(Z + c * L + q * kPanel, p, kPanel, sh.Tm, lane, xs);
         }
       } else {
         constexpr int kCols = kPanel / CL, kTurn = kWarps / kCols;
@@ -666,7 +691,7 @@ __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const i
         const int j = crank + CL * (warp % kCols);
         for (int64_t pan = first + ((turn - o) % kTurn + kTurn) % kTurn * owners; pan < np; pan += kTurn * owners) {
           const int64_t c = pan * kPanel + j;
-          if (c < k) qr_apply_panel<T, VS, true>(Z + c * L + q * kPanel, p, kPanel, sh, lane, xs);
+          if (c < k) qr_apply_panel<T, VS, true>(Z + c * L + q * kPanel, p, kPanel, sh.Tm, lane, xs);
         }
       }
     }
@@ -689,9 +714,7 @@ __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const i
   // Columns rank, rank + group, .. of a CTA, dealt to its warps in turn: every CTA has columns of all
   // panels (with 8 neighbouring columns a CTA, the last of 54 did all 108 panels of k = 432 alone).
   const int64_t top = rank < k ? rank + (k - 1 - rank) / group * group : -1;
-  for (int64_t q = np - 1; q >= 0; --q) {
-    if (top < q * kPanel) continue;  // no column of this CTA from this panel on
-    const QrPanel<T, VS> p = qr_load_panel<T, VS>(V, L, q, width(q), Vs, sh);
+  auto columns = [&](int64_t q, const QrPanel<T, VS>& p, const T(&Tm)[kPanel][kPanel]) {
     for (int64_t c = rank + (int64_t)group * warp; c < k; c += (int64_t)group * kWarps) {
       if (c < q * kPanel) continue;
       T* x = Z + c * L;
@@ -699,8 +722,27 @@ __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const i
         for (int64_t l = lane; l < L; l += 32) x[l] = (l == c) ? Num<T>::one() : Num<T>::zero();
         __syncwarp();
       }
-      qr_apply_panel<T, VS, false>(x + q * kPanel, p, width(q), sh, lane, xs);
+      qr_apply_panel<T, VS, false>(x + q * kPanel, p, width(q), Tm, lane, xs);
     }
+  };
+  const int64_t q0 = top < 0 ? -1 : top / kPanel;  // the first panel with columns of this CTA
+  if (VS && (2 * kPanel + kWarps) * L <= smem_elems) {
+    // two panels in shared memory, the next one's copy in flight (waited for in turn: yb_qr of two
+    // 540 x 432 blocks 2.64 ms instead of 2.48, yb_svd_qr of two 1296 x 1296 16.6 instead of 16.0)
+    T* buf[2] = {Vs, Vs + (kPanel + kWarps) * L};
+    T tm = Num<T>::zero();
+    if (q0 >= 0) tm = qr_fetch_panel<T>(V, L, q0, width(q0), buf[q0 & 1]);
+    for (int64_t q = q0; q >= 0; --q) {
+      const int h = (int)(q & 1);
+      if (threadIdx.x < kPanel * kPanel) sh.Tq[h][threadIdx.x / kPanel][threadIdx.x % kPanel] = tm;
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();  // panel q is there; panel q + 1 is done with
+      if (q > 0) tm = qr_fetch_panel<T>(V, L, q - 1, kPanel, buf[h ^ 1]);
+      columns(q, QrPanel<T, VS>{buf[h], V + q * kPanel * (L + 1), L, (int)(L - q * kPanel)}, sh.Tq[h]);
+    }
+  } else {
+    for (int64_t q = q0; q >= 0; --q)
+      columns(q, qr_load_panel<T, VS>(V, L, q, width(q), Vs, sh), sh.Tm);
   }
   return qr_all<CL>(grid_barrier(ctrl, group));
 }
