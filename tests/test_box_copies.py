@@ -100,3 +100,26 @@ def test_kernel_matches_numpy(dtype, cuda_device):
             assert np.array_equal(got, x.reshape(sizes).transpose(order).ravel())
             back = ops.transpose_backward(torch.from_numpy(got).cuda(), tuple(int(o) for o in order), meta)
             assert np.array_equal(back.cpu().numpy(), x)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('shape,order', [((28, 28, 28, 28), (3, 2, 1, 0)), ((48, 5, 50), (2, 1, 0)),
+                                         ((28, 30, 29, 31), (3, 1, 2, 0))])
+def test_large_copies_with_fuller_tiles_go_by_boxes(shape, order, cuda_device):
+    """Copies of BOX_LARGE elements take boxes where the tiles would be half full and more; the same
+    blocks in a smaller copy keep the tiles. Both are exact, forward and inverse."""
+    import torch
+    from yastn_gb300 import ops
+    n1 = int(np.prod(shape))
+    strides = P.row_major_strides(shape)
+    dims = [shape[o] for o in order]
+    for count, boxes in ((P.BOX_LARGE // n1 + 1, True), (2, False)):
+        tasks = [(i * n1, i * n1, dims, [strides[o] for o in order], P.row_major_strides(dims)) for i in range(count)]
+        plan = P.CopyPlan(tasks, count * n1, count * n1)
+        assert bool(len(plan.packed_with_boxes(False, 8)[2])) == boxes
+        x = torch.arange(count * n1, dtype=torch.float64, device='cuda')
+        y, z = torch.empty_like(x), torch.empty_like(x)
+        ops.run_copy(plan, x, y)
+        assert torch.equal(y.view(count, *dims), x.view(count, *shape).permute(0, *(o + 1 for o in order)))
+        ops.run_copy(plan.swapped(count * n1), y, z)
+        assert torch.equal(z, x)

@@ -233,7 +233,8 @@ BOX_MAX_T = 255      # coordinates within a box are bytes
 BOX_PER_CTA = 16     # boxes of one CTA, fewer where that leaves less than BOX_CTAS CTAs
 BOX_CTAS = 608       # four per SM (two at a time)
 BOX_MIN_MIXED = 1 << 20
-BOX_MIN_SCATTER = 1 << 22
+BOX_MIN_SCATTER = 1 << 21
+BOX_LARGE = 1 << 23
 
 
 def _box_elements(elem):
@@ -334,13 +335,15 @@ def _by_destination(task):
     return (so, do) + tuple(_collapse([sizes[i] for i in o], [ss[i] for i in o], [ds[i] for i in o]))
 
 
-def _wants_box(sizes, ss, ds, elem):
+def _wants_box(sizes, ss, ds, elem, fill=0.5):
     """Whether a collapsed task goes by boxes: a transposition whose 32 x 32 tiles over its innermost
-    source and destination dims (extents y and x) would be less than half full. Measured, 24 M FP64
-    elements in blocks of (shape, order): (15, 14, 13, 13, 12) 43210 as tiles 408, boxes 154 us; (5, 6,
-    5, 7, 6) 43210 2254 and 197; (19, 18, 17, 20) 3210 252 and 123; but (100, 3, 100, 3) 3210 109 and
-    121, (513, 511) 10 98 and 113. Common innermost runs, and dims of fewer than 4, are copied unit by
-    unit: (15, 14, 13, 13, 12) 02314 68, boxes 148 us."""
+    source and destination dims (extents y and x) would be filled to less than ``fill``: half, or 0.9
+    in a copy of BOX_LARGE elements and more. Measured, 24 M FP64 elements in blocks of (shape, order),
+    tiles and boxes, us: (15, 14, 13, 13, 12) 43210 412 and 92; (5, 6, 5, 7, 6) 43210 2277 and 127; (19,
+    18, 17, 20) 3210 258 and 90; (48, 5, 50) 210 150 and 93; (28, 28, 28, 28) 3210 140 and 109; but
+    (100, 3, 100, 3) 3210 109 and 156, (64, 60, 62) 210 100 and 106, (513, 511) 10 98 and 96. (48, 5,
+    50) and (28, 28, 28, 28) at 8 M: 55 and 41, 53 and 49; at 2 M 18 and 21, 16 and 21. Common innermost
+    runs, and dims of fewer than 4, are copied unit by unit: (15, 14, 13, 13, 12) 02314 68 and 121."""
     last = len(sizes) - 1
     if last < 1 or len(sizes) > CP_MAXD or ds[last] != 1 or ss[last] == 1 or sizes[last] < 4:
         return False
@@ -350,7 +353,7 @@ def _wants_box(sizes, ss, ds, elem):
     x, y, T = sizes[last], sizes[ys[-1]], COPY_TILE
     tiles = -(-x // T) * -(-y // T)
     # a block of a single box pays the box's set-up for itself: only where a tile holds little
-    return x * y < 0.5 * T * T * tiles and (x * y < 300 * tiles or
+    return x * y < fill * T * T * tiles and (x * y < 300 * tiles or
                                             np.prod(sizes, dtype=np.int64) >= 4 * _box_elements(elem))
 
 
@@ -383,12 +386,15 @@ class CopyPlan:
             rest, recs, tables = [], [], []
             tasks = self._expanded()
             # an inverse copy lists its dims in its source's order: unit by unit it reads runs and
-            # scatters them, which beats boxes up to tens of MB (32 MB of FP64; 219 MB: 248 and 150 us)
+            # scatters them, which boxes beat from about 2 M elements on (FP64, order 41302 of dims 12..15:
+            # 1.7 M 22.5 and 20.5 us, 3.8 M 39 and 29, 24 M 182 and 95; 3210 of 17..20: 20.5 and 20.5, 33 and
+            # 27, 141 and 90)
             by_dst = [_by_destination(t) for t in tasks]
             scatter = [t is not u for t, u in zip(tasks, by_dst)]
             large = sum(int(np.prod(t[2], dtype=np.int64)) for t, x in zip(tasks, scatter) if x) >= BOX_MIN_SCATTER
+            fill = 0.9 if sum(int(np.prod(t[2], dtype=np.int64)) for t in tasks) >= BOX_LARGE else 0.5
             for task, ordered, x in zip(tasks, by_dst, scatter):
-                box = _box_task(*ordered, elem) if (large or not x) and _wants_box(*ordered[2:], elem) else None
+                box = _box_task(*ordered, elem) if (large or not x) and _wants_box(*ordered[2:], elem, fill) else None
                 if box is None:
                     rest.append(task)
                     continue

@@ -178,10 +178,12 @@ __global__ void __launch_bounds__(kThreads) block_copy_kernel(const Elem* __rest
 // would use a seventh of its lanes. All boxes of a task have one shape: a thread's elements (at most
 // kBoxElems per thread) and their offsets within the box stay in registers for all the boxes of its
 // CTA (worked out for every element of every box they cost more than the memory traffic), a box's
-// origins and clips come from a table, and the next box's loads are in flight while a box is
-// written out. Bound: memory latency; 27 M FP64 elements in blocks of 12..15 per leg, order 41302:
-// 148 us (0.44 of the copy bandwidth; 502 us as tiles, 420 us with the offsets worked out per
-// element, 320 us with 8 elements per thread and two CTAs of 256 threads per SM). Elements past the end of a block are
+// origins and clips come from a table, and the loads of the two boxes after the one that is written
+// out are in flight (cp.async into one of three stages). Bound: memory latency and the part-filled
+// sectors at the ends of runs; 27 M FP64 elements in blocks of 12..15 per leg, order 41302: 104 us (0.6
+// of the copy bandwidth; 502 us as tiles, 420 us with the offsets worked out per element, 148 us with
+// one box in flight, through registers). 24 M elements: 96 us, with six stages 109, with three CTAs per
+// SM (and their spills) 115. Elements past the end of a block are
 // clipped by comparing the coordinates along the (up to four) dims that do not divide evenly, a
 // byte each.
 // Records (YB_BOX_REC int64): [0] dims [1] elements of a box; per dim in source order (outermost
@@ -190,10 +192,27 @@ __global__ void __launch_bounds__(kThreads) block_copy_kernel(const Elem* __rest
 // dims in destination order. Boxes: int64 triples (src offset, dst offset, clip word).
 constexpr int kBoxThreads = 512;
 constexpr int kBoxElems = 4;  // per thread; 2 of 16 bytes
+constexpr int kBoxStages = 3;
+
+// Copies of 4 bytes and more go to shared memory without passing registers.
+template <typename Elem>
+__device__ __forceinline__ void box_load(Elem* to, const Elem* from) {
+  if constexpr (sizeof(Elem) >= 4)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from),
+                 "n"(sizeof(Elem))
+                 : "memory");
+  else
+    *to = __ldg(from);
+}
 
 // Shared-memory slot of element e (in source order): a word of padding per 32, so that the reads along
 // the destination's runs spread over the banks.
 __device__ __forceinline__ int box_slot(int e) { return e + (e >> 5); }
+
+template <typename Elem>
+constexpr int box_slots() {  // of a stage
+  return (sizeof(Elem) >= 16 ? kBoxElems / 2 : kBoxElems) * kBoxThreads * 33 / 32 + 1;
+}
 
 template <typename Elem>
 __global__ void __launch_bounds__(kBoxThreads, 2) box_copy_kernel(const Elem* __restrict__ src, Elem* __restrict__ dst,
@@ -201,13 +220,12 @@ __global__ void __launch_bounds__(kBoxThreads, 2) box_copy_kernel(const Elem* __
                                                                    const int64_t* __restrict__ boxes,
                                                                    const int32_t* __restrict__ items) {
   constexpr int kU = sizeof(Elem) >= 16 ? kBoxElems / 2 : kBoxElems;
-  __shared__ Elem sm[kU * kBoxThreads + kU * kBoxThreads / 32 + 1];
+  extern __shared__ __align__(16) unsigned char box_smem[];
+  Elem* sm = reinterpret_cast<Elem*>(box_smem);  // kBoxStages boxes
   __shared__ int64_t rec[YB_BOX_REC];
   const int4 item = reinterpret_cast<const int4*>(items)[blockIdx.x];  // task, first box, boxes
   if (threadIdx.x < YB_BOX_REC) rec[threadIdx.x] = tasks[(int64_t)item.x * YB_BOX_REC + threadIdx.x];
   const int64_t* box = boxes + 3 * (int64_t)item.y;
-  int64_t bs = __ldg(box), bd = __ldg(box + 1);
-  uint32_t lim = (uint32_t)__ldg(box + 2);
   __syncthreads();
   const int nd = (int)rec[0], count = (int)rec[1];
   int soff[kU], doff[kU], from[kU];
@@ -239,38 +257,43 @@ __global__ void __launch_bounds__(kBoxThreads, 2) box_copy_kernel(const Elem* __
     }
     from[u] = box_slot(at);
   }
-  // the loads of box i + 1 are in flight while box i is written out
-  Elem v[kU];
-  auto load = [&] {
+  int64_t next = __ldg(box);  // source origin and clips of the box that is loaded next
+  uint32_t nlim = (uint32_t)__ldg(box + 2);
+  auto load = [&](int i) {
+    if (i < item.z) {
+      Elem* to = sm + i % kBoxStages * box_slots<Elem>();
 #pragma unroll
-    for (int u = 0; u < kU; ++u)
-      if (__vcmpgeu4(sc[u], lim) == 0) v[u] = __ldg(src + bs + soff[u]);
-  };
-  load();
-  for (int i = 0; i < item.z; ++i) {
-    __syncthreads();  // the box before has been written out
-#pragma unroll
-    for (int u = 0; u < kU; ++u) sm[box_slot((int)threadIdx.x + u * kBoxThreads)] = v[u];
-    Elem* d = dst + bd;
-    const uint32_t dlim = lim;
-    __syncthreads();
-    if (i + 1 < item.z) {
-      box += 3;
-      bs = __ldg(box);
-      bd = __ldg(box + 1);
-      lim = (uint32_t)__ldg(box + 2);
-      load();
+      for (int u = 0; u < kU; ++u)
+        if (__vcmpgeu4(sc[u], nlim) == 0) box_load(to + box_slot((int)threadIdx.x + u * kBoxThreads), src + next + soff[u]);
+      if (i + 1 < item.z) {
+        next = __ldg(box + 3 * (i + 1));
+        nlim = (uint32_t)__ldg(box + 3 * (i + 1) + 2);
+      }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < kBoxStages - 1; ++i) load(i);
+  for (int i = 0; i < item.z; ++i) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kBoxStages - 2) : "memory");
+    __syncthreads();  // box i is there; box i - 1 has been written out
+    load(i + kBoxStages - 1);
+    const Elem* at = sm + i % kBoxStages * box_slots<Elem>();
+    Elem* d = dst + __ldg(box + 3 * i + 1);
+    const uint32_t lim = (uint32_t)__ldg(box + 3 * i + 2);
 #pragma unroll
     for (int u = 0; u < kU; ++u)
-      if (__vcmpgeu4(dc[u], dlim) == 0) d[doff[u]] = sm[from[u]];
+      if (__vcmpgeu4(dc[u], lim) == 0) d[doff[u]] = at[from[u]];
   }
 }
 
 template <typename Elem>
 int launch_box(const void* src, void* dst, const int64_t* tasks, const int64_t* boxes, const int32_t* items,
                int n_items, cudaStream_t s) {
-  box_copy_kernel<Elem><<<n_items, kBoxThreads, 0, s>>>((const Elem*)src, (Elem*)dst, tasks, boxes, items);
+  const int smem = kBoxStages * box_slots<Elem>() * (int)sizeof(Elem);
+  const cudaError_t e = cudaFuncSetAttribute(box_copy_kernel<Elem>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) { set_cuda_error((int)e); return YB_ERR_CUDA; }
+  box_copy_kernel<Elem><<<n_items, kBoxThreads, smem, s>>>((const Elem*)src, (Elem*)dst, tasks, boxes, items);
   return check_launch();
 }
 
