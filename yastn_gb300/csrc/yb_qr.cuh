@@ -22,7 +22,8 @@
 // Why kPairRows = 256: a second CTA helps where it has rows to take (the first 256 are the first
 // CTA's), and its barriers cost what it saves around 432 rows: clusters against single CTAs, yb_svd_qr
 // of two 432 x 432 blocks 2.37 / 2.36 ms, yb_qr of two 216 x 432 ones 1.34 / 1.40, two 540 x 432
-// 2.64 / 2.73, yb_svd_qr of two 1296 x 1296 16.6 / 17.0, yb_qr of two 648 x 1296 6.9 / 7.9.
+// 2.64 / 2.73, yb_svd_qr of two 1296 x 1296 16.6 / 17.0, yb_qr of two 648 x 1296 6.9 / 7.9 (all with
+// Q's panels still loaded in turn).
 //
 // Measured (GB300; before: a warp per column, one reflector at a time, published by itself): yb_qr
 // of two 540 x 432 blocks 7.8 -> 2.5 ms; yb_svd_qr of two 432 x 432 blocks 6.2 -> 2.25 ms, two
@@ -747,18 +748,25 @@ __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const i
   return qr_all<CL>(grid_barrier(ctrl, group));
 }
 
-template <typename T, typename T32, int MAXR, int PER_SM, int CL>
-__global__ void __launch_bounds__(kThreads, PER_SM)
-    svd_qr_kernel(T* __restrict__ work, T32* __restrict__ work32, const int64_t* __restrict__ blocks, int n_blocks,
+template <typename T, typename T32, int MAXR, int CL>
+__device__ __forceinline__ void
+    qr_blocks(T* __restrict__ work, T32* __restrict__ work32, const int64_t* __restrict__ blocks, int n_blocks,
                   int group, unsigned long long* __restrict__ qctrl, const double* __restrict__ scale, int smem_elems) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* Vs = reinterpret_cast<T*>(smem_raw);
   __shared__ QrShared<T> sh;
   const int g = blockIdx.x / group, rank = blockIdx.x % group;
   const int n_groups = gridDim.x / group;
-  qr_sync<CL>();  // every CTA of the cluster runs before its shared memory is written
   // qctrl: [n_blocks ready counters][C_REC words per group]
   unsigned long long* ctrl = qctrl + n_blocks + (int64_t)g * C_REC;
+  if constexpr (CL > 1) {
+    // launched without the clusters, a panel's owner would write to shared memory that is not there
+    if (cooperative_groups::this_cluster().num_blocks() != CL) {
+      if (threadIdx.x == 0) atomicExch(ctrl + C_ERR, 1ull);
+      return;
+    }
+    qr_sync<CL>();  // every CTA of the cluster runs before its shared memory is written
+  }
   for (int b = g; b < n_blocks; b += n_groups) {
     const int64_t* r = blocks + (int64_t)b * YB_SVD_REC;
     if (!r[R_QR]) continue;
@@ -778,6 +786,21 @@ __global__ void __launch_bounds__(kThreads, PER_SM)
   }
 }
 
+template <typename T, typename T32, int MAXR, int PER_SM>
+__global__ void __launch_bounds__(kThreads, PER_SM)
+    svd_qr_kernel(T* __restrict__ work, T32* __restrict__ work32, const int64_t* __restrict__ blocks, int n_blocks,
+                  int group, unsigned long long* __restrict__ qctrl, const double* __restrict__ scale, int smem_elems) {
+  qr_blocks<T, T32, MAXR, 1>(work, work32, blocks, n_blocks, group, qctrl, scale, smem_elems);
+}
+
+template <typename T, typename T32, int MAXR>
+__global__ void __cluster_dims__(kMaxCl, 1, 1) __launch_bounds__(kThreads, 1)
+    svd_qr_cluster_kernel(T* __restrict__ work, T32* __restrict__ work32, const int64_t* __restrict__ blocks,
+                          int n_blocks, int group, unsigned long long* __restrict__ qctrl,
+                          const double* __restrict__ scale, int smem_elems) {
+  qr_blocks<T, T32, MAXR, kMaxCl>(work, work32, blocks, n_blocks, group, qctrl, scale, smem_elems);
+}
+
 // Up to one block per eight SMs: clusters of CL CTAs, one CTA per SM, panels of up to 6 passes of
 // CL x 256 rows in registers, 200 KB of shared memory. Up to one block per SM: the same without
 // clusters, up to 11 (complex: 6) passes of 256 rows. More blocks than SMs, one CTA each: two CTAs
@@ -786,7 +809,9 @@ __global__ void __launch_bounds__(kThreads, PER_SM)
 template <typename T, typename T32, int MAXR, int PER_SM, int CL>
 int qr_launch(void* work, void* work32, const int64_t* blocks, int n_blocks, double* scale, int64_t* qctrl,
               int qctrl_words, int sms, cudaStream_t s, bool* launched) {
-  auto kernel = svd_qr_kernel<T, T32, MAXR, PER_SM, CL>;
+  void (*kernel)(T*, T32*, const int64_t*, int, int, unsigned long long*, const double*, int);
+  if constexpr (CL > 1) kernel = svd_qr_cluster_kernel<T, T32, MAXR>;
+  else kernel = svd_qr_kernel<T, T32, MAXR, PER_SM>;
   const int smem = 200 * 1024 / PER_SM;
   cudaLaunchAttribute attr[2] = {};
   attr[0].id = cudaLaunchAttributeCooperative;
