@@ -374,12 +374,12 @@ int yb_svd_shift_prefill(void* work64, const int64_t* blocks, int n_blocks, int 
  * (M's columns are Z's rows: A^T for wide/square blocks, conj(A) for tall ones) in one
  * cooperative launch (groups of CTAs per block, group barriers with a bounded spin; on
  * timeout qctrl's error word is set), R's rows to [21], the FP32 start X32 = scale_b R and
- * W32 = I, the Householder vectors and tau kept, and Q^T formed in Z. The sweeps then run
+ * W32 = I, the Householder vectors (the panels' T above them) and tau kept, and Q^T formed in Z. The sweeps then run
  * on R's rows (row length k); yb_svd_finalize writes U's columns (wide) or Vh's rows (tall)
  * from X and the sorted W to [22]; the host completes Vh = conj(W_sorted) Q^T (wide) or
  * U = conj(Q) W_sorted^T (tall) with grouped GEMMs. qctrl: int64[qctrl_words] scratch,
- * at least n_blocks + 4 words: per block a counter of published reflectors (warps wait on
- * it with a bounded spin instead of a barrier per Householder step), then 4 words per CTA
+ * at least n_blocks + 4 words: per block a counter of published panels of columns (CTAs wait
+ * on it with a bounded spin instead of a barrier per panel), then 4 words per CTA
  * group (barrier count, generation, error flag, unused); on a timeout a group's error word
  * (qctrl[n_blocks + 4 g + 2]) is set. On a graded spectrum Jacobi from R's rows needs a few
  * FP64 sweeps where Jacobi from A's rows needs tens. */
