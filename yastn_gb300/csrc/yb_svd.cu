@@ -1057,10 +1057,11 @@ int finalize_t(void* work, void* U, double* S, void* Vh, const int64_t* blocks, 
   auto vec = svd_vectors_kernel<T>;
   auto fin = svd_finalize_kernel<T>;
   cudaError_t e = cudaSuccess;
-  if (keys > 24 * 1024) {  // with the static shared memory the total may pass 48 KB
-    e = cudaFuncSetAttribute(vec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)keys);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
+  // dynamic and static shared memory together may pass 48 KB: up to 17.5 KB static in the vectors'
+  // kernel, half a KB in the last one
+  if (keys > 24 * 1024) e = cudaFuncSetAttribute(vec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)keys);
+  if (e == cudaSuccess && smem > 32 * 1024)
+    e = cudaFuncSetAttribute(fin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) { set_cuda_error((int)e); return YB_ERR_CUDA; }
   const unsigned tiles = (unsigned)((max_k + 31) / 32), nb = (unsigned)n_blocks;
   svd_norms_kernel<T><<<dim3(tiles * 4 < 128 ? tiles * 4 : 128, nb), 256, 0, s>>>((const T*)work, S, blocks, mode, shift);
