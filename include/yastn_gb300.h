@@ -299,7 +299,8 @@ int yb_krylov_combine(const void* V, int64_t ldv, const void* coeffs, int m, int
  * state: int64[6*n_blocks + 4]: per block (max |cos| of the sweep in progress as double
  *   bits, converged flag, sweeps run in the current phase, largest |cos| of the last
  *   completed sweep, and the squared noise row norms of the FP32 and FP64 phases as double
- *   bits: (1e-5 scale_b ||A_b||_F)^2 and (1e-14 ||A_b||_F)^2, written by yb_svd_init), then
+ *   bits: (1e-5 scale_b ||A_b||_F)^2 and (1e-14 scale_b ||A_b||_F)^2 (eigh: the latter without
+ *   the scale), written by yb_svd_init), then
  *   the control words of the grid barrier (count, generation, error flag, all-converged
  *   flag). A pair with a row at or below its phase's noise norm is not rotated and does not
  *   count for convergence (rank-deficient blocks would otherwise keep O(1) cosines among
@@ -310,8 +311,8 @@ int yb_krylov_combine(const void* V, int64_t ldv, const void* coeffs, int m, int
  * scale[b] a power of two that brings the block below 1 in magnitude; scale: double
  * [n_blocks] scratch); yb_svd_sweeps with precision 32 (or yb_svd_block_sweeps);
  * yb_svd_widen (W = widen(W32)); the host orthonormalises W (Newton-Schulz with the
- * grouped GEMM, T = W^H W) and forms X = W X_0 (for eigh: yb_svd_shift_prefill, then
- * X += W A); yb_svd_sweeps with precision 64; yb_svd_finalize. yb_svd_sweeps runs every
+ * grouped GEMM, T = W^H W) and forms X = scale_b W X_0 (W A, then yb_svd_scale_x; for eigh, without
+ * the scale: yb_svd_shift_prefill, then X += W A); yb_svd_sweeps with precision 64; yb_svd_finalize. yb_svd_sweeps runs every
  * sweep of a phase in one cooperative launch (rounds separated by a grid barrier with a
  * bounded spin; on timeout the error control word is set and the kernel exits) and stops
  * after the first sweep in which each block's largest rotation |cos| was <= tol_stop, or
@@ -321,7 +322,8 @@ int yb_krylov_combine(const void* V, int64_t ldv, const void* coeffs, int m, int
  * finalize mode 1 writes eigenvalues ascending, mode 2 by descending magnitude, with
  * eigenvectors as columns of U (= W^H); mode 0 is the SVD (S descending; the vectors of
  * singular values at or below the FP64 noise norm completed to orthonormal vectors; state
- * as left by the sweeps, or NULL for a zero noise norm).
+ * as left by the sweeps, or NULL for a zero noise norm; in place of shift the scale, by which S
+ * is divided, or NULL for an X that is not scaled).
  * Replaces svd (backend_torch.py:318-319, torch_svd_gesdd.py:15-21) and eigh
  * (backend_torch.py:369-384, torch_eig_sym.py:14-32) for FP64 and complex128 blocks.
  */
@@ -366,14 +368,17 @@ int yb_svd_scale_wr(void* work64, const int64_t* blocks, int n_blocks, int dtype
                     int64_t* state, void* stream);
 int yb_svd_poison(void* U, void* V, const int64_t* blocks, int n_blocks, int dtype, const int64_t* state,
                   int which, void* stream);
+/* X <- scale_b X for every block. */
+int yb_svd_scale_x(void* work64, const int64_t* blocks, int n_blocks, int dtype, const double* scale,
+                   void* stream);
 int yb_svd_shift_prefill(void* work64, const int64_t* blocks, int n_blocks, int dtype,
                          const double* shift, void* stream);
 /* yb_svd_qr: the QR-preconditioned start (every block of the records has [16] = 1), in
  * place of yb_svd_init. Per block: scale and noise norms as yb_svd_init (the FP32 noise
- * norm is FP64's, 1e-14 scale_b ||A_b||_F), Z = X_0 in FP64, the Householder QR of M = Z^T
+ * norm is FP64's, 1e-14 scale_b ||A_b||_F), Z = scale_b X_0 in FP64, the Householder QR of M = Z^T
  * (M's columns are Z's rows: A^T for wide/square blocks, conj(A) for tall ones) in one
  * cooperative launch (groups of CTAs per block, group barriers with a bounded spin; on
- * timeout qctrl's error word is set), R's rows to [21], the FP32 start X32 = scale_b R and
+ * timeout qctrl's error word is set), R's rows (scaled by scale_b) to [21], the FP32 start X32 = R,
  * W32 = I, the Householder vectors (the panels' T above them) and tau kept, and Q^T formed in Z. The sweeps then run
  * on R's rows (row length k); yb_svd_finalize writes U's columns (wide) or Vh's rows (tall)
  * from X and the sorted W to [22]; the host completes Vh = conj(W_sorted) Q^T (wide) or

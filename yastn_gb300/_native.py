@@ -40,6 +40,7 @@ SIGNATURES = {
     'yb_svd_row_sweeps': ([_vp, _vp, _i, _vp, _i, _i, _i, _i, _d, _i, _vp, _vp, _i64, _vp], _i),
     'yb_svd_widen': ([_vp, _vp, _vp, _i, _i, _vp, _vp], _i),
     'yb_svd_block_sweeps': ([_vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _d, _i, _vp, _vp], _i),
+    'yb_svd_scale_x': ([_vp, _vp, _i, _i, _vp, _vp], _i),
     'yb_svd_shift_prefill': ([_vp, _vp, _i, _i, _vp, _vp], _i),
     'yb_svd_finalize': ([_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp], _i),
     'yb_fill_candidates': ([_vp, _vp, _i, _i, _vp], _i),

@@ -627,7 +627,7 @@ __device__ void qr_factor_panel_long(T* __restrict__ Z, T* __restrict__ V, int64
 // passes of 256 rows a panel may take in registers). False after a barrier timeout.
 template <typename T, typename T32, int MAXR, bool VS, int CL>
 __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const int64_t* __restrict__ r, int group, int rank,
-                         unsigned long long* ready, unsigned long long* ctrl, const double* scale_b, T* Vs,
+                         unsigned long long* ready, unsigned long long* ctrl, T* Vs,
                          int smem_elems, QrShared<T>& sh) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t gt = (int64_t)rank * kThreads + threadIdx.x, ngt = (int64_t)group * kThreads;
@@ -699,13 +699,12 @@ __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const i
   }
   if (!qr_all<CL>(grid_barrier(ctrl, group))) return false;
   // R rows, tau, the FP32 start
-  const double sc = scale_b ? *scale_b : 0.0;  // no FP32 Jacobi start for yb_qr
   for (int64_t e = gt; e < k * k; e += ngt) {
     const int64_t i = e / k, c = e - i * k;
     const T v = (c >= i) ? ldcg_t(Z + c * L + i) : Num<T>::zero();
     RR[e] = v;
-    if (scale_b) {
-      work32[r[R_X32] + e] = to32(rscale(v, sc));
+    if (work32) {  // no FP32 Jacobi start for yb_qr
+      work32[r[R_X32] + e] = to32(v);
       work32[r[R_W32] + e] = (i == c) ? Num<T32>::one() : Num<T32>::zero();
     }
   }
@@ -751,7 +750,7 @@ __device__ bool qr_block(T* __restrict__ work, T32* __restrict__ work32, const i
 template <typename T, typename T32, int MAXR, int CL>
 __device__ __forceinline__ void
     qr_blocks(T* __restrict__ work, T32* __restrict__ work32, const int64_t* __restrict__ blocks, int n_blocks,
-                  int group, unsigned long long* __restrict__ qctrl, const double* __restrict__ scale, int smem_elems) {
+                  int group, unsigned long long* __restrict__ qctrl, int smem_elems) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* Vs = reinterpret_cast<T*>(smem_raw);
   __shared__ QrShared<T> sh;
@@ -770,10 +769,9 @@ __device__ __forceinline__ void
   for (int b = g; b < n_blocks; b += n_groups) {
     const int64_t* r = blocks + (int64_t)b * YB_SVD_REC;
     if (!r[R_QR]) continue;
-    const double* sb = scale ? scale + b : nullptr;
     bool ok;
 #define YB_BLOCK(MAX, VS, C) \
-  qr_block<T, T32, MAX, VS, C>(work, work32, r, group, rank, qctrl + b, ctrl, sb, Vs, smem_elems, sh)
+  qr_block<T, T32, MAX, VS, C>(work, work32, r, group, rank, qctrl + b, ctrl, Vs, smem_elems, sh)
     if constexpr (CL > 1) {
       ok = r[R_LQ] <= kPairRows ? YB_BLOCK(1, true, 1)
            : kPanel * r[R_LQ] <= smem_elems ? YB_BLOCK(MAXR, true, CL) : YB_BLOCK(MAXR, false, CL);
@@ -789,16 +787,15 @@ __device__ __forceinline__ void
 template <typename T, typename T32, int MAXR, int PER_SM>
 __global__ void __launch_bounds__(kThreads, PER_SM)
     svd_qr_kernel(T* __restrict__ work, T32* __restrict__ work32, const int64_t* __restrict__ blocks, int n_blocks,
-                  int group, unsigned long long* __restrict__ qctrl, const double* __restrict__ scale, int smem_elems) {
-  qr_blocks<T, T32, MAXR, 1>(work, work32, blocks, n_blocks, group, qctrl, scale, smem_elems);
+                  int group, unsigned long long* __restrict__ qctrl, int smem_elems) {
+  qr_blocks<T, T32, MAXR, 1>(work, work32, blocks, n_blocks, group, qctrl, smem_elems);
 }
 
 template <typename T, typename T32, int MAXR>
 __global__ void __cluster_dims__(kMaxCl, 1, 1) __launch_bounds__(kThreads, 1)
     svd_qr_cluster_kernel(T* __restrict__ work, T32* __restrict__ work32, const int64_t* __restrict__ blocks,
-                          int n_blocks, int group, unsigned long long* __restrict__ qctrl,
-                          const double* __restrict__ scale, int smem_elems) {
-  qr_blocks<T, T32, MAXR, kMaxCl>(work, work32, blocks, n_blocks, group, qctrl, scale, smem_elems);
+                          int n_blocks, int group, unsigned long long* __restrict__ qctrl, int smem_elems) {
+  qr_blocks<T, T32, MAXR, kMaxCl>(work, work32, blocks, n_blocks, group, qctrl, smem_elems);
 }
 
 // Up to one block per eight SMs: clusters of CL CTAs, one CTA per SM, panels of up to 6 passes of
@@ -807,9 +804,9 @@ __global__ void __cluster_dims__(kMaxCl, 1, 1) __launch_bounds__(kThreads, 1)
 // per SM (the pipe of one is idle while the other waits) with fewer passes and half the shared
 // memory. `launched` false: the clusters do not fit the device, nothing was launched.
 template <typename T, typename T32, int MAXR, int PER_SM, int CL>
-int qr_launch(void* work, void* work32, const int64_t* blocks, int n_blocks, double* scale, int64_t* qctrl,
+int qr_launch(void* work, void* work32, const int64_t* blocks, int n_blocks, int64_t* qctrl,
               int qctrl_words, int sms, cudaStream_t s, bool* launched) {
-  void (*kernel)(T*, T32*, const int64_t*, int, int, unsigned long long*, const double*, int);
+  void (*kernel)(T*, T32*, const int64_t*, int, int, unsigned long long*, int);
   if constexpr (CL > 1) kernel = svd_qr_cluster_kernel<T, T32, MAXR>;
   else kernel = svd_qr_kernel<T, T32, MAXR, PER_SM>;
   const int smem = 200 * 1024 / PER_SM;
@@ -845,14 +842,14 @@ int qr_launch(void* work, void* work32, const int64_t* blocks, int n_blocks, dou
   if (e != cudaSuccess) { set_cuda_error((int)e); return YB_ERR_CUDA; }
   cfg.gridDim = dim3((unsigned)(n_groups * group));
   e = cudaLaunchKernelEx(&cfg, kernel, (T*)work, (T32*)work32, blocks, n_blocks, group, (unsigned long long*)qctrl,
-                         (const double*)scale, smem / (int)sizeof(T));
+                         smem / (int)sizeof(T));
   if (e != cudaSuccess) { set_cuda_error((int)e); return YB_ERR_CUDA; }
   *launched = true;
   return YB_OK;
 }
 
 template <typename T, typename T32>
-int qr_factor(void* work, void* work32, const int64_t* blocks, int n_blocks, double* scale, int64_t* qctrl,
+int qr_factor(void* work, void* work32, const int64_t* blocks, int n_blocks, int64_t* qctrl,
               int qctrl_words, cudaStream_t s) {
   constexpr int kMany = Num<T>::cplx ? 2 : 4, kFew = Num<T>::cplx ? 6 : 11;
   int dev = 0, sms = 0;
@@ -861,13 +858,13 @@ int qr_factor(void* work, void* work32, const int64_t* blocks, int n_blocks, dou
   if (e != cudaSuccess) { set_cuda_error((int)e); return YB_ERR_CUDA; }
   bool launched = false;
   if (n_blocks * 8 <= sms) {
-    const int st = qr_launch<T, T32, 6, 1, kMaxCl>(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, sms, s,
+    const int st = qr_launch<T, T32, 6, 1, kMaxCl>(work, work32, blocks, n_blocks, qctrl, qctrl_words, sms, s,
                                                    &launched);
     if (st != YB_OK || launched) return st;
   }
   return n_blocks <= sms
-             ? qr_launch<T, T32, kFew, 1, 1>(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, sms, s, &launched)
-             : qr_launch<T, T32, kMany, 2, 1>(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, sms, s, &launched);
+             ? qr_launch<T, T32, kFew, 1, 1>(work, work32, blocks, n_blocks, qctrl, qctrl_words, sms, s, &launched)
+             : qr_launch<T, T32, kMany, 2, 1>(work, work32, blocks, n_blocks, qctrl, qctrl_words, sms, s, &launched);
 }
 
 }  // namespace

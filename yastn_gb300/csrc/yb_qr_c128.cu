@@ -3,9 +3,9 @@
 
 namespace yb {
 
-int qr_factor_c128(void* work, void* work32, const int64_t* blocks, int n_blocks, double* scale, int64_t* qctrl,
+int qr_factor_c128(void* work, void* work32, const int64_t* blocks, int n_blocks, int64_t* qctrl,
                   int qctrl_words, cudaStream_t s) {
-  return qr_factor<double2, float2>(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, s);
+  return qr_factor<double2, float2>(work, work32, blocks, n_blocks, qctrl, qctrl_words, s);
 }
 
 }  // namespace yb

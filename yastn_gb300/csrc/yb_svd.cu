@@ -33,7 +33,9 @@ namespace {
 // Per-block Frobenius norm -> shift[b] (eigh: makes a symmetric block positive definite)
 // and scale[b], a power of two that brings the FP32 copy of the block (shift included)
 // below 1 in magnitude, so that FP32 squares and dot products neither overflow nor lose
-// the block to underflow. The rotations, and so W, do not depend on the scale.
+// the block to underflow. The rotations, and so W, do not depend on the scale. An SVD's FP64
+// phase works on the scaled block too (S is scaled back at the end): squared norms and inner
+// products of a block of norm 1e-140 would be subnormal there.
 // A cluster of kFroCtas CTAs per block (one SM's FP64 pipe needs 0.5 ms for the 1.7 M squares of a
 // 1296 x 1296 block); the partial sums are added in CTA order.
 constexpr int kFroCtas = 8;
@@ -76,8 +78,9 @@ __global__ void __cluster_dims__(kFroCtas, 1, 1)
     int e = 0;
     if (bound > 0.0 && bound <= 1.0e300) frexp(bound, &e);
     scale[blockIdx.y] = ldexp(1.0, -e);
-    // the FP32 phase works on scale * A, the FP64 phase on A itself
-    const double t32 = (r[R_QR] ? kNoise64 : kNoise32) * fro * ldexp(1.0, -e), t64 = kNoise64 * fro;
+    // the FP32 phase works on scale * A, the FP64 phase too (eigh: on A + shift itself)
+    const double sf = fro * ldexp(1.0, -e);
+    const double t32 = (r[R_QR] ? kNoise64 : kNoise32) * sf, t64 = kNoise64 * (shift != nullptr ? fro : sf);
     state[(int64_t)blockIdx.y * ST_REC + ST_THR32] = __double_as_longlong(t32 * t32);
     state[(int64_t)blockIdx.y * ST_REC + ST_THR64] = __double_as_longlong(t64 * t64);
   }
@@ -243,6 +246,18 @@ __global__ void svd_scale_wr_kernel(T64* __restrict__ work64, const int64_t* __r
     Rs[e] = k < 2 ? R[e]
                   : rscale(R[e], __longlong_as_double(((long long)2046 << 52) - __double_as_longlong(real_of(d[i]))));
   }
+}
+
+// X = scale_b X, for an SVD whose X was formed from A itself.
+template <typename T64>
+__global__ void svd_scale_x_kernel(T64* __restrict__ work64, const int64_t* __restrict__ blocks,
+                                   const double* __restrict__ scale) {
+  const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
+  const int64_t n = r[R_K] * r[R_L];
+  const double c = scale[blockIdx.y];
+  T64* X = work64 + r[R_X];
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
+    X[e] = rscale(X[e], c);
 }
 
 // X = shift_b * W (eigh: the FP64 phase then adds W A with the grouped GEMM, X = W (A + shift I)).
@@ -628,17 +643,20 @@ int launch_block_sweeps(T* work, const int64_t* blocks, int n_blocks, const int3
 
 // Z = X_0 in FP64 (A, or A^H for tall blocks). Records with [16] = 2 (yb_qr, M = A): Z's
 // rows are the first k columns of A (length L = m).
+// (scaled by scale[b], a power of two, where it is given: see block_fro_kernel).
 template <typename T>
-__global__ void svd_qr_load_kernel(const T* __restrict__ A, T* __restrict__ work, const int64_t* __restrict__ blocks) {
+__global__ void svd_qr_load_kernel(const T* __restrict__ A, T* __restrict__ work, const int64_t* __restrict__ blocks,
+                                   const double* __restrict__ scale) {
   const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
   if (!r[R_QR]) return;
   const int64_t m = r[R_M], n = r[R_N], k = r[R_K], L = r[R_LQ];
   const bool tall = m > n, plain = r[R_QR] == 2;
+  const double sc = scale != nullptr ? scale[blockIdx.y] : 1.0;
   const T* a = A + r[R_A];
   T* Z = work + r[R_Z];
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < k * L; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = e / L, l = e - i * L;
-    Z[e] = plain ? a[l * n + i] : (tall ? cconj_(a[l * n + i]) : a[e]);
+    Z[e] = rscale(plain ? a[l * n + i] : (tall ? cconj_(a[l * n + i]) : a[e]), sc);
   }
 }
 
@@ -814,11 +832,13 @@ __global__ void __launch_bounds__(256) svd_vectors_kernel(T* __restrict__ work, 
        });
 }
 
-// S sorted in place; for an SVD the rows at noise level counted and small completions done here.
+// S sorted in place (mode 0: and divided by scale[b], where that is given); for an SVD the rows at
+// noise level counted and small completions done here.
 template <typename T>
 __global__ void __launch_bounds__(1024) svd_finalize_kernel(T* __restrict__ U, double* __restrict__ S,
                                                             T* __restrict__ Vh, const int64_t* __restrict__ blocks,
-                                                            int mode, const int64_t* __restrict__ state,
+                                                            int mode, const double* __restrict__ scale,
+                                                            const int64_t* __restrict__ state,
                                                             int64_t* __restrict__ n_small) {
   extern __shared__ unsigned char smem_raw[];
   const int64_t* r = blocks + (int64_t)blockIdx.x * YB_SVD_REC;
@@ -842,9 +862,10 @@ __global__ void __launch_bounds__(1024) svd_finalize_kernel(T* __restrict__ U, d
   __syncthreads();
   const double zthr = mode == 0 && state ? sqrt(__longlong_as_double((long long)state[(int64_t)blockIdx.x * ST_REC + ST_THR64]))
                                          : 0.0;
+  const double unscale = mode == 0 && scale ? 1.0 / scale[blockIdx.x] : 1.0;  // a power of two
   for (int i = threadIdx.x; i < k; i += blockDim.x) {
     const double v = cim[i];
-    Sb[final_rank(key, (int)k, i)] = v;
+    Sb[final_rank(key, (int)k, i)] = v * unscale;
     if (!(v > zthr && v > 0.0)) atomicAdd(&n_zero, 1);
   }
   __syncthreads();
@@ -1015,9 +1036,9 @@ int launch_sweeps(T* work, const int64_t* blocks, int n_blocks, const int32_t* p
 }  // namespace
 
 // yb_qr_f64.cu, yb_qr_c128.cu: the factorisation of every block (yb_qr.cuh)
-int qr_factor_f64(void* work, void* work32, const int64_t* blocks, int n_blocks, double* scale, int64_t* qctrl,
+int qr_factor_f64(void* work, void* work32, const int64_t* blocks, int n_blocks, int64_t* qctrl,
                   int qctrl_words, cudaStream_t s);
-int qr_factor_c128(void* work, void* work32, const int64_t* blocks, int n_blocks, double* scale, int64_t* qctrl,
+int qr_factor_c128(void* work, void* work32, const int64_t* blocks, int n_blocks, int64_t* qctrl,
                    int qctrl_words, cudaStream_t s);
 
 template <typename T>
@@ -1042,9 +1063,9 @@ template <typename T>
 int qr_t(const void* a, void* work, void* work32, const int64_t* blocks, int n_blocks, int64_t* state, double* scale,
          int64_t* qctrl, int qctrl_words, cudaStream_t s) {
   if (state) block_fro_kernel<T><<<dim3(kFroCtas, (unsigned)n_blocks), 256, 0, s>>>((const T*)a, blocks, nullptr, scale, state);
-  svd_qr_load_kernel<T><<<dim3(64, (unsigned)n_blocks), 256, 0, s>>>((const T*)a, (T*)work, blocks);
-  const int st = Num<T>::cplx ? qr_factor_c128(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, s)
-                              : qr_factor_f64(work, work32, blocks, n_blocks, scale, qctrl, qctrl_words, s);
+  svd_qr_load_kernel<T><<<dim3(64, (unsigned)n_blocks), 256, 0, s>>>((const T*)a, (T*)work, blocks, scale);
+  const int st = Num<T>::cplx ? qr_factor_c128(work, work32, blocks, n_blocks, qctrl, qctrl_words, s)
+                              : qr_factor_f64(work, work32, blocks, n_blocks, qctrl, qctrl_words, s);
   if (st != YB_OK) return st;
   if (state) svd_state_reset_kernel<<<n_blocks, 32, 0, s>>>(state);
   return check_launch();
@@ -1066,7 +1087,7 @@ int finalize_t(void* work, void* U, double* S, void* Vh, const int64_t* blocks, 
   const unsigned tiles = (unsigned)((max_k + 31) / 32), nb = (unsigned)n_blocks;
   svd_norms_kernel<T><<<dim3(tiles * 4 < 128 ? tiles * 4 : 128, nb), 256, 0, s>>>((const T*)work, S, blocks, mode, shift);
   vec<<<dim3(tiles, nb), 256, keys, s>>>((T*)work, (T*)U, S, (T*)Vh, blocks, mode, state);
-  fin<<<nb, 1024, smem, s>>>((T*)U, S, (T*)Vh, blocks, mode, state, n_small);
+  fin<<<nb, 1024, smem, s>>>((T*)U, S, (T*)Vh, blocks, mode, shift, state, n_small);
   return check_launch();
 }
 
@@ -1258,6 +1279,17 @@ int yb_svd_shift_prefill(void* work64, const int64_t* blocks, int n_blocks, int 
     yb::svd_shift_prefill_kernel<double2><<<grid, 256, 0, s>>>((double2*)work64, blocks, shift);
   else
     return YB_ERR_INVALID;
+  return yb::check_launch();
+}
+
+int yb_svd_scale_x(void* work64, const int64_t* blocks, int n_blocks, int dtype, const double* scale, void* stream) {
+  if (n_blocks == 0) return YB_OK;
+  if (!work64 || !blocks || !scale) return YB_ERR_INVALID;
+  const dim3 grid(64, (unsigned)n_blocks);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (dtype == YB_F64) yb::svd_scale_x_kernel<double><<<grid, 256, 0, s>>>((double*)work64, blocks, scale);
+  else if (dtype == YB_C128) yb::svd_scale_x_kernel<double2><<<grid, 256, 0, s>>>((double2*)work64, blocks, scale);
+  else return YB_ERR_INVALID;
   return yb::check_launch();
 }
 

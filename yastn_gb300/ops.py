@@ -707,6 +707,7 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
             run_gemm(plan.xform, w64, data, w64, beta=1.0)
     else:
         run_gemm(plan.xform, w64, data, w64)
+        N.call('yb_svd_scale_x', _ptr(w64), _ptr(dblocks), nb, code, _ptr(aux), st)
     tol64 = TOL_STOP64_QR if plan.qr else (TOL_STOP64 if mode == 0 else TOL_STOP64_EIGH)
     if BLOCKED_FP64[0] and _row_sweeps(plan, 64, code):
         _run_row_sweeps(plan, w64, dblocks, dpairs, nb, 64, code, max_sweeps, tol64, state)
@@ -719,7 +720,7 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
         N.call('yb_svd_sweeps', _ptr(w64), _ptr(dblocks), nb, _ptr(dpairs), len(plan.pair_items), plan.max_rounds,
                64, code, max_sweeps, tol64, _ptr(state), st)
     N.call('yb_svd_finalize', _ptr(w64), _ptr(U), _ptr(S), _ptr(V) if V is not None else 0, _ptr(dblocks), nb, code,
-           plan.max_k, mode, sp, _ptr(state), _ptr(n_small) if n_small is not None else 0, st, launches=3)
+           plan.max_k, mode, sp if mode else _ptr(aux), _ptr(state), _ptr(n_small) if n_small is not None else 0, st, launches=3)
     if plan.qr:  # the factor that comes from Q: Vh = conj(W) Q^T (wide), U = conj(Q) W^T (tall)
         if emu:
             run_emulated(emu['qv'], w64, w64, V)
