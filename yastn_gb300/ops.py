@@ -474,7 +474,7 @@ def _ozaki_arrays(plan, tile_n, dev):
 def run_emulated(eg, a, b, c):
     """The products of ``eg`` (P.EmulatedGemm) from the flat tensors a and b into c: one split
     launch, one GEMM launch, and a native FP64 launch for the short ones."""
-    if eg.native.outs.size:
+    if eg.native.outs.size or eg.native.split is not None:  # all of its outputs may be split ones
         run_gemm(eg.native, a, b, c)
     if eg.n_tiles == 0:
         return c
