@@ -548,18 +548,35 @@ def transpose_plan(axes, meta_transpose, size):
 # ----------------------------------------------------------------------------- grouped GEMM
 
 class GemmPlan:
-    """Grouped GEMM records: the outputs computed directly (outs, terms, tiles) and, when
-    some outputs' K range is split, their partial products and reduction (``split``)."""
+    """Grouped GEMM records of an output list [(c_off, m, n, ldc, [term tuples])]: the outputs computed
+    directly (outs, terms, tiles) and, when they make too few tiles for the GPU, those with a long K:
+    their K chunks, computed into a workspace, and the reduction (``split``; not with
+    ``allow_split=False``). The records are built where they are first used: a plan whose outputs run
+    on fine tiles (``fine_gemm``; not with ``allow_fine=False``) has no use for them."""
 
-    def __init__(self, outs, terms, tiles, flops, split=None):
-        self.outs = outs
-        self.terms = terms
-        self.tiles = tiles
-        self.flops = flops  # real multiply-adds x 2 (complex counted by the caller)
-        self.split = split
-        # every tile a short skinny one: the plan runs on the kernel of those alone
-        self.all_short = bool(len(tiles)) and bool((tiles[:, 3] == 2).all())
+    def __init__(self, out_list, allow_split=True, allow_fine=True):
+        self.out_list = out_list
+        self.allow_split, self.allow_fine = allow_split, allow_fine
+        # real multiply-adds x 2 (complex counted by the caller)
+        self.flops = sum(2 * m * n * t[2] for _, m, n, _, tl in out_list for t in tl)
         self._dev = {}
+
+    def __getattr__(self, name):
+        if name not in ('outs', 'terms', 'tiles', 'split', 'all_short') or 'out_list' not in self.__dict__:
+            raise AttributeError(name)
+        direct, split = _split_outputs(self.out_list) if self.allow_split else (self.out_list, None)
+        outs, terms = _records(direct)
+        tiles = _tiles_for(outs, terms)
+        # all_short: every tile a short skinny one: the plan runs on the kernel of those alone
+        self.__dict__.update(outs=outs, terms=terms, tiles=tiles, split=split,
+                             all_short=bool(len(tiles)) and bool((tiles[:, 3] == 2).all()))
+        return self.__dict__[name]
+
+    def has_work(self):
+        """Whether there is an element to compute."""
+        if 'out_list' not in self.__dict__:  # read from an older plan file
+            return len(self.tiles) > 0 or self.split is not None
+        return any(o[1] and o[2] for o in self.out_list)
 
 
 class SplitK:
@@ -682,52 +699,43 @@ def _chunks(tl, ck):
 
 
 def _records(out_list):
-    outs, terms, flops = [], [], 0
+    outs, terms = [], []
     for c_off, m, n, ldc, tl in out_list:
         t0 = len(terms)
-        for t in tl:
-            terms.append(t)
-            flops += 2 * m * n * t[2]
+        terms.extend(tl)
         outs.append((c_off, m, n, ldc, t0, len(terms), 0, 0))
-    outs = np.array(outs, dtype=np.int64).reshape(-1, GEMM_OUT_REC)
-    terms = np.array(terms, dtype=np.int64).reshape(-1, GEMM_TERM_REC)
-    return outs, terms, flops
+    return (np.array(outs, dtype=np.int64).reshape(-1, GEMM_OUT_REC),
+            np.array(terms, dtype=np.int64).reshape(-1, GEMM_TERM_REC))
 
 
 def _pack_gemm(out_list, allow_split=True):
-    """out_list: [(c_off, m, n, ldc, [term tuples])] -> GemmPlan. When the outputs make
-    too few tiles for the GPU, outputs with a long K are split into K chunks computed into
-    a workspace and summed by a reduction pass (split-K; not with ``allow_split=False``)."""
-    ck = _split_chunk_k(out_list) if allow_split else None
-    split, whole = None, out_list
-    if ck is not None:
-        direct, parts, red, tasks, ws = [], [], [], [], 0
-        for c_off, m, n, ldc, tl in out_list:
-            if m == 0 or n == 0 or sum(t[2] for t in tl) < 2 * ck:
-                direct.append((c_off, m, n, ldc, tl))
-                continue
-            kk = sum(t[2] for t in tl)
-            nch = -(-kk // ck)
-            ch = _chunks(tl, -(-(-(-kk // nch)) // 16) * 16)  # nch near-equal chunks, multiples of 16
-            for ci, cl in enumerate(ch):
-                parts.append((ws + ci * m * n, m, n, n, cl))
-            ri = len(red)
-            red.append((c_off, m, n, ldc, ws, len(ch), 0, 0))
-            tasks.extend((ri, it) for it in range((m * n + GEMM_RED_ITEM - 1) // GEMM_RED_ITEM))
-            ws += len(ch) * m * n
-        po, pt, _ = _records(parts)
-        split = SplitK(po, pt, _tiles_for(po, pt), np.array(red, dtype=np.int64).reshape(-1, GEMM_RED_REC),
-                       np.array(tasks, dtype=np.int32).reshape(-1, 2), ws)
-        out_list = direct
-    outs, terms, _ = _records(out_list)
-    flops = sum(2 * m * n * t[2] for _, m, n, _, tl in out_list for t in tl)
-    if split is not None:
-        flops += sum(2 * int(o[1]) * int(o[2]) * int(t[2]) for o in split.outs
-                     for t in split.terms[int(o[4]):int(o[5])])
-    plan = GemmPlan(outs, terms, _tiles_for(outs, terms), flops, split)
-    if allow_split:
-        plan.out_list = whole
-    return plan
+    """The GemmPlan of an output list, on fine tiles where `fine_gemm` takes it or, without splits
+    (``allow_split=False``: no workspace), on its own ones."""
+    return GemmPlan(out_list, allow_split, allow_fine=allow_split)
+
+
+def _split_outputs(out_list):
+    """(outputs computed directly, SplitK of those with a long K or None)."""
+    ck = _split_chunk_k(out_list)
+    if ck is None:
+        return out_list, None
+    direct, parts, red, tasks, ws = [], [], [], [], 0
+    for c_off, m, n, ldc, tl in out_list:
+        if m == 0 or n == 0 or sum(t[2] for t in tl) < 2 * ck:
+            direct.append((c_off, m, n, ldc, tl))
+            continue
+        kk = sum(t[2] for t in tl)
+        nch = -(-kk // ck)
+        ch = _chunks(tl, -(-(-(-kk // nch)) // 16) * 16)  # nch near-equal chunks, multiples of 16
+        for ci, cl in enumerate(ch):
+            parts.append((ws + ci * m * n, m, n, n, cl))
+        ri = len(red)
+        red.append((c_off, m, n, ldc, ws, len(ch), 0, 0))
+        tasks.extend((ri, it) for it in range((m * n + GEMM_RED_ITEM - 1) // GEMM_RED_ITEM))
+        ws += len(ch) * m * n
+    po, pt = _records(parts)
+    return direct, SplitK(po, pt, _tiles_for(po, pt), np.array(red, dtype=np.int64).reshape(-1, GEMM_RED_REC),
+                          np.array(tasks, dtype=np.int32).reshape(-1, 2), ws)
 
 
 FINE_TILE = 32           # tiles of yb_grouped_gemm_fine
@@ -751,13 +759,13 @@ def fine_gemm(plan):
     """The FineGemm of ``plan``, or None where it has no 64 x 64 tiles or only short products.
     Measured against the 64 x 64 tiles (us): sectors of 10..129 140 -> 40, up to 240 251 -> 95, up to
     422 558 -> 319, up to 704 2246 -> 1994, complex128 up to 129 531 -> 113."""
-    got = plan.__dict__.get('_fine', 0)
-    if got != 0:
-        return got
-    plan._fine = None
-    out_list = plan.__dict__.get('out_list')
-    if out_list is None:
-        return None
+    if '_fine' not in plan.__dict__:
+        out_list = plan.__dict__.get('out_list')  # none in an older plan file
+        plan._fine = _fine_gemm(out_list) if out_list is not None and plan.__dict__.get('allow_fine', True) else None
+    return plan._fine
+
+
+def _fine_gemm(out_list):
     rest, mine = [], []
     for o in out_list:
         kind0 = o[1] and o[2] and tile_kind(o[1], o[2], [t[2] for t in o[4]]) == 0
@@ -774,14 +782,12 @@ def fine_gemm(plan):
         return -(-o[1] // FINE_TILE) * -(-o[2] // FINE_TILE)
     work = sum(n_tiles(o) * sum(t[2] for t in o[4]) for o in mine)
     ck = max(FINE_MIN_K, -(-work // FINE_UNITS) + 15 & ~15)
-    outs, terms, red, tasks, tiles, ws = [], [], [], [], [], 0
+    outs, terms, red, tasks, ws = [], [], [], [], 0
 
     def add(c_off, m, n, ldc, tl, partial):
-        oi, t0 = len(outs), len(terms)
+        t0 = len(terms)
         terms.extend(tl)
         outs.append((c_off, m, n, ldc, t0, len(terms), int(partial), 0))
-        kk = sum(t[2] for t in tl)
-        tiles.extend((kk, oi, tr, tc) for tr in range(-(-m // FINE_TILE)) for tc in range(-(-n // FINE_TILE)))
     for c_off, m, n, ldc, tl in mine:
         kk = sum(t[2] for t in tl)
         nch = max(1, (2 * kk + ck) // (2 * ck))
@@ -794,14 +800,19 @@ def fine_gemm(plan):
         tasks.extend((len(red), it) for it in range(-(-m * n // GEMM_RED_ITEM)))
         red.append((c_off, m, n, ldc, ws, len(ch), 0, 0))
         ws += len(ch) * m * n
-    tiles.sort(key=lambda x: -x[0])
-    plan._fine = FineGemm(_pack_gemm(rest, allow_split=False) if rest else None,
-                          np.array(outs, dtype=np.int64).reshape(-1, GEMM_OUT_REC),
-                          np.array(terms, dtype=np.int64).reshape(-1, GEMM_TERM_REC),
-                          np.array([(oi, tr, tc, 0) for _, oi, tr, tc in tiles], dtype=np.int32).reshape(-1, 4),
-                          np.array(red, dtype=np.int64).reshape(-1, GEMM_RED_REC),
-                          np.array(tasks, dtype=np.int32).reshape(-1, 2), ws)
-    return plan._fine
+    outs = np.array(outs, dtype=np.int64).reshape(-1, GEMM_OUT_REC)
+    terms = np.array(terms, dtype=np.int64).reshape(-1, GEMM_TERM_REC)
+    # all tiles of an output, row by row; those of the longest K first
+    order = sorted(range(len(outs)), key=lambda i: -int(terms[outs[i, 4]:outs[i, 5], 2].sum()))
+    tiles = []
+    for oi in order:
+        nr, nc = -(-int(outs[oi, 1]) // FINE_TILE), -(-int(outs[oi, 2]) // FINE_TILE)
+        t = np.zeros((nr * nc, 4), dtype=np.int32)
+        t[:, 0], t[:, 1], t[:, 2] = oi, np.repeat(np.arange(nr), nc), np.tile(np.arange(nc), nr)
+        tiles.append(t)
+    return FineGemm(GemmPlan(rest, allow_fine=False) if rest else None, outs, terms, np.concatenate(tiles),
+                    np.array(red, dtype=np.int64).reshape(-1, GEMM_RED_REC),
+                    np.array(tasks, dtype=np.int32).reshape(-1, 2), ws)
 
 
 def dot_coverage(meta_dot):

@@ -375,7 +375,7 @@ def dot_ozaki(A, B, meta_dot, Dsize, slices=OZAKI_SLICES):
         tc = plan.tuned_tc
     # the native sectors (disjoint outputs) run on a second stream beside the split and the
     # emulated GEMM, and the current stream waits for them (a fork and join inside a CUDA graph)
-    fork = len(plan.native.tiles) > 0 or plan.native.split is not None
+    fork = plan.native.has_work()
     if fork:
         main, side, keep = torch.cuda.current_stream(A.device), _side_stream(A.device), []
         side.wait_stream(main)
@@ -474,7 +474,7 @@ def _ozaki_arrays(plan, tile_n, dev):
 def run_emulated(eg, a, b, c):
     """The products of ``eg`` (P.EmulatedGemm) from the flat tensors a and b into c: one split
     launch, one GEMM launch, and a native FP64 launch for the short ones."""
-    if eg.native.outs.size or eg.native.split is not None:  # all of its outputs may be split ones
+    if eg.native.has_work():
         run_gemm(eg.native, a, b, c)
     if eg.n_tiles == 0:
         return c
