@@ -123,7 +123,8 @@ int yb_map_gather(const void* src, void* dst, int dtype, const int32_t* map, int
 /* ==== family (b): grouped sum-of-products GEMM ========================================
  * For every output block o:  C_o = alpha * sum_{t in terms(o)} op(A_t) op(B_t) + beta * C_o
  * outs: n_out records of YB_GEMM_OUT_REC int64:
- *   [0] c offset (elements) [1] m [2] n [3] ldc [4] first term [5] end term
+ *   [0] c offset (elements) [1] m [2] n [3] ldc [4] first term [5] end term  [6] partial product
+ *   (yb_grouped_gemm_fine) [7] flag index (yb_grouped_gemm_flagged)
  * terms: records of YB_GEMM_TERM_REC int64:
  *   [0] a offset [1] b offset [2] k [3] a row stride [4] a col stride
  *   [5] b row stride [6] b col stride [7] flags (bit0: conj A, bit1: conj B)
@@ -153,6 +154,11 @@ int yb_grouped_gemm(const void* a, const void* b, void* c, int dtype,
 int yb_grouped_gemm_fine(const void* a, const void* b, void* c, void* ws, int dtype, const int64_t* outs,
                          const int64_t* terms, const int32_t* tiles, int n_tiles, double alpha, double beta,
                          void* stream);
+/* yb_grouped_gemm_flagged: the same (C assigned, no partial products) for the outputs with
+ * flags[output record [7]] != 0 only; the others are left as they are. */
+int yb_grouped_gemm_flagged(const void* a, const void* b, void* c, int dtype, const int64_t* outs,
+                            const int64_t* terms, const int32_t* tiles, int n_tiles, const int64_t* flags,
+                            void* stream);
 /* yb_grouped_gemm_short: yb_grouped_gemm for plans whose tiles are all of kind 2 (the
  * contractions of a tensor with a small MPO block): a kernel of its own with few registers,
  * eight warps per SM scheduler, all loads of a thread's columns issued before its FMAs. */
@@ -368,6 +374,13 @@ int yb_svd_scale_wr(void* work64, const int64_t* blocks, int n_blocks, int dtype
                     int64_t* state, void* stream);
 int yb_svd_poison(void* U, void* V, const int64_t* blocks, int n_blocks, int dtype, const int64_t* state,
                   int which, void* stream);
+/* flags[b] = 1 for the blocks (with a QR start, k >= k_min) whose products with W must not be formed
+ * from digits: those where the factor W Q^T would lose entries that are small for their row of W and
+ * their component of Q at once (blocks graded by columns). W as widened, Q^T and R as left by
+ * yb_svd_qr; at_masks: per block its offset in masks, scratch of (2 (k + L) ceil(k / 32) + k + L) int32
+ * words per block. flags zeroed by the caller. Three launches. */
+int yb_svd_graded(const void* work64, const int64_t* blocks, int n_blocks, int dtype, int k_min, const int64_t* state,
+                  const int64_t* at_masks, int32_t* masks, int64_t* flags, void* stream);
 /* X <- scale_b X for every block. */
 int yb_svd_scale_x(void* work64, const int64_t* blocks, int n_blocks, int dtype, const double* scale,
                    void* stream);

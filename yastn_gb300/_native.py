@@ -25,6 +25,7 @@ SIGNATURES = {
     'yb_gemm_reduce': ([_vp, _vp, _i, _vp, _vp, _i, _d, _d, _vp], _i),
     'yb_grouped_gemm': ([_vp, _vp, _vp, _i, _vp, _vp, _vp, _i, _d, _d, _vp], _i),
     'yb_grouped_gemm_fine': ([_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _i, _d, _d, _vp], _i),
+    'yb_grouped_gemm_flagged': ([_vp, _vp, _vp, _i, _vp, _vp, _vp, _i, _vp, _vp], _i),
     'yb_grouped_gemm_short': ([_vp, _vp, _vp, _i, _vp, _vp, _vp, _i, _d, _d, _vp], _i),
     'yb_svd_init': ([_vp, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp], _i),
     'yb_svd_qr': ([_vp, _vp, _vp, _vp, _i, _i, _vp, _vp, _vp, _i, _vp], _i),
@@ -40,6 +41,7 @@ SIGNATURES = {
     'yb_svd_row_sweeps': ([_vp, _vp, _i, _vp, _i, _i, _i, _i, _d, _i, _vp, _vp, _i64, _vp], _i),
     'yb_svd_widen': ([_vp, _vp, _vp, _i, _i, _vp, _vp], _i),
     'yb_svd_block_sweeps': ([_vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _d, _i, _vp, _vp], _i),
+    'yb_svd_graded': ([_vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp], _i),
     'yb_svd_scale_x': ([_vp, _vp, _i, _i, _vp, _vp], _i),
     'yb_svd_shift_prefill': ([_vp, _vp, _i, _i, _vp, _vp], _i),
     'yb_svd_finalize': ([_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp], _i),

@@ -1103,17 +1103,53 @@ def emulated_gemm(out_list, s, cplx=False):
                            'outs' + sfx: outs, 'tiles' + sfx: tiles, 'n_tiles': len(tiles)})
 
 
+class FlaggedGemm:
+    """Products (one term per output, C assigned) of the blocks whose flag is set, for
+    yb_grouped_gemm_flagged: whole K (a launch that finds no flag set costs its tiles' look alone)."""
+
+    def __init__(self, out_list, blocks):
+        outs, terms, tiles = [], [], []
+        for (c_off, m, n, ldc, tl), b in sorted(zip(out_list, blocks), key=lambda x: -x[0][4][0][2]):
+            tiles.extend((len(outs), tr, tc, 0) for tr in range(-(-m // FINE_TILE)) for tc in range(-(-n // FINE_TILE)))
+            outs.append((c_off, m, n, ldc, len(terms), len(terms) + 1, 0, b))
+            terms.extend(tl)
+        self.outs = np.array(outs, dtype=np.int64).reshape(-1, GEMM_OUT_REC)
+        self.terms = np.array(terms, dtype=np.int64).reshape(-1, GEMM_TERM_REC)
+        self.tiles = np.array(tiles, dtype=np.int32).reshape(-1, 4)
+        self._dev = {}
+
+
+class SvdGuard:
+    """The same products as the emulated ones of a block SVD with a QR start, by name, for the blocks
+    that yb_svd_graded flags, and the offsets and the size of its scratch."""
+
+    def __init__(self, plan, lists):
+        at, size = [], 0
+        for r in plan.blocks:
+            k, L = int(r[9]), int(r[17])
+            at.append(size)
+            size += 2 * (k + L) * (-(-k // 32)) + k + L
+        self.at, self.size = np.array(at, dtype=np.int64), size
+        self.gemm = {}
+        for name, lst in lists.items():
+            keep = [(o, b) for o, b in lst if o[4][0][2] >= OZAKI_MIN_DIM]  # the shorter ones are native
+            self.gemm[name] = FlaggedGemm([o for o, _ in keep], [b for _, b in keep])
+        self._dev = {}
+
+
 def svd_emulated(plan, s, cplx):
     """The products of the block SVD's FP64 steps as emulated GEMMs, from the records of ``plan``:
     T = W^H W and W' = W (1.5 - 0.5 T) from W and back from Wn, X = W X_0 (QR start: W R; else W A
-    into T, ``xa``), and the factor that comes from Q."""
+    into T, ``xa``), and the factor that comes from Q; for a QR start with its SvdGuard ('guard': None
+    where all products are native ones)."""
     got = plan.__dict__.get('_emulated')
-    if got is not None:
+    if got is not None and 'guard' in got:
         return got
     w0, t0, n0, ws = plan.w_range
     gram, ns, gram2, ns2, xr, xa, qu, qv = [], [], [], [], [], [], [], []
     cj = int(cplx)
-    for r in plan.blocks:
+    of_q = {'qu': [], 'qv': []}
+    for b, r in enumerate(plan.blocks):
         a0, m, n, u0, v0, x0, W, k, tall = (int(r[i]) for i in (0, 1, 2, 3, 5, 6, 7, 9, 12))
         T, Wn = W + ws, W + 2 * ws
         gram.append((T, k, k, k, [(W, W, k, 1, k, k, 1, cj)]))
@@ -1127,11 +1163,18 @@ def svd_emulated(plan, s, cplx):
                 qu.append((u0, m, k, k, [(Z, WS, k, 1, LQ, 1, k, cj)]))
             else:
                 qv.append((v0, k, n, n, [(WS, Z, k, k, 1, LQ, 1, 0)]))
+            of_q['qu' if tall else 'qv'].append(b)
         elif m == n:
             xa.append((T, k, k, k, [(W, a0, k, k, 1, n, 1, 0)]))
     got = {name: emulated_gemm(lst, s, cplx)
            for name, lst in (('gram', gram), ('ns', ns), ('gram2', gram2), ('ns2', ns2), ('xr', xr), ('xa', xa),
                              ('qu', qu), ('qv', qv))}
+    got['guard'] = None
+    if plan.qr and got['gram'].n_tiles:
+        lists = {name: list(zip(lst, range(len(lst)))) for name, lst in (('gram', gram), ('ns', ns), ('gram2', gram2),
+                                                                         ('ns2', ns2))}
+        lists.update(qu=list(zip(qu, of_q['qu'])), qv=list(zip(qv, of_q['qv'])))
+        got['guard'] = SvdGuard(plan, lists)
     plan._emulated = got
     return got
 

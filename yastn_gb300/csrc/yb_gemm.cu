@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(kThreads) grouped_gemm_kernel(const typename F
 // threads, 2 x 2 outputs each (eight warps of 8 rows x 16 columns: warps outside a small sector skip
 // their FMAs), the next 16 k loaded into registers while the current ones are multiplied. Outputs
 // with [6] = 1 go to the workspace as they are (partial products), the others to C with alpha and
-// beta. Bound: the DFMA rate. Measured against 64 x 64 tiles: 13 sectors of 10..129 140 -> 40 us (16 us
+// beta. With flags, only the outputs whose flag (at [7]) is set are computed. Bound: the DFMA rate. Measured against 64 x 64 tiles: 13 sectors of 10..129 140 -> 40 us (16 us
 // of FMAs), of 16..704 2246 -> 1994 us, complex128 sectors of 10..129 531 -> 113 us.
 constexpr int kFine = 32;
 
@@ -504,13 +504,14 @@ __global__ void __launch_bounds__(kThreads) fine_gemm_kernel(const typename F::T
                                                               const int64_t* __restrict__ outs,
                                                               const int64_t* __restrict__ terms,
                                                               const int32_t* __restrict__ tiles, double alpha,
-                                                              double beta) {
+                                                              double beta, const int64_t* __restrict__ flags) {
   using T = typename F::T;
   constexpr int kL = kFine * kK / kThreads;  // elements of each operand a thread loads per step
   __shared__ __align__(16) T As[2][kK][kFine + 2];
   __shared__ __align__(16) T Bs[2][kK][kFine + 2];
   const int4 tl = reinterpret_cast<const int4*>(tiles)[blockIdx.x];
   const int64_t* orec = outs + (int64_t)tl.x * YB_GEMM_OUT_REC;
+  if (flags != nullptr && flags[orec[7]] == 0) return;
   const int64_t c_off = orec[0], m = orec[1], n = orec[2], ldc = orec[3];
   const int t0 = (int)orec[4], t1 = (int)orec[5];
   const bool partial = orec[6] != 0;
@@ -665,22 +666,35 @@ extern "C" int yb_gemm_reduce(void* c, const void* p, int dtype, const int64_t* 
   return yb::check_launch();
 }
 
-extern "C" int yb_grouped_gemm_fine(const void* a, const void* b, void* c, void* ws, int dtype, const int64_t* outs,
-                                    const int64_t* terms, const int32_t* tiles, int n_tiles, double alpha,
-                                    double beta, void* stream) {
+static int fine_gemm(const void* a, const void* b, void* c, void* ws, int dtype, const int64_t* outs,
+                     const int64_t* terms, const int32_t* tiles, int n_tiles, double alpha, double beta,
+                     const int64_t* flags, void* stream) {
   if (n_tiles == 0) return YB_OK;
   if (!a || !b || !c || !outs || !terms || !tiles || n_tiles < 0) return YB_ERR_INVALID;
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype == YB_F64) {
     yb::fine_gemm_kernel<yb::Real><<<n_tiles, yb::kThreads, 0, s>>>((const double*)a, (const double*)b, (double*)c,
-                                                                    (double*)ws, outs, terms, tiles, alpha, beta);
+                                                                    (double*)ws, outs, terms, tiles, alpha, beta, flags);
   } else if (dtype == YB_C128) {
     yb::fine_gemm_kernel<yb::Cplx><<<n_tiles, yb::kThreads, 0, s>>>((const double2*)a, (const double2*)b, (double2*)c,
-                                                                    (double2*)ws, outs, terms, tiles, alpha, beta);
+                                                                    (double2*)ws, outs, terms, tiles, alpha, beta, flags);
   } else {
     return YB_ERR_INVALID;
   }
   return yb::check_launch();
+}
+
+extern "C" int yb_grouped_gemm_fine(const void* a, const void* b, void* c, void* ws, int dtype, const int64_t* outs,
+                                    const int64_t* terms, const int32_t* tiles, int n_tiles, double alpha,
+                                    double beta, void* stream) {
+  return fine_gemm(a, b, c, ws, dtype, outs, terms, tiles, n_tiles, alpha, beta, nullptr, stream);
+}
+
+extern "C" int yb_grouped_gemm_flagged(const void* a, const void* b, void* c, int dtype, const int64_t* outs,
+                                       const int64_t* terms, const int32_t* tiles, int n_tiles, const int64_t* flags,
+                                       void* stream) {
+  if (n_tiles != 0 && !flags) return YB_ERR_INVALID;
+  return fine_gemm(a, b, c, nullptr, dtype, outs, terms, tiles, n_tiles, 1.0, 0.0, flags, stream);
 }
 
 extern "C" int yb_grouped_gemm(const void* a, const void* b, void* c, int dtype, const int64_t* outs,

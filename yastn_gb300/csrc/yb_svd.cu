@@ -248,6 +248,154 @@ __global__ void svd_scale_wr_kernel(T64* __restrict__ work64, const int64_t* __r
   }
 }
 
+// Which blocks take their products with W from the FP64 kernel. Digits hold 57 bits below the largest
+// element of a row of W and of a component of Q (a column of Q^T): an output V_ij = sum_l W_il Q_jl
+// whose terms are all small against (max_l |W_il|) (max_l |Q_jl|) loses its relative accuracy,
+// which an FP64 sum keeps. Such outputs are where A is graded by columns (rows of 24 columns over 12
+// decades: V to 8e-5 in the smallest entries, A - U S V to 4e-6 of the column; FP64 5e-12 and 4e-14);
+// no scaling of l repairs both triangles of V. A pair (i, j) counts as such unless some l has both
+// elements within 2^-kGradedBits of their maxima (the output then holds 47 bits, what the sweeps leave
+// of an entry of a graded block), or no l has both nonzero. In a block that is not graded pairs count by
+// chance, up to 8 % where a row of W has one large element; the block is flagged where a row or
+// a component has more than a quarter of its pairs. Rows of R at noise level were not rotated (W's row is a unit vector, its
+// vector in V arbitrary) and are left out. The masks are bits, so the pairs of two 1296 x 1296
+// blocks take some 10 us.
+constexpr int kGradedBits = 5;
+
+struct GradedAt {  // a block's masks: [A big][A nonzero][B big][B nonzero][fails of A][fails of B]
+  uint32_t *a, *b;
+  int *na, *nb;
+  int k, L, nw;
+};
+__device__ __forceinline__ GradedAt graded_at(const int64_t* r, const int64_t* at, int32_t* masks) {
+  GradedAt g;
+  g.k = (int)r[R_K];
+  g.L = (int)r[R_LQ];
+  g.nw = (g.k + 31) / 32;
+  g.a = reinterpret_cast<uint32_t*>(masks + at[blockIdx.y]);
+  g.b = g.a + 2 * (int64_t)g.k * g.nw;
+  g.na = reinterpret_cast<int*>(g.b + 2 * (int64_t)g.L * g.nw);
+  g.nb = g.na + g.k;
+  return g;
+}
+
+// The masks: rows of W by a warp each (R's row tells noise), components of Q 32 to a CTA.
+template <typename T64>
+__global__ void __launch_bounds__(256) svd_graded_masks_kernel(const T64* __restrict__ work64,
+                                                               const int64_t* __restrict__ blocks, int k_min,
+                                                               const int64_t* __restrict__ state,
+                                                               const int64_t* __restrict__ at, int32_t* __restrict__ masks) {
+  const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
+  if (!r[R_QR] || r[R_K] < k_min) return;
+  const GradedAt g = graded_at(r, at, masks);
+  const double thr = __longlong_as_double((long long)state[(int64_t)blockIdx.y * ST_REC + ST_THR64]);
+  const T64 *W = work64 + r[R_W], *R = work64 + r[R_RR], *Z = work64 + r[R_Z];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ int red[8][32];
+  for (int i = blockIdx.x * 8 + warp; i < g.k; i += gridDim.x * 8) {
+    const T64* w = W + (int64_t)i * g.k;
+    double n2 = 0.0;
+    int top = -2000;
+    for (int l = lane; l < g.k; l += 32) {
+      n2 += cabs2(R[(int64_t)i * g.k + l]);
+      top = max(top, top_exponent(w[l]));
+    }
+    n2 = warp_sum(n2);
+    top = __reduce_max_sync(0xffffffffu, top);
+    const bool noise = !(n2 > thr);
+    for (int u = 0; u < g.nw; ++u) {
+      const int l = 32 * u + lane, e = l < g.k ? top_exponent(w[l]) : -2000;
+      const uint32_t big = __ballot_sync(0xffffffffu, l < g.k && (noise || (e > -2000 && e >= top - kGradedBits)));
+      const uint32_t nz = __ballot_sync(0xffffffffu, e > -2000);
+      if (lane == 0) {
+        g.a[(int64_t)i * g.nw + u] = big;
+        g.a[((int64_t)g.k + i) * g.nw + u] = nz;
+      }
+    }
+    if (lane == 0) g.na[i] = 0;
+  }
+  for (int j0 = blockIdx.x * 32; j0 < g.L; j0 += gridDim.x * 32) {
+    const int j = j0 + lane;
+    int top = -2000;
+#pragma unroll 4
+    for (int l = warp; l < g.k; l += 8)
+      if (j < g.L) top = max(top, top_exponent(Z[(int64_t)l * g.L + j]));
+    red[warp][lane] = top;
+    __syncthreads();
+    for (int v = 0; v < 8; ++v) top = max(top, red[v][lane]);
+    for (int u = warp; u < g.nw; u += 8) {
+      uint32_t big = 0, nz = 0;
+#pragma unroll 4
+      for (int t = 0; t < 32; ++t) {
+        const int l = 32 * u + t;
+        const int e = l < g.k && j < g.L ? top_exponent(Z[(int64_t)l * g.L + j]) : -2000;
+        if (e > -2000) {
+          nz |= 1u << t;
+          big |= (e >= top - kGradedBits ? 1u : 0u) << t;
+        }
+      }
+      if (j < g.L) {
+        g.b[(int64_t)j * g.nw + u] = big;
+        g.b[((int64_t)g.L + j) * g.nw + u] = nz;
+      }
+    }
+    if (warp == 0 && j < g.L) g.nb[j] = 0;
+    __syncthreads();
+  }
+}
+
+// The pairs, 32 x 32 to a CTA: a thread has one row of W and four components of Q.
+__global__ void __launch_bounds__(256) svd_graded_pairs_kernel(const int64_t* __restrict__ blocks, int k_min,
+                                                               const int64_t* __restrict__ at, int32_t* __restrict__ masks) {
+  const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
+  if (!r[R_QR] || r[R_K] < k_min) return;
+  const GradedAt g = graded_at(r, at, masks);
+  __shared__ uint32_t sa[2][32][33], sb[2][32][33];
+  const int ti = (g.k + 31) / 32, tj = (g.L + 31) / 32;
+  const int i = threadIdx.x >> 3, jq = (threadIdx.x & 7) * 4;
+  for (int64_t tile = blockIdx.x; tile < (int64_t)ti * tj; tile += gridDim.x) {
+    const int i0 = (int)(tile / tj) * 32, j0 = (int)(tile % tj) * 32;
+    uint32_t any[4] = {0, 0, 0, 0}, both[4] = {0, 0, 0, 0};
+    bool done = false;
+    for (int u0 = 0; u0 < g.nw && !done; u0 += 32) {
+      const int nu = min(32, g.nw - u0);
+      __syncthreads();
+      for (int e = threadIdx.x; e < 2 * 32 * nu; e += 256) {
+        const int half = e / (32 * nu), v = e / nu % 32, u = e % nu;
+        sa[half][v][u] = i0 + v < g.k ? g.a[((int64_t)half * g.k + i0 + v) * g.nw + u0 + u] : 0u;
+        sb[half][v][u] = j0 + v < g.L ? g.b[((int64_t)half * g.L + j0 + v) * g.nw + u0 + u] : 0u;
+      }
+      __syncthreads();
+      for (int u = 0; u < nu; ++u)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          any[q] |= sa[0][i][u] & sb[0][jq + q][u];
+          both[q] |= sa[1][i][u] & sb[1][jq + q][u];
+        }
+      done = __syncthreads_and(any[0] && any[1] && any[2] && any[3]);
+    }
+    int fails = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)  // beyond the edges nothing is nonzero
+      if (any[q] == 0 && both[q] != 0) {
+        ++fails;
+        atomicAdd(g.nb + j0 + jq + q, 1);
+      }
+    if (fails) atomicAdd(g.na + i0 + i, fails);
+  }
+}
+
+__global__ void svd_graded_flags_kernel(const int64_t* __restrict__ blocks, int k_min, const int64_t* __restrict__ at,
+                                        int32_t* __restrict__ masks, int64_t* __restrict__ flags) {
+  const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
+  if (!r[R_QR] || r[R_K] < k_min) return;
+  const GradedAt g = graded_at(r, at, masks);
+  bool on = false;
+  for (int i = threadIdx.x; i < g.k; i += blockDim.x) on = on || 4 * (int64_t)g.na[i] > g.L;
+  for (int j = threadIdx.x; j < g.L; j += blockDim.x) on = on || 4 * (int64_t)g.nb[j] > g.k;
+  if (on) flags[blockIdx.y] = 1;
+}
+
 // X = scale_b X, for an SVD whose X was formed from A itself.
 template <typename T64>
 __global__ void svd_scale_x_kernel(T64* __restrict__ work64, const int64_t* __restrict__ blocks,
@@ -1279,6 +1427,23 @@ int yb_svd_shift_prefill(void* work64, const int64_t* blocks, int n_blocks, int 
     yb::svd_shift_prefill_kernel<double2><<<grid, 256, 0, s>>>((double2*)work64, blocks, shift);
   else
     return YB_ERR_INVALID;
+  return yb::check_launch();
+}
+
+int yb_svd_graded(const void* work64, const int64_t* blocks, int n_blocks, int dtype, int k_min, const int64_t* state,
+                  const int64_t* at_masks, int32_t* masks, int64_t* flags, void* stream) {
+  if (n_blocks == 0) return YB_OK;
+  if (!work64 || !blocks || !state || !at_masks || !masks || !flags) return YB_ERR_INVALID;
+  const dim3 grid(64, (unsigned)n_blocks);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (dtype == YB_F64)
+    yb::svd_graded_masks_kernel<double><<<grid, 256, 0, s>>>((const double*)work64, blocks, k_min, state, at_masks, masks);
+  else if (dtype == YB_C128)
+    yb::svd_graded_masks_kernel<double2><<<grid, 256, 0, s>>>((const double2*)work64, blocks, k_min, state, at_masks, masks);
+  else
+    return YB_ERR_INVALID;
+  yb::svd_graded_pairs_kernel<<<dim3(152, (unsigned)n_blocks), 256, 0, s>>>(blocks, k_min, at_masks, masks);
+  yb::svd_graded_flags_kernel<<<dim3(1, (unsigned)n_blocks), 256, 0, s>>>(blocks, k_min, at_masks, masks, flags);
   return yb::check_launch();
 }
 

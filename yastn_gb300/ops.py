@@ -501,6 +501,20 @@ def run_emulated(eg, a, b, c):
     return c
 
 
+def _run_flagged(guard, name, a, b, c, flags):
+    """The products ``name`` of a P.SvdGuard (None: there are none) for the blocks with a flag."""
+    if guard is None:
+        return
+    key = (name, c.device)
+    args = guard._dev.get(key)
+    if args is None:  # addresses of the records, kept with them
+        g = guard.gemm[name]
+        d = _dev(g, 'flagged', (g.outs, g.terms, g.tiles), c.device)
+        args = guard._dev[key] = (_ptr(d[0]), _ptr(d[1]), _ptr(d[2]), len(g.tiles)), d
+    if args[0][3]:
+        N.call('yb_grouped_gemm_flagged', _ptr(a), _ptr(b), _ptr(c), _dtype_code(c.dtype), *args[0], _ptr(flags), _stream())
+
+
 _SMS = {}
 
 
@@ -642,11 +656,11 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
     dblocks, dpairs = _dev(plan, 'svd', (plan.blocks, plan.pair_items), dev)
     w64 = torch.empty(plan.n64, dtype=torch.complex128 if cplx else torch.float64, device=dev)
     w32 = torch.empty(plan.n32, dtype=torch.complex64 if cplx else torch.float32, device=dev)
-    # control words: [state][state after the FP32 phase][completion counts][QR flags], read once at the
-    # end: the host never waits between the phases
+    # control words: [state][state after the FP32 phase][completion counts][QR flags][graded blocks], read
+    # once at the end: the host never waits between the phases
     n_st, n_qr = SVD_STATE_REC * nb + 4, (nb + 4 * min(nb, 4096)) if plan.qr else 0
-    ctl = torch.zeros(2 * n_st + nb + n_qr, dtype=torch.int64, device=dev)
-    state, qctrl = ctl[:n_st], ctl[2 * n_st + nb:]
+    ctl = torch.zeros(2 * n_st + 2 * nb + n_qr, dtype=torch.int64, device=dev)
+    state, qctrl = ctl[:n_st], ctl[2 * n_st + nb:2 * n_st + nb + n_qr]
     n_small = ctl[2 * n_st:2 * n_st + nb] if mode == 0 else None
     aux = torch.empty(2 * nb, dtype=torch.float64, device=dev)  # [scale | shift]
     shift = aux[nb:] if mode != 0 else None
@@ -675,15 +689,26 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
     # one rounding per 400 contracted indices; R's grading is taken out of X = W R first): their
     # errors are no larger than the DFMA kernel's, which the FP64 pipe bounds: 2.7 against 0.46 ms
     # for all products of two 432 x 432 blocks, 55 against 3.7 ms for two 1296 x 1296, 0.64 against
-    # 0.10 ms in the eigh of five blocks up to 110. Short products (K < 16) stay native; the results of a
-    # block with a non-finite entry, which digits cannot hold, are made NaN (yb_svd_poison).
-    emu = None
-    if SVD_EMULATED[0]:
+    # 0.10 ms in the eigh of five blocks up to 110. Short products (K < 16) stay native, the products with W
+    # of a block graded by columns are formed again by the native kernel (yb_svd_graded: digits scaled per
+    # row and column lose the small entries of its factors); the results of a block with a non-finite
+    # entry, which digits cannot hold, are made NaN (yb_svd_poison).
+    emu = guard = flags = None
+    if SVD_EMULATED[0] and (plan.qr or mode != 0):
         emu = P.svd_emulated(plan, OZAKI_SLICES, cplx)
+        guard = emu['guard']
+        if guard is not None:
+            flags = ctl[2 * n_st + nb + n_qr:]
+            (at,) = _dev(guard, 'at', (guard.at,), dev)
+            masks = torch.empty(guard.size, dtype=torch.int32, device=dev)
+            N.call('yb_svd_graded', _ptr(w64), _ptr(dblocks), nb, code, P.OZAKI_MIN_DIM, _ptr(state), _ptr(at),
+                   _ptr(masks), _ptr(flags), st, launches=3)
         for gram, ns in (('gram', 'ns'), ('gram2', 'ns2')):
             run_emulated(emu[gram], w64, w64, w64)
+            _run_flagged(guard, gram, w64, w64, w64, flags)
             N.call('yb_svd_ns_prep', _ptr(w64), _ptr(dblocks), nb, code, ws, st)
             run_emulated(emu[ns], w64, w64, w64)
+            _run_flagged(guard, ns, w64, w64, w64, flags)
     else:
         W, Wn = w64[w0:w0 + ws], w64[n0:n0 + ws]
         for _ in range(NS_STEPS):
@@ -723,15 +748,16 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
            plan.max_k, mode, sp if mode else _ptr(aux), _ptr(state), _ptr(n_small) if n_small is not None else 0, st, launches=3)
     if plan.qr:  # the factor that comes from Q: Vh = conj(W) Q^T (wide), U = conj(Q) W^T (tall)
         if emu:
-            run_emulated(emu['qv'], w64, w64, V)
-            run_emulated(emu['qu'], w64, w64, U)
+            for name, F in (('qv', V), ('qu', U)):
+                run_emulated(emu[name], w64, w64, F)
+                _run_flagged(guard, name, w64, w64, F, flags)
             N.call('yb_svd_poison', _ptr(U), _ptr(V), _ptr(dblocks), nb, code, _ptr(state), 1, st)
         else:
             run_gemm(plan.qfin_v, w64, w64, V)
             run_gemm(plan.qfin_u, w64, w64, U)
     host = ctl.cpu()
     _svd_state_check(host[n_st:2 * n_st], nb, 'FP32', False)
-    if plan.qr and bool(host[2 * n_st + nb:][nb + 2::4].any()):
+    if plan.qr and bool(host[2 * n_st + nb:2 * n_st + nb + n_qr][nb + 2::4].any()):
         raise RuntimeError("yastn_gb300 svd: QR group barrier timed out")
     _svd_state_check(host[:n_st], nb, 'FP64', True)
     nz = host[2 * n_st:2 * n_st + nb].numpy()
