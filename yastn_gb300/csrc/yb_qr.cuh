@@ -133,14 +133,15 @@ __device__ __forceinline__ T warp_sums(T (&v)[N], int lane) {
 }
 
 // Waits (thread 0 polls, bounded) until *flag >= target; on timeout raises *err and returns (the
-// caller carries on with whatever it reads: the host sees the error word and fails).
+// caller carries on with whatever it reads: the host sees the error word and fails). Once *err is
+// up, a wait lasts 64 polls: one timeout ends those of all later panels too.
 __device__ __forceinline__ void qr_wait(const unsigned long long* flag, unsigned long long target,
                                         unsigned long long* err) {
   if (threadIdx.x == 0) {
     long long spins = 0;
     while (*(volatile const unsigned long long*)flag < target) {
       if (spins > 16) __nanosleep(32);
-      if (++spins > kSpinLimit) {
+      if (++spins > kSpinLimit || ((spins & 63) == 0 && *(volatile const unsigned long long*)err != 0)) {
         atomicExch(err, 1ull);
         break;
       }
