@@ -222,7 +222,8 @@ __device__ __forceinline__ double trsm_sub(double a, double b) { return a - b; }
 __device__ __forceinline__ double2 trsm_sub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double trsm_re(double a) { return a; }
 __device__ __forceinline__ double trsm_re(double2 a) { return a.x; }
-// v / d from ri = 1 / d: the product corrected by its residual; the division itself where 1 / d leaves
+// v / d from ri = 1 / d: the product corrected by its residual (P. W. Markstein, IBM J. Res. Dev. 34,
+// 1990), within 2^-52 of the quotient; the division itself where 1 / d leaves
 // the normal numbers (d zero or subnormal, infinite or close to it) and for an infinite quotient
 __device__ __forceinline__ double trsm_div(double v, double d, double ri) {
   if (!(fabs(ri) < 0x1p1000 && fabs(ri) > 0x1p-1000)) return v / d;

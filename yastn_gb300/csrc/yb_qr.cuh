@@ -283,8 +283,10 @@ __device__ __forceinline__ void qr_apply_panel(T* __restrict__ x, const QrPanel<
 // sign(Re alpha) Im alpha / s), 1 / (alpha - beta) = conj(alpha - beta) / ((s + |Re alpha|)^2 + (Im alpha)^2);
 // ts = conj(tau sc) = -1 / beta.
 // All panels wait for this chain: 12 FP64 instructions of 64 cycles for a real column (the square
-// root and the reciprocal by one third-order step each from an FP32 start, scalings and signs by
-// integers) instead of 28; 2.7 k -> 1.6 k cycles a column with the updates' factors. Norms whose squares
+// root by a step of Householder's iteration of third order as in rsqrt64 of yb_jacobi.cuh, the reciprocal by
+// one of the hyperpower iteration of third order, z (1 + e + e^2) with e = 1 - d z (M. Altman, Pacific J.
+// Math. 10, 1960), both from an FP32 start with e below 5e-7: 1e-19 is left; scalings and signs by
+// integers; results within 2^-50 of the exact ones for this alpha and xn) instead of 28; 2.7 k -> 1.6 k cycles a column with the updates' factors. Norms whose squares
 // leave 2^+-900 take the library's functions.
 template <typename T>
 __device__ __forceinline__ void qr_scalars(T alpha, double xn, T& tau, T& sc, T& diag, double& ts) {
