@@ -368,12 +368,12 @@ int yb_svd_ns_prep(void* work64, const int64_t* blocks, int n_blocks, int dtype,
 /* T = W D and Wn = D^-1 R (at t_delta and 2 t_delta elements after W) for blocks with a QR start, D
  * the powers of two of a two-sided equilibration of R: the operands of X = W R for a product whose
  * digits are scaled per row and column. X's storage is scratch. Three launches. The FP64 noise
- * norm in state of a block whose R is not finite becomes NaN: yb_svd_poison then writes NaN to its
- * X (which 0, U = the workspace) or to the factor that comes from Q (which 1). */
-int yb_svd_scale_wr(void* work64, const int64_t* blocks, int n_blocks, int dtype, int64_t t_delta,
+ * norm in state of a block of k >= k_min whose R is not finite becomes NaN: yb_svd_poison then writes
+ * NaN to its X (which 0, U = the workspace) or to the factor that comes from Q (which 1). */
+int yb_svd_scale_wr(void* work64, const int64_t* blocks, int n_blocks, int dtype, int64_t t_delta, int k_min,
                     int64_t* state, void* stream);
 int yb_svd_poison(void* U, void* V, const int64_t* blocks, int n_blocks, int dtype, const int64_t* state,
-                  int which, void* stream);
+                  int k_min, int which, void* stream);
 /* flags[b] = 1 for the blocks (with a QR start, k >= k_min) whose products with W must not be formed
  * from digits: those where the factor W Q^T would lose entries that are small for their row of W and
  * their component of Q at once (blocks graded by columns). W as widened, Q^T and R as left by

@@ -34,8 +34,8 @@ SIGNATURES = {
     'yb_trsm_rt': ([_vp, _vp, _vp, _i, _i, _vp], _i),
     'yb_svd_sweeps': ([_vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _d, _vp, _vp], _i),
     'yb_svd_ns_prep': ([_vp, _vp, _i, _i, _i64, _vp], _i),
-    'yb_svd_scale_wr': ([_vp, _vp, _i, _i, _i64, _vp, _vp], _i),
-    'yb_svd_poison': ([_vp, _vp, _vp, _i, _i, _vp, _i, _vp], _i),
+    'yb_svd_scale_wr': ([_vp, _vp, _i, _i, _i64, _i, _vp, _vp], _i),
+    'yb_svd_poison': ([_vp, _vp, _vp, _i, _i, _vp, _i, _i, _vp], _i),
     'yb_svd_row_aux': ([_i64, _i64], _i64),
     'yb_svd_row_limit': ([_i, _i], _i),
     'yb_svd_row_sweeps': ([_vp, _vp, _i, _vp, _i, _i, _i, _i, _d, _i, _vp, _vp, _i64, _vp], _i),

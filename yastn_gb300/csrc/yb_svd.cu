@@ -164,10 +164,11 @@ __device__ __forceinline__ double real_of(double2 v) { return v.x; }
 __device__ __forceinline__ void set_real(double& d, double v) { d = v; }
 __device__ __forceinline__ void set_real(double2& d, double v) { d = make_double2(v, 0.0); }
 
-// A non-finite R (exponent 1024) marks its block: its FP64 noise norm becomes NaN (it is NaN or Inf
-// already unless the block's norm overflowed), see svd_poison_kernel.
+// A non-finite R (exponent 1024) marks its block, if that has products from digits (k >= k_min): its FP64
+// noise norm becomes NaN (it is NaN or Inf already unless the block's norm overflowed), see
+// svd_poison_kernel.
 template <typename T64>
-__global__ void svd_col_exponents_kernel(T64* __restrict__ work64, const int64_t* __restrict__ blocks,
+__global__ void svd_col_exponents_kernel(T64* __restrict__ work64, const int64_t* __restrict__ blocks, int k_min,
                                          int64_t* __restrict__ state) {
   const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
   if (!r[R_QR]) return;
@@ -184,7 +185,7 @@ __global__ void svd_col_exponents_kernel(T64* __restrict__ work64, const int64_t
     __syncthreads();
     if (warp == 0 && j < k) {
       for (int w = 1; w < 8; ++w) e = max(e, red[w][lane]);
-      if (e == 1024) state[(int64_t)blockIdx.y * ST_REC + ST_THR64] = 0x7ff8000000000000ll;
+      if (e == 1024 && k >= k_min) state[(int64_t)blockIdx.y * ST_REC + ST_THR64] = 0x7ff8000000000000ll;
       set_real(work64[r[R_X] + j], (double)e);
     }
     __syncthreads();
@@ -196,11 +197,11 @@ __global__ void svd_col_exponents_kernel(T64* __restrict__ work64, const int64_t
 // factor that comes from Q (U of tall blocks, Vh of the others).
 template <typename T64>
 __global__ void svd_poison_kernel(T64* __restrict__ U, T64* __restrict__ V, const int64_t* __restrict__ blocks,
-                                  const int64_t* __restrict__ state, int which) {
+                                  const int64_t* __restrict__ state, int k_min, int which) {
   const double thr = __longlong_as_double((long long)state[(int64_t)blockIdx.y * ST_REC + ST_THR64]);
-  if (thr == thr) return;
   const int64_t* r = blocks + (int64_t)blockIdx.y * YB_SVD_REC;
   const int64_t k = r[R_K];
+  if (thr == thr || k < k_min) return;
   const bool tall = r[R_M] > r[R_N];
   T64* p = which == 0 ? U + r[R_X] : (tall ? U + r[R_U] : V + r[R_V]);
   const int64_t n = which == 0 ? k * r[R_L] : (tall ? r[R_M] * k : k * r[R_N]);
@@ -1380,18 +1381,18 @@ int yb_svd_ns_prep(void* work64, const int64_t* blocks, int n_blocks, int dtype,
   return yb::check_launch();
 }
 
-int yb_svd_scale_wr(void* work64, const int64_t* blocks, int n_blocks, int dtype, int64_t t_delta, int64_t* state,
-                    void* stream) {
+int yb_svd_scale_wr(void* work64, const int64_t* blocks, int n_blocks, int dtype, int64_t t_delta, int k_min,
+                    int64_t* state, void* stream) {
   if (n_blocks == 0) return YB_OK;
   if (!work64 || !blocks || !state || t_delta <= 0) return YB_ERR_INVALID;
   const dim3 grid(64, (unsigned)n_blocks);
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype == YB_F64) {
-    yb::svd_col_exponents_kernel<double><<<grid, 256, 0, s>>>((double*)work64, blocks, state);
+    yb::svd_col_exponents_kernel<double><<<grid, 256, 0, s>>>((double*)work64, blocks, k_min, state);
     yb::svd_row_scales_kernel<double><<<grid, 256, 0, s>>>((double*)work64, blocks);
     yb::svd_scale_wr_kernel<double><<<grid, 256, 0, s>>>((double*)work64, blocks, t_delta);
   } else if (dtype == YB_C128) {
-    yb::svd_col_exponents_kernel<double2><<<grid, 256, 0, s>>>((double2*)work64, blocks, state);
+    yb::svd_col_exponents_kernel<double2><<<grid, 256, 0, s>>>((double2*)work64, blocks, k_min, state);
     yb::svd_row_scales_kernel<double2><<<grid, 256, 0, s>>>((double2*)work64, blocks);
     yb::svd_scale_wr_kernel<double2><<<grid, 256, 0, s>>>((double2*)work64, blocks, t_delta);
   } else {
@@ -1400,16 +1401,16 @@ int yb_svd_scale_wr(void* work64, const int64_t* blocks, int n_blocks, int dtype
   return yb::check_launch();
 }
 
-int yb_svd_poison(void* U, void* V, const int64_t* blocks, int n_blocks, int dtype, const int64_t* state, int which,
-                  void* stream) {
+int yb_svd_poison(void* U, void* V, const int64_t* blocks, int n_blocks, int dtype, const int64_t* state, int k_min,
+                  int which, void* stream) {
   if (n_blocks == 0) return YB_OK;
   if (!U || !blocks || !state || which < 0 || which > 1 || (which == 1 && !V)) return YB_ERR_INVALID;
   const dim3 grid(8, (unsigned)n_blocks);
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype == YB_F64)
-    yb::svd_poison_kernel<double><<<grid, 256, 0, s>>>((double*)U, (double*)V, blocks, state, which);
+    yb::svd_poison_kernel<double><<<grid, 256, 0, s>>>((double*)U, (double*)V, blocks, state, k_min, which);
   else if (dtype == YB_C128)
-    yb::svd_poison_kernel<double2><<<grid, 256, 0, s>>>((double2*)U, (double2*)V, blocks, state, which);
+    yb::svd_poison_kernel<double2><<<grid, 256, 0, s>>>((double2*)U, (double2*)V, blocks, state, k_min, which);
   else
     return YB_ERR_INVALID;
   return yb::check_launch();

@@ -718,9 +718,9 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
             W.copy_(Wn)
     if plan.qr:
         if emu:
-            N.call('yb_svd_scale_wr', _ptr(w64), _ptr(dblocks), nb, code, ws, _ptr(state), st, launches=3)
+            N.call('yb_svd_scale_wr', _ptr(w64), _ptr(dblocks), nb, code, ws, P.OZAKI_MIN_DIM, _ptr(state), st, launches=3)
             run_emulated(emu['xr'], w64, w64, w64)  # X = W R = T Wn
-            N.call('yb_svd_poison', _ptr(w64), 0, _ptr(dblocks), nb, code, _ptr(state), 0, st)
+            N.call('yb_svd_poison', _ptr(w64), 0, _ptr(dblocks), nb, code, _ptr(state), P.OZAKI_MIN_DIM, 0, st)
         else:
             run_gemm(plan.xform, w64, w64, w64)
     elif shift is not None:
@@ -751,7 +751,7 @@ def _jacobi(data, plan, U, S, V, mode, max_sweeps=MAX_SWEEPS):
             for name, F in (('qv', V), ('qu', U)):
                 run_emulated(emu[name], w64, w64, F)
                 _run_flagged(guard, name, w64, w64, F, flags)
-            N.call('yb_svd_poison', _ptr(U), _ptr(V), _ptr(dblocks), nb, code, _ptr(state), 1, st)
+            N.call('yb_svd_poison', _ptr(U), _ptr(V), _ptr(dblocks), nb, code, _ptr(state), P.OZAKI_MIN_DIM, 1, st)
         else:
             run_gemm(plan.qfin_v, w64, w64, V)
             run_gemm(plan.qfin_u, w64, w64, U)
