@@ -7,6 +7,7 @@ Plans depend only on the metadata, so they are cached by the identity of the tup
 (YASTN memoises its metadata with ``lru_cache``, so the same tuple object comes back)
 and, failing that, by value.
 """
+import math
 import pickle
 from collections import OrderedDict
 
@@ -283,27 +284,27 @@ def _box_task(so, do, sizes, ss, ds, elem):
             targets.update(got * f for f in (1, 2, 3, 4, 6, 8) if f <= sizes[i])
             got *= sizes[i]
             targets.add(got)
-    best = None
+    best, total = None, math.prod(sizes)
     for target in sorted(x for x in targets if 1 < x <= cap):
         t = [-(-n // -(-n // x)) for n, x in zip(sizes, extents(target))]
-        count = int(np.prod(t, dtype=np.int64))
+        count = math.prod(t)
         if count <= cap:
-            full = np.prod([-(-n // x) for n, x in zip(sizes, t)], dtype=np.int64) * (-(-count // 512) * 512)
-            cost = sum(32 / (r * elem) for r in runs(t)) + 0.5 * float(full) / float(np.prod(sizes, dtype=np.int64))
+            full = math.prod(-(-n // x) for n, x in zip(sizes, t)) * (-(-count // 512) * 512)
+            cost = sum(32 / (r * elem) for r in runs(t)) + 0.5 * full / total
             if best is None or cost < best[0]:
                 best = (cost, t)
     if best is None:
         return None
     t = best[1]
     clipped = [i for i in range(nd) if sizes[i] % t[i]]
-    if np.prod(t, dtype=np.int64) > cap or len(clipped) > 4 or \
+    if math.prod(t) > cap or len(clipped) > 4 or \
             any(sum((x - 1) * abs(b) for x, b in zip(t, st)) >= 2 ** 31 for st in (ss, ds)):
         return None
     sm, at = [0] * nd, 1
     for i in reversed(by_src):
         sm[i], at = at, at * t[i]
     rec = np.zeros(BOX_REC, dtype=np.int64)
-    rec[0], rec[1] = nd, np.prod(t, dtype=np.int64)
+    rec[0], rec[1] = nd, math.prod(t)
     for d, i in enumerate(by_src):
         m, sh = fast_div_consts(t[i])
         rec[8 + d], rec[16 + d], rec[24 + d], rec[32 + d], rec[40 + d] = t[i], ss[i], ds[i], sm[i], m | (sh << 32)
@@ -354,7 +355,7 @@ def _wants_box(sizes, ss, ds, elem, fill=0.5):
     tiles = -(-x // T) * -(-y // T)
     # a block of a single box pays the box's set-up for itself: only where a tile holds little
     return x * y < fill * T * T * tiles and (x * y < 300 * tiles or
-                                            np.prod(sizes, dtype=np.int64) >= 4 * _box_elements(elem))
+                                            math.prod(sizes) >= 4 * _box_elements(elem))
 
 
 class CopyPlan:
@@ -391,19 +392,24 @@ class CopyPlan:
             # 27, 141 and 90)
             by_dst = [_by_destination(t) for t in tasks]
             scatter = [t is not u for t, u in zip(tasks, by_dst)]
-            large = sum(int(np.prod(t[2], dtype=np.int64)) for t, x in zip(tasks, scatter) if x) >= BOX_MIN_SCATTER
-            fill = 0.9 if sum(int(np.prod(t[2], dtype=np.int64)) for t in tasks) >= BOX_LARGE else 0.5
-            for task, ordered, x in zip(tasks, by_dst, scatter):
-                box = _box_task(*ordered, elem) if (large or not x) and _wants_box(*ordered[2:], elem, fill) else None
-                if box is None:
-                    rest.append(task)
-                    continue
-                recs.append(box[0])
-                tables.append(box[1])
+            counts = [math.prod(t[2]) for t in tasks]
+            large = sum(n for n, x in zip(counts, scatter) if x) >= BOX_MIN_SCATTER
+            fill = 0.9 if sum(counts) >= BOX_LARGE else 0.5
+            wants = [(large or not x) and _wants_box(*t[2:], elem, fill) for t, x in zip(by_dst, scatter)]
+            boxes = {}
             # a second launch for the rest is worth it from about a million elements on (below, both
-            # are latency: 8 + 6 us against 8..14)
-            if rest and sum(int(r[1]) * len(x) for r, x in zip(recs, tables)) < BOX_MIN_MIXED:
-                rest, recs, tables = self._expanded(), [], []
+            # are latency: 8 + 6 us against 8..14): no boxes are planned for less
+            if all(wants) or sum(n for n, w in zip(counts, wants) if w) >= BOX_MIN_MIXED:
+                boxes = {i: b for i, b in ((i, _box_task(*t, elem)) for i, (t, w) in enumerate(zip(by_dst, wants)) if w)
+                         if b is not None}
+            if len(boxes) < len(tasks) and sum(counts[i] for i in boxes) < BOX_MIN_MIXED:
+                boxes = {}
+            for i, task in enumerate(tasks):
+                if i in boxes:
+                    recs.append(boxes[i][0])
+                    tables.append(boxes[i][1])
+                else:
+                    rest.append(task)
             total = sum(len(x) for x in tables)
             per = max(1, min(BOX_PER_CTA, total // BOX_CTAS))
             items, first = [], 0
@@ -452,7 +458,7 @@ class CopyPlan:
                 ss = [x // 2 for x in ss[:-1]] + [1]
                 ds = [x // 2 for x in ds[:-1]] + [1]
                 so, do = so // 2, do // 2
-            count = int(np.prod(sizes, dtype=np.int64))
+            count = math.prod(sizes)
             if count >= 2 ** 31:
                 raise PlanError("copy task larger than 2^31 units")
             rec = np.zeros(COPY_REC, dtype=np.int64)
