@@ -32,3 +32,16 @@ def test_completion_of_low_rank_blocks(m, n, rank, cplx, emulated, cuda_device):
     assert np.abs((U * S) @ V - A).max() <= 1e-12 * np.abs(A).max() * k
     assert np.abs(U.conj().T @ U - np.eye(k)).max() <= 1e-12 * k
     assert np.abs(V @ V.conj().T - np.eye(k)).max() <= 1e-12 * k
+
+
+def test_completion_plans_are_bounded(cuda_device):
+    """The counts of completed vectors differ from call to call: the plan of the blocks does not collect
+    a completion plan for each."""
+    rng = np.random.default_rng(0)
+    n = 260
+    meta = (((0, n * n), (n, n), (0, n * n), (n, n), (0, n), (0, n * n), (n, n)),)
+    for rank in range(1, 2 * ops.MAX_COMPLETIONS + 1):
+        A = rng.normal(size=(n, rank)) @ rng.normal(size=(rank, n))
+        ops.svd(torch.from_numpy(A.ravel()).cuda(), meta, (n * n, n, n * n))
+    kept = P.svd_plan(meta, None, False, qr=True)._completion
+    assert 0 < len(kept) <= ops.MAX_COMPLETIONS

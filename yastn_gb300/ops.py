@@ -615,6 +615,7 @@ BLOCKED_FP64 = [True]  # FP64 phase likewise, on 4-row super-vectors (False: one
 ROWS_PER_SUPER = [None]  # super-vector height (None: largest of 16, 8, 4 that fits)
 NS_STEPS = 2          # Newton-Schulz steps: non-orthogonality ~1e-6 -> 1e-12 -> ~eps
 SVD_EMULATED = [True]  # FP64 products inside svd / eigh on the tensor cores (False: the native grouped GEMM)
+MAX_COMPLETIONS = 8   # completion plans kept with an SvdPlan
 SVD_QR = [True]       # svd: Jacobi on the rows of R of a Householder QR (few FP64 sweeps on graded spectra)
 
 
@@ -771,12 +772,16 @@ def _complete(plan, U, V, nz, cplx, emulated=False):
     (yb_fill_candidates), projected twice off the k - nz earlier vectors by grouped GEMMs
     (C = V_g^H G, G -= V_g C), orthonormalised by the batched Householder QR, and copied into
     the factor's last nz vectors (U columns or Vh rows, whichever the rows of X built)."""
-    key = tuple(int(x) for x in nz)
-    cache = plan.__dict__.setdefault('_completion', {})
-    if key not in cache:
-        cache[key] = P.completion_plans(plan.blocks, nz, cplx)
-    dev = U.device
-    for cp in cache[key]:
+    dev, cache = U.device, plan.__dict__.setdefault('_completion', {})
+    # the counts depend on the data: the last few only, and per stream (their records on the device go
+    # back to the allocator of the stream that has used them)
+    key = (_stream(),) + tuple(int(x) for x in nz)
+    plans = cache.get(key)
+    if plans is None:
+        plans = cache[key] = P.completion_plans(plan.blocks, nz, cplx)
+        while len(cache) > MAX_COMPLETIONS:
+            cache.pop(next(iter(cache)), None)
+    for cp in plans:
         F = U if cp.to_u else V
         G = torch.empty(max(cp.G, 1), dtype=F.dtype, device=dev)
         C = torch.empty(max(cp.C, 1), dtype=F.dtype, device=dev)
