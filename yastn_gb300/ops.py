@@ -779,8 +779,8 @@ def _complete(plan, U, V, nz, cplx, emulated=False):
     plans = cache.get(key)
     if plans is None:
         plans = cache[key] = P.completion_plans(plan.blocks, nz, cplx)
-        while len(cache) > MAX_COMPLETIONS:
-            cache.pop(next(iter(cache)), None)
+        for old in list(cache)[:-MAX_COMPLETIONS]:  # list: one step, other threads insert too
+            cache.pop(old, None)
     for cp in plans:
         F = U if cp.to_u else V
         G = torch.empty(max(cp.G, 1), dtype=F.dtype, device=dev)
