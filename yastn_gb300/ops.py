@@ -375,15 +375,19 @@ def dot_ozaki(A, B, meta_dot, Dsize, slices=OZAKI_SLICES):
         tc = plan.tuned_tc
     # the native sectors (disjoint outputs) run on a second stream beside the split and the
     # emulated GEMM, and the current stream waits for them (a fork and join inside a CUDA graph)
-    fork = plan.native.has_work()
-    if fork:
-        main, side, keep = torch.cuda.current_stream(A.device), _side_stream(A.device), []
-        side.wait_stream(main)
+    if not plan.native.has_work():
+        _ozaki_run(plan, A, B, out, slices, tc)
+        return out
+    main, side, keep = torch.cuda.current_stream(A.device), _side_stream(A.device), []
+    side.wait_stream(main)
+    try:
         run_gemm(plan.native, A, B, out, stream=side.cuda_stream, keep=keep)
-    _ozaki_run(plan, A, B, out, slices, tc)
-    if fork:
+        _ozaki_run(plan, A, B, out, slices, tc)
+    finally:
+        # also where a launch or an allocation failed: the memory of out and of the workspaces in keep
+        # may be given to later work of the main stream
         main.wait_stream(side)
-        del keep  # after the wait: its memory may be given to later work of the main stream
+        del keep
     return out
 
 
