@@ -3,24 +3,30 @@
 //
 // Each block A (m x n, row-major) is handled in its "wide" orientation: the k=min(m,n)
 // vectors to orthogonalise are the rows of A (m <= n) or of A^H (m > n), each of length
-// L=max(m,n), held in a workspace X; rotations are accumulated in W (k x k), so that
-// X = W X_0 at every step. A parallel round-robin ordering (circle method over
-// N = k rounded up to even) pairs all vectors in N-1 rounds of N/2 disjoint pairs; one
-// warp rotates one pair and all blocks advance together.
+// L=max(m,n), held in a workspace X (an SVD with a QR start: the rows of R, of length k);
+// rotations are accumulated in W (k x k), so that X = W X_0 at every step.
 //
 // GB300 has ~60x more FP32 than FP64 throughput, so the sweeps run in two phases:
 //   1. FP32 sweeps on (X32, W32) (float or complex64) until the rows are orthogonal to
-//      about 1e-4 (a blocked variant keeps super-vectors of rows in shared memory);
+//      about 1e-4;
 //   2. the host orthonormalises W = widen(W32) with Newton-Schulz steps and forms
-//      X = W X_0 with the FP64 grouped GEMM; then FP64 sweeps polish (X, W) until a
+//      X = W X_0 (emulated products on the tensor cores, the native FP64 ones for blocks that
+//      svd_graded_flags_kernel names); then FP64 sweeps polish (X, W) until a
 //      sweep whose largest |cos| was below tol_stop (typically 2-3 sweeps).
-// One persistent cooperative launch runs all the sweeps of a phase; rounds are separated
+// The sweeps of rows that fit a warp's registers are those of yb_jacobi.cuh. This file holds the
+// start, the products' scalings, the finalisation and the sweeps of longer rows (more than 2624
+// elements in FP32, 1312 in FP64, half of each for complex data): super-vectors of rows in shared
+// memory or one pair per warp, paired by a round-robin ordering (circle method over
+// N = k rounded up to even, N-1 rounds of N/2 disjoint pairs; all blocks advance together). One
+// persistent cooperative launch runs all the sweeps of a phase; rounds are separated
 // by a grid barrier whose spin is bounded (an error flag is raised and the kernel exits
 // if it ever times out). Finally S = row norms (descending), the normalised rows give Vh
-// (wide) or U (tall, conjugated), and W^H gives the other factor.
+// (wide) or U (tall, conjugated), and W^H gives the other factor (with a QR start the other way
+// round, see below).
 //
 // A rotation is applied when |<x_p, x_q>| > sqrt(L) eps ||x_p|| ||x_q|| (the threshold of
-// LAPACK's one-sided Jacobi); the angle follows Rutishauser's formula with hypot. For
+// LAPACK's one-sided Jacobi); the angle of the sweeps here follows Rutishauser's formula with hypot
+// (yb_jacobi.cuh: its tangent in FP32). For
 // complex rows the phase u = g/|g| of g = <x_p, x_q> = sum_l x_p[l] conj(x_q[l]) is first
 // moved onto x_q, which makes the pair's inner product real, and the real rotation of
 // (|x_p|^2, |x_q|^2, |g|) follows: x_p <- c x_p - s u x_q, x_q <- s x_p + c u x_q (unitary).
@@ -258,9 +264,11 @@ __global__ void svd_scale_wr_kernel(T64* __restrict__ work64, const int64_t* __r
 // elements within 2^-kGradedBits of their maxima (the output then holds 47 bits, what the sweeps leave
 // of an entry of a graded block), or no l has both nonzero. In a block that is not graded pairs count by
 // chance, up to 8 % where a row of W has one large element; the block is flagged where a row or
-// a component has more than a quarter of its pairs. Rows of R at noise level were not rotated (W's row is a unit vector, its
-// vector in V arbitrary) and are left out. The masks are bits, so the pairs of two 1296 x 1296
-// blocks take some 10 us.
+// a component has more than a quarter of its pairs. Rows of R at noise level were not rotated (W's
+// row is a unit vector, its vector in V arbitrary) and are left out. The masks are bits: a word has 32
+// terms of a pair. Bound: latency; the three launches take 23 us for nine blocks of 24..93, 44 for two
+// 432 x 432, 264 for two 1296 x 1296 (of 2.1, 9.0 and 55 ms of the call's device time), the five
+// flagged launches that find no flag 31 to 44 us.
 constexpr int kGradedBits = 5;
 
 struct GradedAt {  // a block's masks: [A big][A nonzero][B big][B nonzero][fails of A][fails of B]
@@ -770,11 +778,6 @@ int launch_block_sweeps(T* work, const int64_t* blocks, int n_blocks, const int3
   return YB_OK;
 }
 
-// Finalisation: singular values = row norms, sorted descending (index tie-break), U, S, Vh
-// written; vectors of zero norm are completed to an orthonormal set.
-// mode 0: SVD. mode 1/2: Hermitian eigendecomposition of a block shifted by shift[b]
-// (lambda = sigma - shift), eigenvectors = columns of W^H, ordered ascending (1) or by
-// |lambda| descending (2); Vh is not written.
 // ---------------------------------------------------------------- QR preconditioning
 // A block whose spectrum is graded (singular values spread over many decades, as in the
 // projector blocks of a corner transfer matrix step) keeps one-sided Jacobi busy for tens of
@@ -787,12 +790,11 @@ int launch_block_sweeps(T* work, const int64_t* blocks, int n_blocks, const int3
 //   tall:  A = conj(Q R);                 =>  U = conj(Q) W^T,  Vh = conj(Y)
 // (Y: rows of X = W R normalised, W: the accumulated rotations). Z holds M's columns as
 // rows (Z = X_0, k rows of length L); the factorisation leaves R in Z's upper part and the
-// Householder vectors below the diagonal (LAPACK's geqr2 layout, transposed); Q^T is then
-// formed in place (org2r, backward accumulation).
+// Householder vectors in V (yb_qr.cuh); Q^T is then formed in place (backward accumulation).
 
-// Z = X_0 in FP64 (A, or A^H for tall blocks). Records with [16] = 2 (yb_qr, M = A): Z's
-// rows are the first k columns of A (length L = m).
-// (scaled by scale[b], a power of two, where it is given: see block_fro_kernel).
+// Z = X_0 in FP64 (A, or A^H for tall blocks), scaled by scale[b], a power of two, where it is given
+// (see block_fro_kernel). Records with [16] = 2 (yb_qr, M = A): Z's rows are the first k columns of
+// A (length L = m).
 template <typename T>
 __global__ void svd_qr_load_kernel(const T* __restrict__ A, T* __restrict__ work, const int64_t* __restrict__ blocks,
                                    const double* __restrict__ scale) {
@@ -858,7 +860,12 @@ __global__ void qr_finalize_kernel(const T* __restrict__ work, T* __restrict__ Q
   }
 }
 
-// The finalisation takes three launches: the rows' norms (a warp per row, all SMs) into S, unsorted;
+// Finalisation: singular values = row norms, sorted descending (index tie-break), U, S, Vh
+// written; vectors of values at noise level are completed to an orthonormal set.
+// mode 0: SVD. mode 1/2: Hermitian eigendecomposition of a block shifted by shift[b]
+// (lambda = sigma - shift), eigenvectors = columns of W^H, ordered ascending (1) or by
+// |lambda| descending (2); Vh is not written.
+// It takes three launches: the rows' norms (a warp per row, all SMs) into S, unsorted;
 // the vectors, each CTA gathering 32 positions of the descending order through shared memory (both
 // the reads of X's and W's rows and the writes of U's columns coalesce); S sorted in place and the
 // rows at noise level counted, with their completion, by one CTA per block. Positions are ranks,

@@ -1,6 +1,7 @@
-// Shared by the block SVD / eigh kernels (yb_svd.cu, yb_jacobi.cu): the record layout of the
-// blocks, the per-block state, numeric traits of the four working types, the Jacobi rotation of
-// a row pair and the bounded grid barrier of the cooperative launches.
+// Shared by the block SVD / eigh / QR kernels (yb_svd.cu, yb_jacobi.cuh, yb_qr.cuh): the record
+// layout of the blocks, the per-block state, numeric traits of the four working types, the Jacobi
+// rotation of a row pair in the sweeps of yb_svd.cu and the bounded grid barrier of the cooperative
+// launches.
 #pragma once
 #include <float.h>
 #include "yb_common.cuh"
