@@ -321,7 +321,8 @@ int yb_krylov_combine(const void* V, int64_t ldv, const void* coeffs, int m, int
  * the scale: yb_svd_shift_prefill, then X += W A); yb_svd_sweeps with precision 64; yb_svd_finalize. yb_svd_sweeps runs every
  * sweep of a phase in one cooperative launch (rounds separated by a grid barrier with a
  * bounded spin; on timeout the error control word is set and the kernel exits) and stops
- * after the first sweep in which each block's largest rotation |cos| was <= tol_stop, or
+ * after the first sweep in which each block's largest rotation |cos| was <= tol_stop (precision 64
+ * with tol_stop > 1e-9: and that times the sweep's largest tangent <= 1e-12), or
  * after max_sweeps (the host reads the state and maps non-convergence to an error).
  * shift != NULL (eigh): per-block shifts c_b = ||A_b||_F + 1 are computed and A_b + c_b I
  * is decomposed (Hermitian positive definite, so its SVD is its eigendecomposition);

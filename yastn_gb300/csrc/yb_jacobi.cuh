@@ -118,10 +118,11 @@ struct Row {
 
 // One pair: the warp's row P and the row q in shared memory ([x: 32 NU | w: 32 NU],
 // zeros beyond the row) with state qs.
-// Returns true if it was rotated.
+// Returns true if it was rotated. |cos| to maxcos; FP64: a tangent of kTanMin and more to *maxtan (shared memory).
 template <typename T, int NU>
 __device__ __forceinline__ bool rotate(Row<T, NU>& P, T* __restrict__ q, RowState<typename Num<T>::R>* __restrict__ qs,
-                                       int lane, typename Num<T>::R thr2, float thr_cos, int& maxcos) {
+                                       int lane, typename Num<T>::R thr2, float thr_cos, int& maxcos,
+                                       int* __restrict__ maxtan) {
   using R = typename Num<T>::R;
   const R al = P.s.nrm, be = qs->nrm;
   if (!(above(al, thr2) && above(be, thr2))) return false;
@@ -158,7 +159,8 @@ __device__ __forceinline__ bool rotate(Row<T, NU>& P, T* __restrict__ q, RowStat
   const float cosv = pair_cos(al, be, ga);
   maxcos = max(maxcos, __float_as_int(cosv));
   if (!(cosv > thr_cos)) return false;
-  const R t = (R)pair_tan(al, be, ga);
+  const float tf = pair_tan(al, be, ga);
+  const R t = (R)tf;
   const R u1 = t * t + R(1);
   const R c = inv_sqrt(u1), ci = u1 * c;  // 1 / sqrt(1 + t^2) and its inverse
   const R a = t * (dy * P.s.i), b = t * (c * c) * (P.s.d * iy);
@@ -184,7 +186,7 @@ __device__ __forceinline__ bool rotate(Row<T, NU>& P, T* __restrict__ q, RowStat
   P.s.d *= c;
   P.s.i *= ci;
   const R ndy = dy * ci, niy = iy * c;
-  if (fabsf((float)t) > 0.25f) {  // a large angle may cancel: the norms from the rows
+  if (fabsf(tf) > 0.25f) {  // a large angle may cancel: the norms from the rows
     R s0 = 0, s1 = 0;
 #pragma unroll
     for (int v = 0; v < NU; ++v) {
@@ -200,6 +202,7 @@ __device__ __forceinline__ bool rotate(Row<T, NU>& P, T* __restrict__ q, RowStat
     qs->nrm = nb;
     qs->d = ndy;
     qs->i = niy;
+    if (sizeof(R) == 8 && fabsf(tf) > kTanMin) atomicMax(maxtan, __float_as_int(fabsf(tf)));
   }
   return true;
 }
@@ -304,11 +307,12 @@ __global__ void __launch_bounds__(BRM * 32) jacobi_rows_kernel(T* __restrict__ w
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* Trows = reinterpret_cast<T*>(smem_raw);  // [br][64 NU]
   __shared__ RowState<R> tst[BRM];
-  __shared__ int s_flag, s_last;
+  __shared__ int s_flag, s_last, s_tan;
   __shared__ Place s_place;
   const Aux aux = aux_of(aux_words, n_blocks, n_pairs);
   unsigned long long* err = reinterpret_cast<unsigned long long*>(state + (int64_t)n_blocks * ST_REC) + C_ERR;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) s_tan = 0;
 
   // Waits (thread 0, bounded) until ready() holds; returns false on timeout. Ends with a barrier.
   auto wait = [&](auto ready) {
@@ -501,7 +505,13 @@ __global__ void __launch_bounds__(BRM * 32) jacobi_rows_kernel(T* __restrict__ w
           st_release(ver + s, value);
         }
       };
-      auto report = [&] {  // largest |cos| of the item's pairs to the block's running maximum
+      // largest |cos| and tangent of the item's pairs to the block's running maxima (a barrier lies between
+      // the last rotation and this, and between this and the next one)
+      auto report = [&] {
+        if (!f32 && threadIdx.x == 0 && s_tan) {
+          atomicMax((unsigned long long*)st + ST_LASTCOS, (unsigned long long)__double_as_longlong((double)__int_as_float(s_tan)));
+          s_tan = 0;
+        }
         if (lane == 0 && maxcos)
           atomicMax((unsigned long long*)st, (unsigned long long)__double_as_longlong((double)__int_as_float(maxcos)));
         maxcos = 0;
@@ -545,7 +555,7 @@ __global__ void __launch_bounds__(BRM * 32) jacobi_rows_kernel(T* __restrict__ w
                   P.w[u] = pr[(NU + u) * 32 + lane];
                 }
                 P.s = tst[p];
-                if (rotate<T, NU>(P, Trows + (size_t)q * stride, tst + q, lane, thr2, thr_cos, maxcos)) {
+                if (rotate<T, NU>(P, Trows + (size_t)q * stride, tst + q, lane, thr2, thr_cos, maxcos, &s_tan)) {
 #pragma unroll
                   for (int u = 0; u < NU; ++u) {
                     pr[u * 32 + lane] = P.x[u];
@@ -574,10 +584,11 @@ __global__ void __launch_bounds__(BRM * 32) jacobi_rows_kernel(T* __restrict__ w
             if (atomicAdd(blk + B_ARR, 1ull) + 1ull == (unsigned long long)n_it) {
               __threadfence();
               const double mc = __longlong_as_double((long long)__ldcg((const long long*)st + ST_MAXCOS));
+              const double mt = __longlong_as_double((long long)__ldcg((const long long*)st + ST_LASTCOS));
+              const bool conv = stops(mc, mt, tol_stop, mixed_stop<R>(tol_stop), is.x + 1);
               st[ST_SWEEPS] = is.x + 1;
-              st[ST_LASTCOS] = __double_as_longlong(mc);
+              st[ST_LASTCOS] = conv || is.x + 1 >= max_sweeps ? __double_as_longlong(mc) : 0;
               st[ST_MAXCOS] = 0;
-              const bool conv = mc <= tol_stop;
               if (conv) st[ST_CONV] = 1;
               blk[B_ARR] = 0ull;
               __threadfence();
@@ -638,7 +649,7 @@ __global__ void __launch_bounds__(BRM * 32) jacobi_rows_kernel(T* __restrict__ w
             if (warp < br) {
               int q = warp + i;
               q -= q >= br ? br : 0;
-              rotate<T, NU>(P, Trows + (size_t)q * stride, tst + q, lane, thr2, thr_cos, maxcos);
+              rotate<T, NU>(P, Trows + (size_t)q * stride, tst + q, lane, thr2, thr_cos, maxcos, &s_tan);
             }
             __syncthreads();
           }

@@ -463,7 +463,7 @@ __device__ __forceinline__ void rotate_rows(T* __restrict__ a, T* __restrict__ b
 
 template <typename T>
 __device__ __forceinline__ void rotate_pair(T* __restrict__ X, T* __restrict__ W, int64_t k, int64_t L, int64_t p,
-                                            int64_t q, int lane, int64_t* st) {
+                                            int64_t q, int lane, int64_t* st, bool mixed) {
   using R = typename Num<T>::R;
   T* xp = X + p * L;
   T* xq = X + q * L;
@@ -488,7 +488,7 @@ __device__ __forceinline__ void rotate_pair(T* __restrict__ X, T* __restrict__ W
   R c = 0, s = 0;
   T u = Num<T>::one();
   const R thr2 = (R)__longlong_as_double((long long)st[sizeof(R) == 4 ? ST_THR32 : ST_THR64]);
-  if (!Rotation<T>::get(al_, be_, ga_, L, lane, st + ST_MAXCOS, c, s, u, thr2)) return;
+  if (!Rotation<T>::get(al_, be_, ga_, L, lane, st + ST_MAXCOS, c, s, u, thr2, mixed)) return;
   rotate_rows<T>(xp, xq, L, lane, c, s, u);
   rotate_rows<T>(W + p * k, W + q * k, k, lane, c, s, u);
 }
@@ -506,6 +506,7 @@ __global__ void __launch_bounds__(kThreads) svd_sweeps_kernel(T* __restrict__ wo
   const int64_t nwarps = (int64_t)gridDim.x * kWarps;
   const int rx = sizeof(typename Num<T>::R) == 4 ? R_X32 : R_X;
   const int rw = sizeof(typename Num<T>::R) == 4 ? R_W32 : R_W;
+  const bool mixed = mixed_stop<typename Num<T>::R>(tol_stop);
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     for (int round = 0; round < max_rounds; ++round) {
       for (int64_t item = gwarp; item < n_items; item += nwarps) {
@@ -526,7 +527,7 @@ __global__ void __launch_bounds__(kThreads) svd_sweeps_kernel(T* __restrict__ wo
         }
         if (p >= k || q >= k) continue;  // the dummy vector of an odd count
         if (p > q) { const int64_t tq = p; p = q; q = tq; }
-        rotate_pair<T>(work + r[rx], work + r[rw], k, L, p, q, lane, st);
+        rotate_pair<T>(work + r[rx], work + r[rw], k, L, p, q, lane, st, mixed);
       }
       if (!grid_barrier(ctrl, gridDim.x)) return;
     }
@@ -538,10 +539,10 @@ __global__ void __launch_bounds__(kThreads) svd_sweeps_kernel(T* __restrict__ wo
         int64_t* st = state + (int64_t)b * ST_REC;
         if (st[ST_CONV]) continue;
         const double mc = __longlong_as_double((long long)st[ST_MAXCOS]);
-        st[ST_SWEEPS] += 1;
-        st[ST_LASTCOS] = st[ST_MAXCOS];
+        const bool conv = stops(mc, __longlong_as_double((long long)st[ST_LASTCOS]), tol_stop, mixed, st[ST_SWEEPS] += 1);
+        st[ST_LASTCOS] = conv || sweep + 1 == max_sweeps ? st[ST_MAXCOS] : 0;
         st[ST_MAXCOS] = 0;
-        if (mc <= tol_stop) st[ST_CONV] = 1; else any_active = 1;
+        if (conv) st[ST_CONV] = 1; else any_active = 1;
       }
       __syncthreads();
       if (threadIdx.x == 0) ctrl[C_DONE] = any_active ? 0ull : 1ull;
@@ -577,6 +578,7 @@ __global__ void __launch_bounds__(BR * 32) svd_block_sweeps_kernel(T* __restrict
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rx = sizeof(typename Num<T>::R) == 4 ? R_X32 : R_X;
   const int rw = sizeof(typename Num<T>::R) == 4 ? R_W32 : R_W;
+  const bool mixed = mixed_stop<typename Num<T>::R>(tol_stop);
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     for (int round = 0; round < max_rounds; ++round) {
       for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
@@ -669,7 +671,7 @@ __global__ void __launch_bounds__(BR * 32) svd_block_sweeps_kernel(T* __restrict
               R c = 0, s = 0;
               T u = Num<T>::one();
               const R thr2 = (R)__longlong_as_double((long long)st[sizeof(R) == 4 ? ST_THR32 : ST_THR64]);
-              if (Rotation<T>::get(al_, be_, ga_, L, lane, st + ST_MAXCOS, c, s, u, thr2)) {
+              if (Rotation<T>::get(al_, be_, ga_, L, lane, st + ST_MAXCOS, c, s, u, thr2, mixed)) {
                 if (in_regs) {
 #pragma unroll
                   for (int v = 0; v < RR; ++v) {
@@ -735,10 +737,10 @@ __global__ void __launch_bounds__(BR * 32) svd_block_sweeps_kernel(T* __restrict
         int64_t* st = state + (int64_t)b * ST_REC;
         if (st[ST_CONV]) continue;
         const double mc = __longlong_as_double((long long)st[ST_MAXCOS]);
-        st[ST_SWEEPS] += 1;
-        st[ST_LASTCOS] = st[ST_MAXCOS];
+        const bool conv = stops(mc, __longlong_as_double((long long)st[ST_LASTCOS]), tol_stop, mixed, st[ST_SWEEPS] += 1);
+        st[ST_LASTCOS] = conv || sweep + 1 == max_sweeps ? st[ST_MAXCOS] : 0;
         st[ST_MAXCOS] = 0;
-        if (mc <= tol_stop) st[ST_CONV] = 1; else any_active = 1;
+        if (conv) st[ST_CONV] = 1; else any_active = 1;
       }
       __syncthreads();
       if (threadIdx.x == 0) ctrl[C_DONE] = any_active ? 0ull : 1ull;

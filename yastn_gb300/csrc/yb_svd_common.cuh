@@ -17,7 +17,8 @@ constexpr long long kSpinLimit = 1ll << 22;
 enum { R_A = 0, R_M, R_N, R_U, R_S, R_V, R_X, R_W, R_P, R_K, R_L, R_NP, R_T, R_X32, R_W32, R_NSUP,
        R_QR, R_LQ, R_Z, R_VQ, R_TAU, R_RR, R_WS, R_NSUP64 };
 // per-block state (int64): [0] max |cos| of the sweep in progress (double bits),
-// [1] converged flag, [2] sweeps run in the current phase, [3] largest |cos| of the last sweep,
+// [1] converged flag, [2] sweeps run in the current phase, [3] largest |cos| of the last sweep (until
+// then the largest tangent of the sweep in progress, see stops),
 // [4], [5] squared row norms (double bits) at or below which a row is rounding noise in the
 // FP32 / FP64 phase: a pair with such a row is neither rotated nor counted for convergence,
 // and the finalisation completes the vectors of those rows like those of zero values
@@ -138,6 +139,21 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// When a phase ends. A sweep whose largest |cos| is c leaves about c^2 where its rotations are small. One
+// by a large tangent t, of two rows of nearly equal norm, moves their cosines with other rows, up to
+// c, to where the sweep has already been: about t c is left. Equal singular values meet that: blocks
+// of 3 to 20 such values stopped at c <= 1e-7 had vectors orthogonal to 4e-8 only. So an SVD's
+// FP64 phase (mixed) ends after a sweep with c <= tol_stop and t c <= kMixed; eigh's stop is low enough by
+// itself. Tangents below kTanMin cannot matter. After kMixedSweeps sweeps c alone decides.
+constexpr double kMixed = 1e-12;
+constexpr float kTanMin = 1e-6f;
+constexpr int kMixedSweeps = 16;
+template <typename R>
+__host__ __device__ __forceinline__ bool mixed_stop(double tol_stop) { return sizeof(R) == 8 && tol_stop > 1e-9; }
+__device__ __forceinline__ bool stops(double maxcos, double maxtan, double tol_stop, bool mixed, int64_t sweeps) {
+  return maxcos <= tol_stop && (!mixed || maxcos * maxtan <= kMixed || sweeps >= kMixedSweeps);
+}
+
 // Jacobi rotation of a row pair from its warp-local partial sums al_ = |x_p|^2, be_ =
 // |x_q|^2, ga_ = <x_p, x_q> (Rutishauser's formulas): returns true (every lane) if the pair
 // is rotated, with (c, s) and the phase u (1 for real rows). |cos| of the pair goes to the
@@ -163,8 +179,9 @@ __device__ __forceinline__ double gabs(double2 g) { return hypot(g.x, g.y); }
 template <typename T>
 struct Rotation {
   using R = typename Num<T>::R;
-  // scalar part: from the summed (al, be, g) to (c, s, u); |cos| to the running maximum
-  __device__ static bool scalar(R al, R be, T ga, int64_t L, int64_t* st, R& c, R& s, T& u, R thr2) {
+  // scalar part: from the summed (al, be, g) to (c, s, u); |cos| (st) and, with mixed, |tan| to the
+  // running maxima
+  __device__ static bool scalar(R al, R be, T ga, int64_t L, int64_t* st, R& c, R& s, T& u, R thr2, bool mixed) {
     if (!(al > thr2 && be > thr2 && al > R(0) && be > R(0))) return false;
     const R g = gabs(ga);
     const R cosv = g / (sqrt(al) * sqrt(be));
@@ -180,12 +197,15 @@ struct Rotation {
       zeta = (be - al) / (R(2) * ga);
     }
     const R t = copysign(R(1), zeta) / (fabs(zeta) + hypot(R(1), zeta));
+    if (mixed && fabs(t) > R(kTanMin))
+      atomicMax((unsigned long long*)st + (ST_LASTCOS - ST_MAXCOS), (unsigned long long)__double_as_longlong((double)fabs(t)));
     c = R(1) / sqrt(fma(t, t, R(1)));
     s = c * t;
     return true;
   }
   // thr2: squared noise norm of the phase; a pair with a row at or below it is left alone
-  __device__ static bool get(R al_, R be_, T ga_, int64_t L, int lane, int64_t* st, R& c, R& s, T& u, R thr2) {
+  __device__ static bool get(R al_, R be_, T ga_, int64_t L, int lane, int64_t* st, R& c, R& s, T& u, R thr2,
+                             bool mixed) {
     const R al = warp_sum(al_), be = warp_sum(be_);
     warp_sum_t<T>(ga_);
     if constexpr (sizeof(R) == 4) {
@@ -210,7 +230,7 @@ struct Rotation {
       return true;
     } else {
       int rot = 0;
-      if (lane == 0) rot = scalar(al, be, ga_, L, st, c, s, u, thr2) ? 1 : 0;
+      if (lane == 0) rot = scalar(al, be, ga_, L, st, c, s, u, thr2, mixed) ? 1 : 0;
       rot = __shfl_sync(0xffffffffu, rot, 0);
       if (!rot) return false;
       c = __shfl_sync(0xffffffffu, c, 0);

@@ -608,7 +608,8 @@ MAX_SWEEPS32 = 40
 TOL_STOP32 = 1.0e-4   # FP32 phase ends after a sweep whose largest rotation |cos| is below this
 TOL_STOP64 = 1.0e-8   # FP64 phase: idem; Jacobi converges quadratically (a sweep that starts at
                       # max |cos| c leaves ~c^2), so the residual after such a sweep is ~1e-16
-TOL_STOP64_QR = 1.0e-7  # the same for the QR-preconditioned SVD (separated, graded rows: ~1e-14 left)
+TOL_STOP64_QR = 1.0e-7  # the same for the QR-preconditioned SVD (separated, graded rows: ~1e-14 left; for
+                        # rows of nearly equal norm the kernels go on, see stops in yb_svd_common.cuh)
 TOL_STOP64_EIGH = 1.0e-11  # eigh: the shifted block A + shift I (shift = ||A||_F + 1) has its singular
                            # values clustered around the shift, so a sweep that starts at |cos| c leaves
                            # ~c^2 shift / gap rather than c^2: 1e-8 left 1e-9 relative reconstruction
