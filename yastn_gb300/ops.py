@@ -620,7 +620,8 @@ BLOCKED_FP64 = [True]  # FP64 phase likewise, on 4-row super-vectors (False: one
 ROWS_PER_SUPER = [None]  # super-vector height (None: largest of 16, 8, 4 that fits)
 NS_STEPS = 2          # Newton-Schulz steps: non-orthogonality ~1e-6 -> 1e-12 -> ~eps
 SVD_EMULATED = [True]  # FP64 products inside svd / eigh on the tensor cores (False: the native grouped GEMM)
-MAX_COMPLETIONS = 8   # completion plans kept with an SvdPlan
+MAX_COMPLETIONS = 64  # completion plans kept with an SvdPlan (a differentiated CTMRG step of 8 iterations has 28
+                      # SVDs of one structure, each with its own counts, and runs them twice)
 SVD_QR = [True]       # svd: Jacobi on the rows of R of a Householder QR (few FP64 sweeps on graded spectra)
 
 
